@@ -31,7 +31,7 @@
 namespace swe {
 
 struct AdjConsts {
-    float g, half_g, dry, eps, dx, dy;
+    float g, half_g, dry, dx, dy;
 };
 
 // The reverse step needs derivative values to float accuracy, not the forward's
@@ -112,7 +112,7 @@ __device__ void adj_face_fwd(FaceIn lo, FaceIn hi, const AdjConsts& k, float F[3
     }
     const float UL[3] = {HL, XL, YL}, UR[3] = {HR, XR, YR};
     const float spread = sR - sL;
-    const float den = spread > k.eps ? spread : 1.f;
+    const float den = spread > kHllEps ? spread : 1.f;
     for (int q = 0; q < 3; ++q) {
         const float m = adiv(sR * fL[q] - sL * fR[q] + sL * sR * (UR[q] - UL[q]), den);
         F[q] = sL >= 0.f ? fL[q] : (sR <= 0.f ? fR[q] : m);
@@ -161,7 +161,7 @@ __device__ void adj_face_vjp(FaceIn lo, FaceIn hi, const AdjConsts& k, const flo
     }
     const float UL[3] = {HL, XL, YL}, UR[3] = {HR, XR, YR};
     const float spread = sR - sL;
-    const bool use_spread = spread > k.eps;
+    const bool use_spread = spread > kHllEps;
     const float den = use_spread ? spread : 1.f;
     const bool take_l = sL >= 0.f, take_r = !take_l && sR <= 0.f;
     // ---- reverse ----

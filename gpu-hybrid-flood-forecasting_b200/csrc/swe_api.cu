@@ -1222,10 +1222,17 @@ int swe_domain_create(const swe_domain_desc* desc, swe_domain_t* out) {
             int e = 0;
             return v > 0.f && std::frexp(v, &e) == 0.5f && e > -120 && e < 120;
         };
-        dd.k.pow2 = pow2(dd.k.dx) && pow2(dd.k.dy) ? 1 : 0;
+        dd.k.forms = pow2(dd.k.dx) && pow2(dd.k.dy) ? kFormPow2 : 0;
     }
-    dd.k.eps = (float)1.0e-12;
     dd.k.expo = (float)(7.0 / 3.0);
+    dd.k.one = 1.0f;
+    {
+        // Range of the controls within which no scaled term of the branch-free
+        // exact arithmetic (swe_exact.cuh) over- or underflows.
+        auto within = [](float v, int lo, int hi) { return v >= std::ldexp(1.0f, lo) && v <= std::ldexp(1.0f, hi); };
+        if (within(dd.k.g, -6, 6) && within(dd.k.dry, -30, 0) && within(dd.k.dx, -10, 17) && within(dd.k.dy, -10, 17))
+            dd.k.forms |= kFormQuick;
+    }
     dd.dx = q.dx;
     dd.dy = q.dy;
     dd.g = q.gravity;
@@ -1320,7 +1327,7 @@ int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const floa
     al.s.dt_rain = (float)dr;
     al.s.dt_g = (float)dg;
     al.dt_rate = (float)dru;
-    al.k = AdjConsts{d->dd.k.g, d->dd.k.half_g, d->dd.k.dry, d->dd.k.eps, d->dd.k.dx, d->dd.k.dy};
+    al.k = AdjConsts{d->dd.k.g, d->dd.k.half_g, d->dd.k.dry, d->dd.k.dx, d->dd.k.dy};
     al.rdx = 1.0f / d->dd.k.dx;
     al.rdy = 1.0f / d->dd.k.dy;
     const int64_t n = (int64_t)rows * d->dd.cols;
@@ -2266,7 +2273,6 @@ int swe_max_inverse_dt_noalloc(const float* h, const float* hu, const float* hv,
     k.dry = (float)dry_tolerance;
     k.dx = (float)dx;
     k.dy = (float)dy;
-    k.eps = (float)1.0e-12;
     k.expo = (float)(7.0 / 3.0);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // The ticket must start at zero; clear it in case an earlier launch was cut short.

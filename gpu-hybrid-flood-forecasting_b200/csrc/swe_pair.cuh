@@ -2,12 +2,12 @@
 //
 // A lane owns two neighbouring cells and carries their fields as float2.  In
 // the fast policy every add/multiply/fma of a pair is one packed sm_100
-// instruction (__fadd2_rn / __fmul2_rn / __ffma2_rn).  The exact policy keeps
-// the scalar __fadd_rn / __fmul_rn per component: those are documented never
-// to be merged into a fused multiply-add, a guarantee the packed forms do not
-// state (measured: packed exact arithmetic drifted by ulps from the reference
-// on a lake at rest, the scalar form is bit-identical).  Divisions, square
-// roots, compares and selects are per component in both policies.
+// instruction (__fadd2_rn / __fmul2_rn / __ffma2_rn).  The exact policy here
+// keeps the scalar __fadd_rn / __fmul_rn per component: those are documented
+// never to be merged into a fused multiply-add, which the packed forms are.
+// It is the general form, for any operands; the march runs its branch-free
+// packed form (swe_exact.cuh) and falls back to this one per row.  Compares and
+// selects are per component in both policies.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -71,6 +71,14 @@ __device__ __forceinline__ auto all_true<float2>() { return B2{true, true}; }
 template <class M>
 struct P;
 
+// The operations of P<ExactMath> with a slow path of their own are calls: the
+// march runs them only for rows outside the range of swe_exact.cuh, and inlined
+// they were most of its instructions.
+__device__ __noinline__ inline float ieee_div(float a, float b) { return __fdiv_rn(a, b); }
+__device__ __noinline__ inline float ieee_sqrt(float a) { return __fsqrt_rn(a); }
+__device__ __noinline__ inline float ieee_hypot(float a, float b) { return ExactMath::hypot(a, b); }
+__device__ __noinline__ inline float ieee_pow73(float x, float e) { return pow73_exact(x, e); }
+
 template <>
 struct P<ExactMath> {
     static constexpr bool kExact = true;
@@ -86,18 +94,18 @@ struct P<ExactMath> {
     __device__ static __forceinline__ float2 mul(float2 a, float2 b) {
         return {__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)};
     }
-    __device__ static __forceinline__ float div(float a, float b) { return __fdiv_rn(a, b); }
+    __device__ static __forceinline__ float div(float a, float b) { return ieee_div(a, b); }
     __device__ static __forceinline__ float2 div(float2 a, float2 b) {
-        return {__fdiv_rn(a.x, b.x), __fdiv_rn(a.y, b.y)};
+        return {ieee_div(a.x, b.x), ieee_div(a.y, b.y)};
     }
-    __device__ static __forceinline__ float sqrt(float a) { return __fsqrt_rn(a); }
-    __device__ static __forceinline__ float2 sqrt(float2 a) { return {__fsqrt_rn(a.x), __fsqrt_rn(a.y)}; }
-    __device__ static __forceinline__ float hypot(float a, float b) { return ExactMath::hypot(a, b); }
+    __device__ static __forceinline__ float sqrt(float a) { return ieee_sqrt(a); }
+    __device__ static __forceinline__ float2 sqrt(float2 a) { return {ieee_sqrt(a.x), ieee_sqrt(a.y)}; }
+    __device__ static __forceinline__ float hypot(float a, float b) { return ieee_hypot(a, b); }
     __device__ static __forceinline__ float2 hypot(float2 a, float2 b) {
-        return {ExactMath::hypot(a.x, b.x), ExactMath::hypot(a.y, b.y)};
+        return {ieee_hypot(a.x, b.x), ieee_hypot(a.y, b.y)};
     }
-    __device__ static __forceinline__ float pow73(float x, float e) { return powf(x, e); }
-    __device__ static __forceinline__ float2 pow73(float2 x, float e) { return {powf(x.x, e), powf(x.y, e)}; }
+    __device__ static __forceinline__ float pow73(float x, float e) { return ieee_pow73(x, e); }
+    __device__ static __forceinline__ float2 pow73(float2 x, float e) { return {ieee_pow73(x.x, e), ieee_pow73(x.y, e)}; }
 };
 
 template <>
@@ -144,11 +152,12 @@ struct FaceT {
 // Step constants as scalars and as splatted pairs.
 struct KPair {
     float2 g, half_g, dry, eps, zero, one, tiny;
+    float2 g_up, eps_up;  // 2^64 g and 2^32 eps (branch-free exact arithmetic, swe_exact.cuh)
 };
 
 __device__ __forceinline__ KPair make_kpair(const Consts& k) {
-    return {splat(k.g), splat(k.half_g), splat(k.dry), splat(k.eps), splat(0.f), splat(1.f),
-            splat(1.0e-30f)};
+    return {splat(k.g), splat(k.half_g), splat(k.dry), splat(kHllEps), splat(0.f), splat(1.f),
+            splat(1.0e-30f), splat(k.g * 1.8446744073709552e19f), splat(kHllEps * 4294967296.0f)};
 }
 
 // Velocities of a cell or a pair of cells (numpy_solver/shallow_water_2d.py:60-63).

@@ -41,10 +41,17 @@ struct Consts {
     float half_g;  // float(0.5 * g)
     float dry;     // float(dry_tolerance)
     float dx, dy;  // float(dx), float(dy)
-    float eps;     // float(1e-12)   HLL denominator guard
     float expo;    // float(7/3)     Manning exponent
-    int pow2;      // 1: dx and dy are powers of two, so x / dx == x * (1 / dx) exactly
+    float one;     // 1 as a run-time value (see PairOps in swe_exact.cuh)
+    int forms;     // kFormPow2 | kFormQuick
 };
+
+// dx and dy are powers of two, so x / dx == x * (1 / dx) exactly.
+constexpr int kFormPow2 = 1;
+// The controls lie inside the range of the branch-free exact arithmetic (swe_exact.cuh).
+constexpr int kFormQuick = 2;
+
+constexpr float kHllEps = 1.0e-12f;  // HLL denominator guard
 
 // Per-step float32 scalars: float(dt), float(dt*rate), float(dt*g).
 struct StepScalars {
@@ -375,7 +382,7 @@ __device__ __forceinline__ FaceFlux face_flux(const Cell& lo, const Cell& hi, co
         fR2 = M::add(M::mul(YR, unR), pR);
     }
     const float spread = M::sub(sR, sL);
-    const float den = spread > k.eps ? spread : 1.0f;
+    const float den = spread > kHllEps ? spread : 1.0f;
     const float rden = M::recip(den);
     const float s01 = M::mul(sL, sR);
     const float m0 = M::over(M::add(M::sub(M::mul(sR, fL0), M::mul(sL, fR0)), M::mul(s01, M::sub(HR, HL))), rden);

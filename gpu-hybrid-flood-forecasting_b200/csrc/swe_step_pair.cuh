@@ -15,17 +15,21 @@
 // ring).
 #pragma once
 
+#include "swe_exact.cuh"
 #include "swe_pair.cuh"
 #include "swe_step.cuh"
+
+#include <type_traits>
 
 namespace swe {
 
 struct KScalar {
     float g, half_g, dry, eps, zero, one, tiny;
+    float g_up, eps_up;
 };
 
 __device__ __forceinline__ KScalar make_kscalar(const Consts& k) {
-    return {k.g, k.half_g, k.dry, k.eps, 0.f, 1.f, 1.0e-30f};
+    return {k.g, k.half_g, k.dry, kHllEps, 0.f, 1.f, 1.0e-30f, k.g * 1.8446744073709552e19f, kHllEps * 4294967296.0f};
 }
 
 constexpr int kRing = 4;  // rows in flight per warp (a power of two)
@@ -117,8 +121,15 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     // Exact arithmetic divides by dx and dy as the reference does; when both are
     // powers of two that is the multiplication by their (exact) reciprocals, the
     // same correctly rounded result (a warp-uniform branch).
-    const bool pow2 = k.pow2 != 0;
+    const bool pow2 = (k.forms & kFormPow2) != 0;
     const float2 rdxe = splat(__frcp_rn(k.dx)), rdye = splat(__frcp_rn(k.dy));
+    // Exact arithmetic: the operations of the branch-free form, and whether the
+    // domain's controls and the step's dt allow it at all.
+    const PairOps po{splat(k.one), splat(-k.one)};
+    const SoloOps so1;
+    using Quick = std::conditional_t<A::kExact, QuickExact, M>;
+    const bool ieee_domain = A::kExact && (k.forms & kFormQuick) == 0;
+    bool ieee_step = ieee_domain, ieee_batch = false;  // rows that take the IEEE operations (warp-uniform)
     auto over_dx = [&](float2 a) {
         if constexpr (A::kExact) return pow2 ? A::mul(a, rdxe) : A::div(a, dx2);
         else return A::mul(a, rdxe);  // not used by the fast policy
@@ -157,7 +168,8 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         cp_async_commit();
     };
     // Ring row qi into registers, ghost ring applied; its slot is refilled with row qi+kRing.
-    auto consume = [&](int qi, CellT<float2>& c) {
+    // Returns the row's largest depth or speed in exact arithmetic (see kQuickLimit).
+    auto consume = [&](int qi, CellT<float2>& c) -> float {
         cp_async_wait<kRing - 1>();
         const int slot = qi & (kRing - 1);
         const int q = r0 - 1 + qi;
@@ -191,8 +203,15 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         }
         c.z = fv[3];
         c.nm = fv[4];
-        set_vel_t<M>(c, kp);
+        float big = 0.f;
+        if constexpr (A::kExact) {
+            quick_vel(po, c, kp);
+            big = max3_nan(max3_nan(c.h.x, fabsf(c.u.x), fabsf(c.v.x)), c.h.y, max3_nan(fabsf(c.u.y), fabsf(c.v.y), 0.f));
+        } else {
+            set_vel_t<M>(c, kp);
+        }
         issue(qi + kRing);
+        return big;
     };
 
     struct {
@@ -223,7 +242,25 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     for (int qi = 0; qi < kRing; ++qi) issue(qi);
 
     CellT<float2> R0, R1;
+    float big0 = 0.f, big1 = 0.f;  // their rows' largest depth or speed (exact arithmetic)
     float2 yT0, yT1, yT2;
+
+    // A face, and an addition, of one policy: the march's own (fast arithmetic, or
+    // the IEEE operations of exact arithmetic) or the branch-free exact form.
+    auto face = [&](auto policy, auto axis, const CellT<float2>& lo, const CellT<float2>& hi) -> FaceT<float2> {
+        if constexpr (std::is_same_v<decltype(policy), QuickExact>)
+            return quick_face<decltype(axis)::value, MASKED>(po, lo, hi, kp);
+        else
+            return face_t<decltype(axis)::value, M, MASKED>(lo, hi, kp);
+    };
+    auto plus = [&](auto policy, float2 a, float2 b) -> float2 {
+        if constexpr (std::is_same_v<decltype(policy), QuickExact>)
+            return po.add(a, b);
+        else
+            return A::add(a, b);
+    };
+    constexpr std::integral_constant<int, 0> kY{};
+    constexpr std::integral_constant<int, 1> kX{};
 
     // The x-faces of a row: (cell 0 | cell 1) and (cell 1 | first cell of the next lane).
     // Returns the lo-side fluxes of both cells' left faces and the hi-side of their right faces.
@@ -232,7 +269,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         float2 r0, r1, r2;  // flux leaving through each cell's right face (lo side)
         float2 e0;          // mass flux through each cell's right face (east outflow)
     };
-    auto xfaces = [&](const CellT<float2>& cur, int j) -> XF {
+    auto xfaces = [&](auto policy, const CellT<float2>& cur, int j) -> XF {
         // The face reads depth, bed and velocities of its two cells (and n^2 for
         // the mask): the neighbour's momenta are not moved.
         float rh = __shfl_down_sync(0xffffffffu, cur.h.x, 1);
@@ -252,8 +289,8 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         xhi.nm = f2(cur.nm.y, rnm);
         xhi.u = f2(cur.u.y, ru);
         xhi.v = f2(cur.v.y, rv);
-        const FaceT<float2> fx = face_t<1, M, MASKED>(cur, xhi, kp);
-        const float2 xh1 = A::add(fx.f1, fx.corr_hi);
+        const FaceT<float2> fx = face(policy, kX, cur, xhi);
+        const float2 xh1 = plus(policy, fx.f1, fx.corr_hi);
         float up0 = __shfl_up_sync(0xffffffffu, fx.f0.y, 1);
         float up1 = __shfl_up_sync(0xffffffffu, xh1.y, 1);
         float up2 = __shfl_up_sync(0xffffffffu, fx.f2.y, 1);
@@ -262,7 +299,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         }
         XF x;
         x.r0 = fx.f0;
-        x.r1 = A::add(fx.f1, fx.corr_lo);
+        x.r1 = plus(policy, fx.f1, fx.corr_lo);
         x.r2 = fx.f2;
         x.l0 = f2(up0, fx.f0.x);
         x.l1 = f2(up1, xh1.x);
@@ -274,13 +311,40 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     struct Row {
         float2 h, hu, hv;
     };
+    struct Update {
+        Row o;
+        float2 u0, rain;  // depth after the rain, before the clip; the rain
+        float2 inv;       // inverse CFL dt of the new cells (run mode)
+        float big;        // exact arithmetic: the largest speed behind inv, or the largest new value
+    };
     // Cell update of one row from its faces: bottom (b*), top (t*, lo side), x-faces.
-    auto update = [&](int r, const CellT<float2>& cur, float2 b0, float2 b1, float2 b2, float2 t0, float2 t1,
-                      float2 t2, const XF& x) -> Row {
+    auto update = [&](auto policy, int r, const CellT<float2>& cur, float2 b0, float2 b1, float2 b2, float2 t0,
+                      float2 t1, float2 t2, const XF& x) -> Update {
+        constexpr bool kQuick = std::is_same_v<decltype(policy), QuickExact>;
         const auto act = MASKED ? act_of(cur.nm) : all_true<float2>();
         const float2 n2 = MASKED ? vabs(cur.nm) : cur.nm;
+        const float2 up = splat(kUp), down = splat(kDown);
         float2 u0, u1, u2;
-        if constexpr (A::kExact) {
+        if constexpr (kQuick) {
+            if (pow2) {
+                const float2 d0 = po.add(po.mul(po.sub(x.r0, x.l0), rdxe), po.mul(po.sub(t0, b0), rdye));
+                const float2 d1 = po.add(po.mul(po.sub(x.r1, x.l1), rdxe), po.mul(po.sub(t1, b1), rdye));
+                const float2 d2 = po.add(po.mul(po.sub(x.r2, x.l2), rdxe), po.mul(po.sub(t2, b2), rdye));
+                u0 = po.sub(cur.h, po.mul(dt2, d0));
+                u1 = po.sub(cur.hu, po.mul(dt2, d1));
+                u2 = po.sub(cur.hv, po.mul(dt2, d2));
+            } else {
+                // The divergence times kUp; dt / kUp is exact.
+                const float2 dtd2 = po.mul(dt2, down);
+                auto div_up = [&](float2 xr, float2 xl, float2 yt, float2 yb) {
+                    return po.add(quick_div(po, po.mul(po.sub(xr, xl), up), dx2, rdxe),
+                                  quick_div(po, po.mul(po.sub(yt, yb), up), dy2, rdye));
+                };
+                u0 = po.sub(cur.h, po.mul(dtd2, div_up(x.r0, x.l0, t0, b0)));
+                u1 = po.sub(cur.hu, po.mul(dtd2, div_up(x.r1, x.l1, t1, b1)));
+                u2 = po.sub(cur.hv, po.mul(dtd2, div_up(x.r2, x.l2, t2, b2)));
+            }
+        } else if constexpr (A::kExact) {
             u0 = A::sub(cur.h, A::mul(dt2, A::add(over_dx(A::sub(x.r0, x.l0)), over_dy(A::sub(t0, b0)))));
             u1 = A::sub(cur.hu, A::mul(dt2, A::add(over_dx(A::sub(x.r1, x.l1)), over_dy(A::sub(t1, b1)))));
             u2 = A::sub(cur.hv, A::mul(dt2, A::add(over_dx(A::sub(x.r2, x.l2)), over_dy(A::sub(t2, b2)))));
@@ -294,10 +358,20 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             const int64_t mo = (int64_t)r * d.spitch;
             rain = A::mul(dtr2, f2(__ldg(d.mult + mo + min(c0, d.cols - 1)), __ldg(d.mult + mo + min(c0 + 1, d.cols - 1))));
         }
-        u0 = A::add(u0, rain);
+        u0 = plus(policy, u0, rain);
         const float2 h = vmax(u0, kp.zero);
-        float2 qx, qy;
-        if constexpr (A::kExact) {
+        float2 qx, qy, deep, rdeep;
+        if constexpr (kQuick) {
+            const float2 norm = quick_hypot(u1, u2);
+            deep = vmax(h, kp.dry);
+            rdeep = quick_rcp(po, deep);
+            const float2 pw = quick_pow73(po, deep, rdeep);
+            const float2 fr = quick_div(po, po.mul(po.mul(dtg2, n2), norm), pw, quick_rcp(po, pw));
+            const float2 den = po.mul(po.add(kp.one, fr), up);
+            const float2 rden = quick_rcp(po, den);
+            qx = quick_div(po, po.mul(u1, up), den, rden);
+            qy = quick_div(po, po.mul(u2, up), den, rden);
+        } else if constexpr (A::kExact) {
             const float2 norm = A::hypot(u1, u2);
             const float2 fr = A::div(A::mul(A::mul(dtg2, n2), norm), A::pow73(vmax(h, kp.dry), k.expo));
             const float2 den = A::add(kp.one, fr);
@@ -312,42 +386,64 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             qy = A::mul(u2, rd);
         }
         const auto wet = act & gt(h, kp.dry);
-        Row o;
-        o.h = sel(act, h, kp.zero);
-        o.hu = sel(wet, qx, kp.zero);
-        o.hv = sel(wet, qy, kp.zero);
+        Update w;
+        w.o.h = sel(act, h, kp.zero);
+        w.o.hu = sel(wet, qx, kp.zero);
+        w.o.hv = sel(wet, qy, kp.zero);
+        w.u0 = u0;
+        w.rain = rain;
+        w.big = 0.f;
         if constexpr (RUN) {
-            const float2 w = A::sqrt(A::mul(kp.g, o.h));
-            float2 inv;
-            if constexpr (A::kExact) {
+            if constexpr (kQuick) {
+                // Where the new cell is wet, its depth is `deep`; elsewhere its momenta are zero.
+                const float2 c = po.mul(quick_celerity_up(po, w.o.h, kp.g_up), down);
+                const float2 su = po.add(vabs(quick_div(po, w.o.hu, deep, rdeep)), c);
+                const float2 sv = po.add(vabs(quick_div(po, w.o.hv, deep, rdeep)), c);
+                if (pow2) w.inv = po.add(po.mul(su, rdxe), po.mul(sv, rdye));
+                else w.inv = po.add(quick_div(po, su, dx2, rdxe), quick_div(po, sv, dy2, rdye));
+                w.big = max3_nan(max3_nan(su.x, su.y, 0.f), sv.x, sv.y);
+            } else if constexpr (A::kExact) {
+                const float2 c = A::sqrt(A::mul(kp.g, w.o.h));
                 CellT<float2> nc;
-                nc.h = o.h;
-                nc.hu = o.hu;
-                nc.hv = o.hv;
+                nc.h = w.o.h;
+                nc.hu = w.o.hu;
+                nc.hv = w.o.hv;
                 set_vel_t<M>(nc, kp);
-                inv = A::add(over_dx(A::add(vabs(nc.u), w)), over_dy(A::add(vabs(nc.v), w)));
+                w.inv = A::add(over_dx(A::add(vabs(nc.u), c)), over_dy(A::add(vabs(nc.v), c)));
             } else {
+                const float2 c = A::sqrt(A::mul(kp.g, w.o.h));
                 // The new momenta are zero wherever h <= dry, so 1/max(h, dry) gives the
                 // same velocities as the dry-cell rule of the reference.
-                const float2 rh = A::rcp(vmax(o.h, kp.dry));
-                inv = A::fma(A::add(vabs(A::mul(o.hu, rh)), w), rdx2, A::mul(A::add(vabs(A::mul(o.hv, rh)), w), rdy2));
+                const float2 rh = A::rcp(vmax(w.o.h, kp.dry));
+                w.inv = A::fma(A::add(vabs(A::mul(w.o.hu, rh)), c), rdx2, A::mul(A::add(vabs(A::mul(w.o.hv, rh)), c), rdy2));
             }
+        } else if constexpr (kQuick) {
+            // Compared with kQuickLimit like a speed; a momentum may be larger by the depth.
+            const float2 s = splat(1.0f / kQuickLimit);
+            const float2 a = vabs(po.mul(w.o.hu, s)), b = vabs(po.mul(w.o.hv, s));
+            w.big = max3_nan(max3_nan(a.x, a.y, w.o.h.x), max3_nan(b.x, b.y, w.o.h.y), 0.f);
+        }
+        return w;
+    };
+    // The row's share of the CFL maximum and the ledger.
+    auto account = [&](const CellT<float2>& cur, const Update& w, const XF& x) {
+        if constexpr (RUN) {
+            const auto act = MASKED ? act_of(cur.nm) : all_true<float2>();
             // Inactive cells have h = hu = hv = 0 and so inv = 0; lanes past the edge are masked.
-            inv = A::mul(inv, vmask);
+            const float2 inv = A::mul(w.inv, vmask);
             // Maximum without the NaN test per cell: a NaN or infinite inverse dt
             // turns the float volume partial into NaN (0 * NaN, 0 * inf), and the
             // fold reports the step as non-finite.
             maxinv = fmaxf(maxinv, fmaxf(inv.x, inv.y));
-            lg.vol = lfma(inv, kp.zero, lfma(o.h, vmask, lg.vol));
-            if (d.mult != nullptr) lg.rain = lfma(rain, vmask, lg.rain);
-            lg.clip = lfma(neg(vmin(u0, kp.zero)), vmask, lg.clip);
+            lg.vol = lfma(inv, kp.zero, lfma(w.o.h, vmask, lg.vol));
+            if (d.mult != nullptr) lg.rain = lfma(w.rain, vmask, lg.rain);
+            lg.clip = lfma(neg(vmin(w.u0, kp.zero)), vmask, lg.clip);
             if constexpr (MASKED) {
-                lg.mask = lfma(sel(act, kp.zero, h), vmask, lg.mask);
+                lg.mask = lfma(sel(act, kp.zero, vmax(w.u0, kp.zero)), vmask, lg.mask);
                 if (d.mult == nullptr) acc.rain_cells += (act.x && valid.x ? 1u : 0u) + (act.y && valid.y ? 1u : 0u);
             }
             lg.out_x = lfma(x.e0, emask, lg.out_x);
         }
-        return o;
     };
     auto store = [&](int r, const Row& o) {
         const uint32_t so = (uint32_t)r * (uint32_t)out.pitch + (uint32_t)c0;
@@ -409,10 +505,23 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         CellT<float> l{L[0].h, L[0].hu, L[0].hv, L[0].z, L[0].nm, 0.f, 0.f};
         CellT<float> e{E[0].h, E[0].hu, E[0].hv, E[0].z, E[0].nm, 0.f, 0.f};
         CellT<float> q{Q[0].h, Q[0].hu, Q[0].hv, Q[0].z, Q[0].nm, 0.f, 0.f};
-        set_vel_t<M>(l, ks);
-        set_vel_t<M>(e, ks);
-        set_vel_t<M>(q, ks);
-        const FaceT<float> f = face_t<1, M, MASKED>(l, e, ks);
+        FaceT<float> f;
+        if constexpr (A::kExact) {
+            quick_vel(so1, l, ks);
+            quick_vel(so1, e, ks);
+            quick_vel(so1, q, ks);
+            f = quick_face<1, MASKED>(so1, l, e, ks);
+            const float big = max3_nan(max3_nan(l.h, fabsf(l.u), fabsf(l.v)), max3_nan(e.h, fabsf(e.u), fabsf(e.v)),
+                                       max3_nan(q.h, fabsf(q.u), fabsf(q.v)));
+            // Rows whose edge cells leave the range take the IEEE operations, here and in the rows.
+            ieee_batch = ieee_domain || __any_sync(0xffffffffu, !(big < kQuickLimit));
+        }
+        if (!A::kExact || ieee_batch) {
+            set_vel_t<M>(l, ks);
+            set_vel_t<M>(e, ks);
+            set_vel_t<M>(q, ks);
+            f = face_t<1, M, MASKED>(l, e, ks);
+        }
         sm.left[0][lane] = f.f0;
         sm.left[1][lane] = A::add(f.f1, f.corr_hi);
         sm.left[2][lane] = f.f2;
@@ -426,18 +535,37 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     };
 
     // One row: `cur` is row r, `nxt` row r+1; afterwards `cur` receives row r+2.
-    auto row = [&](const int r, const int j, CellT<float2>& cur, const CellT<float2>& nxt) {
-        const FaceT<float2> fy = face_t<0, M, MASKED>(cur, nxt, kp);
-        const XF x = xfaces(cur, j);
-        const Row o = update(r, cur, yT0, yT1, yT2, fy.f0, fy.f1, A::add(fy.f2, fy.corr_lo), x);
+    auto row = [&](const int r, const int j, CellT<float2>& cur, const CellT<float2>& nxt, float& big_cur,
+                   const float big_nxt) {
+        FaceT<float2> fy;
+        XF x;
+        Update w;
+        float2 t2;
+        auto evaluate = [&](auto policy, const CellT<float2>& c, const CellT<float2>& n) {
+            fy = face(policy, kY, c, n);
+            x = xfaces(policy, c, j);
+            t2 = plus(policy, fy.f2, fy.corr_lo);
+            w = update(policy, r, c, yT0, yT1, yT2, fy.f0, fy.f1, t2, x);
+        };
+        evaluate(Quick{}, cur, nxt);
+        if constexpr (A::kExact) {
+            const float big = max3_nan(big_cur, big_nxt, w.big);
+            if (__any_sync(0xffffffffu, !(big < kQuickLimit)) || ieee_step || ieee_batch) {
+                CellT<float2> c = cur, n = nxt;
+                set_vel_t<M>(c, kp);
+                set_vel_t<M>(n, kp);
+                evaluate(M{}, c, n);
+            }
+        }
+        account(cur, w, x);
         if constexpr (RUN) {
             if (r == d.rows - 1) lg.out_y = lfma(fy.f0, vmask, lg.out_y);
         }
         yT0 = fy.f0;
         yT1 = fy.f1;
         yT2 = A::add(fy.f2, fy.corr_hi);
-        store(r, o);
-        if (LAST_CONSUME || r + 1 < r1) consume(r + 3 - r0, cur);
+        store(r, w.o);
+        if (LAST_CONSUME || r + 1 < r1) big_cur = consume(r + 3 - r0, cur);
     };
     // The first batch's strip edges are loaded before the ring's first rows are
     // waited for, and the step is planned while the ring's rows are in flight,
@@ -456,11 +584,23 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         ndtdy2 = splat(-mp.s.dt * rdy);
         snap = mp.snap;
         dtd = mp.dtd;
+        if constexpr (A::kExact) {
+            const float adt = fabsf(mp.s.dt);
+            ieee_step = ieee_domain || !(adt < kUp) || (adt != 0.f && adt < kDown);
+        }
     }
-    consume(0, R1);  // row r0-1
-    consume(1, R0);  // row r0
+    big1 = consume(0, R1);  // row r0-1
+    big0 = consume(1, R0);  // row r0
     {
-        const FaceT<float2> f = face_t<0, M, MASKED>(R1, R0, kp);
+        FaceT<float2> f = face(Quick{}, kY, R1, R0);
+        if constexpr (A::kExact) {
+            if (ieee_step || __any_sync(0xffffffffu, !(max3_nan(big0, big1, 0.f) < kQuickLimit))) {
+                CellT<float2> c = R1, n = R0;
+                set_vel_t<M>(c, kp);
+                set_vel_t<M>(n, kp);
+                f = face(M{}, kY, c, n);
+            }
+        }
         yT0 = f.f0;
         yT1 = f.f1;
         yT2 = A::add(f.f2, f.corr_hi);
@@ -468,14 +608,14 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             if (r0 == 0) lg.out_y = lfma(neg(f.f0), vmask, lg.out_y);
         }
     }
-    consume(2, R1);  // row r0+1
+    big1 = consume(2, R1);  // row r0+1
     for (int rb = r0; rb < r1; rb += kBatch) {
         flush_ledger();
         if (rb != r0) batch(rb);
         const int re = min(rb + kBatch, r1);
         for (int r = rb; r < re; r += 2) {
-            row(r, r - rb, R0, R1);
-            if (r + 1 < re) row(r + 1, r + 1 - rb, R1, R0);
+            row(r, r - rb, R0, R1, big0, big1);
+            if (r + 1 < re) row(r + 1, r + 1 - rb, R1, R0, big1, big0);
         }
     }
     flush_ledger();
@@ -648,6 +788,7 @@ struct EnsParams {
     int cta_begin[kEnsParamMembers + 1];
     int n_members, n_items, parity;
 };
+static_assert(sizeof(EnsParams) <= 32764, "the member table must fit the kernel parameters");
 
 template <class M, int THREADS, bool MASKED>
 __global__ void __launch_bounds__(THREADS, SWE_ENS_MINBLOCKS)
