@@ -230,9 +230,22 @@ void dispatch(int V, int arith, bool run, bool masked, F&& f) {
     }
 }
 
+// Rows per warp of a grid that does not fill the GPU: a step then lasts as long
+// as one warp's march, so it is split until every scheduler has two warps (kFewWarps
+// per SM), but not below the split that fills one wave (`one_wave`), and not
+// beyond 4 rows, where more warps in the wave are worth more.  Measured (us a step in
+// blocks of 100 steps, fast unless said, at 1 / 2 / 4 / 8 rows): 128^2 7.3 / 8.0 /
+// 8.7 / 11.5; 300 x 420 9.8 / 8.7 / 9.2 / 12.0; 256^2 exact 10.2 / 10.5 / 12.0 / 16.2;
+// 512^2 exact 23 / 16.5 / 14.1 / 16.7; 700^2 at 4 / 6 / 8 rows 13.7 / 14.4 / 14.3.
+constexpr int kFewWarps = 8;
+
+int march_rows(int64_t one_wave, int64_t two_a_scheduler) {
+    return (int)std::max<int64_t>(one_wave, std::min<int64_t>(two_a_scheduler, 4));
+}
+
 // Work items are (strip of 32*V columns) x (chunk of R rows), one per warp.  R is
 // chosen so that all warps are resident at once (one full wave at the kernel's
-// occupancy), which equalises the work of every SM; chunks keep >= 4 rows.
+// occupancy), which equalises the work of every SM; smaller grids see march_rows.
 Plan make_plan(const swe_domain* d, int V, bool run) {
     Plan p;
     p.V = V;
@@ -253,9 +266,11 @@ Plan make_plan(const swe_domain* d, int V, bool run) {
     const int64_t warps_avail = (int64_t)occ * d->sms * wpb;
     int R = d->rows_per_warp_override;
     if (R <= 0) {
-        const int64_t chunks = std::max<int64_t>(1, warps_avail / p.nstrips);
-        R = (int)((rows + chunks - 1) / chunks);
-        R = std::max(R, std::min(4, rows));
+        auto rows_for = [&](int64_t warps) {
+            const int64_t chunks = std::max<int64_t>(1, warps / p.nstrips);
+            return (rows + chunks - 1) / chunks;
+        };
+        R = march_rows(rows_for(warps_avail), rows_for((int64_t)kFewWarps * d->sms));
     }
     p.rows_per_warp = R;
     const int64_t chunks = (rows + R - 1) / R;

@@ -82,19 +82,20 @@ __device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) { return __
 // values unused), which keeps the row body free of that branch; the plain step
 // measured 0.6 % faster with it, the ensemble kernel spills with it.
 //
-// EDGES (the plain run-mode step): with epar >= 0, the domain keeps its
-// strip-boundary columns (DomainDev::edge) and `in` is ping-pong buffer epar.
-// The strip edges are then read from edge[epar] where the neighbouring cells
-// lie inside the grid (one coalesced access per quantity for 32 rows, where
-// the state would need one cache line per row), and lanes 0 and 31 write the
-// strip's first and last columns of `out` into edge[epar ^ 1] for the next
-// step.  In fast arithmetic the 2048^2 step measured 7 % faster with it and
-// the ensemble of 16 x 1024^2 members (114-row marches) 6 % (the 64-member mix,
-// 256-row marches, the same); in exact arithmetic (more registers) it spilled
-// and measured 1.5 % slower, so exact marches load their edges from the state.
+// Run mode, with epar >= 0: the domain keeps its strip-boundary columns
+// (DomainDev::edge) and `in` is ping-pong buffer epar.  The strip edges are then
+// read from edge[epar] (one coalesced access per quantity for 32 rows, where the
+// state would need one cache line per row), and lanes 0 and 31 write the strip's
+// first and last columns of `out` into edge[epar ^ 1] for the next step.  In fast
+// arithmetic the 2048^2 step measured 7 % faster with it and the ensemble of 16 x
+// 1024^2 members (114-row marches) 6 % (the 64-member mix, 256-row marches, the
+// same); in exact arithmetic 256^2 takes 7.0 us (8.2 without), 512^2 11.3 (12.2),
+// 1024^2 24.2 (26.0), 2048^2 77.8 (80.0).  The strips at the grid's own edges
+// read theirs there too: the ghost column is the mirrored edge column (128^2
+// fast 6.6 us a step instead of 7.5, 300 x 420 7.2 instead of 7.5).
 static_assert(kEdgeStrip == 2 * kWarp, "a paired-march strip is 2 x 32 columns");
 
-template <class M, bool RUN, bool MASKED, bool LAST_CONSUME, bool EDGES, class PlanFn>
+template <class M, bool RUN, bool MASKED, bool LAST_CONSUME, class PlanFn>
 __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& in,
                                             const StateOut& out, PlanFn&& plan_fn, const Control* ctl,
                                             int r0, int r1, int x0w, WarpSmem& sm, StepAccum& acc, int epar = -1) {
@@ -140,7 +141,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     };
     // This lane's column run of the next step's edges (lanes 0 and 31), or null.
     float* ep = nullptr;
-    if (EDGES && epar >= 0) {
+    if (RUN && epar >= 0) {
         const int eb = x0w / kEdgeStrip;
         if (lane == 0) ep = d.edge[epar ^ 1] + edge_index(d, eb, 3, 0);
         else if (lane == kWarp - 1 && valid.y) ep = d.edge[epar ^ 1] + edge_index(d, eb + 1, 0, 0);
@@ -456,7 +457,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             out.hu[so] = o.hu.x;
             out.hv[so] = o.hv.x;
         }
-        if (EDGES && ep != nullptr) {
+        if (RUN && ep != nullptr) {
             const bool first = lane == 0;
             ep[r] = first ? o.h.x : o.h.y;
             ep[r + d.edge_rows] = first ? o.hu.x : o.hu.y;
@@ -483,23 +484,26 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         const int rr = min(rb + lane, d.rows - 1);
         Cell L[1], E[1], Q[1];
         const int b = x0w / kEdgeStrip;
-        const float* ein = EDGES && epar >= 0 ? d.edge[epar] : nullptr;
-        if (EDGES && ein != nullptr && x0w > 0) {
-            L[0] = {__ldg(ein + edge_index(d, b, 0, rr)), __ldg(ein + edge_index(d, b, 1, rr)),
-                    __ldg(ein + edge_index(d, b, 2, rr)), __ldg(d.edge_static + edge_static_index(d, b, 0, rr)),
-                    __ldg(d.edge_static + edge_static_index(d, b, 1, rr)), 0.f, 0.f};
-            E[0] = {__ldg(ein + edge_index(d, b, 3, rr)), __ldg(ein + edge_index(d, b, 4, rr)),
-                    __ldg(ein + edge_index(d, b, 5, rr)), __ldg(d.edge_static + edge_static_index(d, b, 2, rr)),
-                    __ldg(d.edge_static + edge_static_index(d, b, 3, rr)), 0.f, 0.f};
+        const float* ein = RUN && epar >= 0 ? d.edge[epar] : nullptr;
+        if (RUN && ein != nullptr) {
+            // The grid's own edges: the ghost column is the mirrored edge column.  Past a
+            // partial strip the last column's ghost sits in the strip itself (consume), so
+            // the cell right of it is not read: any cell does.
+            const bool west = x0w == 0, full = x0w + kEdgeStrip <= d.cols, east = x0w + kEdgeStrip >= d.cols;
+            auto side = [&](int bd, int right) -> Cell {
+                return {__ldg(ein + edge_index(d, bd, 3 * right + 0, rr)), __ldg(ein + edge_index(d, bd, 3 * right + 1, rr)),
+                        __ldg(ein + edge_index(d, bd, 3 * right + 2, rr)),
+                        __ldg(d.edge_static + edge_static_index(d, bd, 2 * right + 0, rr)),
+                        __ldg(d.edge_static + edge_static_index(d, bd, 2 * right + 1, rr)), 0.f, 0.f};
+            };
+            L[0] = side(b, west ? 1 : 0);
+            E[0] = side(b, 1);
+            Q[0] = side(full ? b + 1 : b, east && full ? 0 : 1);
+            if (west && d.bnd[0] == 0) L[0].hu = -L[0].hu;
+            if (east && d.bnd[1] == 0) Q[0].hu = -Q[0].hu;
         } else {
             load_cells<1>(d, in, rr, x0w - 1, L);
             load_cells<1>(d, in, rr, x0w, E);
-        }
-        if (EDGES && ein != nullptr && x0w + kEdgeStrip < d.cols) {
-            Q[0] = {__ldg(ein + edge_index(d, b + 1, 3, rr)), __ldg(ein + edge_index(d, b + 1, 4, rr)),
-                    __ldg(ein + edge_index(d, b + 1, 5, rr)), __ldg(d.edge_static + edge_static_index(d, b + 1, 2, rr)),
-                    __ldg(d.edge_static + edge_static_index(d, b + 1, 3, rr)), 0.f, 0.f};
-        } else {
             load_cells<1>(d, in, rr, x0w + kWarp * 2, Q);
         }
         CellT<float> l{L[0].h, L[0].hu, L[0].hv, L[0].z, L[0].nm, 0.f, 0.f};
@@ -660,7 +664,7 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
             return MarchPlan{pl.s, pl.snap, pl.dt, pl.go};
         };
         const bool went = r0 < d.upd_hi
-                              ? march_pair<M, true, MASKED, true, !P<M>::kExact>(d, p.in, p.out, plan_fn, p.ctl, r0, r1,
+                              ? march_pair<M, true, MASKED, true>(d, p.in, p.out, plan_fn, p.ctl, r0, r1,
                                                                   strip * kWarp * 2, s_warp[wib], acc,
                                                                   d.edge[0] ? p.par : -1)
                               : plan_fn().go != 0;
@@ -680,7 +684,7 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
         warp_end_step(p.ctl, &p.slots[gw], s_warp[wib].old, p.par, in.pos.steps, gw % kMaxStripes, a);
     } else {
         if (r0 < d.upd_hi)
-            march_pair<M, false, MASKED, true, false>(d, p.in, p.out, [&]() { return MarchPlan{p.s, -1, 0.0, 1}; }, nullptr, r0,
+            march_pair<M, false, MASKED, true>(d, p.in, p.out, [&]() { return MarchPlan{p.s, -1, 0.0, 1}; }, nullptr, r0,
                                          r1, strip * kWarp * 2, s_warp[wib], acc);
     }
 }
@@ -730,7 +734,7 @@ __device__ __forceinline__ void ensemble_item(const MemberDev& md, int slot, int
     const StateOut out{md.buf[par ^ 1][0], md.buf[par ^ 1][1], md.buf[par ^ 1][2], md.pitch};
     StepAccum acc;
     acc.zero();
-    const bool went = r0 < md.d.rows ? march_pair<M, true, MASKED, false, !P<M>::kExact>(md.d, in, out, plan_fn, md.ctl,
+    const bool went = r0 < md.d.rows ? march_pair<M, true, MASKED, false>(md.d, in, out, plan_fn, md.ctl,
                                                                    r0, r1, strip * kWarp * 2, sm, acc,
                                                                    md.d.edge[0] ? par : -1)
                                      : plan_fn().go != 0;
