@@ -15,7 +15,7 @@
 // only for h > dry; hypot only for a non-zero norm; HLL speed min/max route to
 // the selected argument; the flux select follows the taken branch.
 //
-// Two kernels per reverse step:
+// One kernel per reverse step, adj_march_kernel; or two, where lam_out aliases lam:
 //   adj_cell_kernel  recomputes the cell's forward update (its four faces) and
 //                    reverses the pointwise part (rain, clip, friction, masks):
 //                    lambda_upd = dL/d(upd) per cell, plus the n^2 and rain
@@ -26,9 +26,44 @@
 //                    faces' contributions into lambda = lambda_upd + their sum.
 #pragma once
 
+#include "swe_pair.cuh"
 #include "swe_step.cuh"
 
 namespace swe {
+
+// Plain arithmetic on one value and on a pair of cells (packed f32x2; the
+// compiler fuses multiply-adds of both).  The reverse needs no rounding order.
+struct V2 {
+    float2 v;
+};
+__device__ __forceinline__ V2 operator+(V2 a, V2 b) { return {__fadd2_rn(a.v, b.v)}; }
+__device__ __forceinline__ V2 operator-(V2 a) { return {{-a.v.x, -a.v.y}}; }
+__device__ __forceinline__ V2 operator-(V2 a, V2 b) { return a + (-b); }
+__device__ __forceinline__ V2 operator*(V2 a, V2 b) { return {__fmul2_rn(a.v, b.v)}; }
+__device__ __forceinline__ V2 operator*(float a, V2 b) { return V2{splat(a)} * b; }
+__device__ __forceinline__ V2 sel(B2 p, V2 a, V2 b) { return {sel(p, a.v, b.v)}; }
+__device__ __forceinline__ B2 gt(V2 a, float b) { return {a.v.x > b, a.v.y > b}; }
+__device__ __forceinline__ B2 ge(V2 a, V2 b) { return {a.v.x >= b.v.x, a.v.y >= b.v.y}; }
+__device__ __forceinline__ V2 vmax(V2 a, V2 b) { return {vmax(a.v, b.v)}; }
+__device__ __forceinline__ V2 vmin(V2 a, V2 b) { return {vmin(a.v, b.v)}; }
+__device__ __forceinline__ V2 vabs(V2 a) { return {vabs(a.v)}; }
+template <class T>
+__device__ __forceinline__ T lit(float a);
+template <>
+__device__ __forceinline__ float lit<float>(float a) { return a; }
+template <>
+__device__ __forceinline__ V2 lit<V2>(float a) { return {splat(a)}; }
+// A flag per cell of T.
+template <class T>
+struct FlagOf {
+    using type = bool;
+};
+template <>
+struct FlagOf<V2> {
+    using type = B2;
+};
+template <class T>
+using Flag = typename FlagOf<T>::type;
 
 struct AdjConsts {
     float g, half_g, dry, dx, dy;
@@ -36,46 +71,48 @@ struct AdjConsts {
 
 // The reverse step needs derivative values to float accuracy, not the forward's
 // rounding: approximate division, square root and power (a few ulp) keep it cheap.
-__device__ __forceinline__ float adiv(float a, float b) { return __fdividef(a, b); }
+// A reciprocal is formed once per divisor and multiplied.
+__device__ __forceinline__ float arcp(float a) { return rcp_approx(a); }
+__device__ __forceinline__ V2 arcp(V2 a) { return {{rcp_approx(a.v.x), rcp_approx(a.v.y)}}; }
 __device__ __forceinline__ float asqrt(float a) {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
     return r;
 }
+__device__ __forceinline__ V2 asqrt(V2 a) { return {{asqrt(a.v.x), asqrt(a.v.y)}}; }
 __device__ __forceinline__ float apow(float x, float e) {  // x > 0
     float l, r;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(l * e));
     return r;
 }
+__device__ __forceinline__ V2 apow(V2 x, float e) { return {{apow(x.v.x, e), apow(x.v.y, e)}}; }
 
-// One side of a face: the cell's state, its velocities (m/h where h > dry, else
-// 0: computed once per cell and shared by the cell's four faces) and whether it
-// is active.
-struct FaceIn {
-    float h, hu, hv, z, u, v;
-    bool act;
+// One side of a face: the cell's depth and bed, its velocities (m/h where h >
+// dry, else 0) and 1/h, computed once per cell and shared by its four faces, and
+// whether it is active.
+template <class T>
+struct FaceInT {
+    T h, z, u, v, rh;
+    Flag<T> act;
 };
+using FaceIn = FaceInT<float>;
 
 __device__ __forceinline__ FaceIn face_in(float h, float hu, float hv, float z, bool act, float dry) {
     const bool wet = h > dry;
-    return {h, hu, hv, z, wet ? adiv(hu, h) : 0.f, wet ? adiv(hv, h) : 0.f, act};
+    const float rh = arcp(h);
+    return {h, z, wet ? hu * rh : 0.f, wet ? hv * rh : 0.f, rh, act};
 }
 
 __device__ __forceinline__ FaceIn face_in(const Cell& c, float dry) {
     return face_in(c.h, c.hu, c.hv, c.z, active(c.nm), dry);
 }
 
-// The mirrored copy of a cell across a wall: the normal momentum and velocity change sign.
+// The mirrored copy of a cell across a wall: the normal velocity changes sign.
 template <int AXIS>
 __device__ __forceinline__ FaceIn mirror(FaceIn c) {
-    if (AXIS == 1) {
-        c.hu = -c.hu;
-        c.u = -c.u;
-    } else {
-        c.hv = -c.hv;
-        c.v = -c.v;
-    }
+    if (AXIS == 1) c.u = -c.u;
+    else c.v = -c.v;
     return c;
 }
 
@@ -97,8 +134,9 @@ __device__ void adj_face_fwd(FaceIn lo, FaceIn hi, const AdjConsts& k, float F[3
     const float uL = L.u, vL = L.v, uR = R.u, vR = R.v;
     const float XL = HL * uL, YL = HL * vL, XR = HR * uR, YR = HR * vR;
     const float nL = AXIS == 1 ? XL : YL, nR = AXIS == 1 ? XR : YR;
-    const float unL = HL > k.dry ? adiv(nL, HL) : 0.f, unR = HR > k.dry ? adiv(nR, HR) : 0.f;
-    const float tL = HL > k.dry ? adiv(YL, HL) : 0.f, tR = HR > k.dry ? adiv(YR, HR) : 0.f;
+    const float rHL = arcp(HL), rHR = arcp(HR);
+    const float unL = HL > k.dry ? nL * rHL : 0.f, unR = HR > k.dry ? nR * rHR : 0.f;
+    const float tL = HL > k.dry ? YL * rHL : 0.f, tR = HR > k.dry ? YR * rHR : 0.f;
     const float cL = asqrt(k.g * HL), cR = asqrt(k.g * HR);
     const float sL = fminf(unL - cL, unR - cR), sR = fmaxf(unL + cL, unR + cR);
     const float pL = k.half_g * HL * HL, pR = k.half_g * HR * HR;
@@ -112,165 +150,129 @@ __device__ void adj_face_fwd(FaceIn lo, FaceIn hi, const AdjConsts& k, float F[3
     }
     const float UL[3] = {HL, XL, YL}, UR[3] = {HR, XR, YR};
     const float spread = sR - sL;
-    const float den = spread > kHllEps ? spread : 1.f;
+    const float rden = arcp(spread > kHllEps ? spread : 1.f);
     for (int q = 0; q < 3; ++q) {
-        const float m = adiv(sR * fL[q] - sL * fR[q] + sL * sR * (UR[q] - UL[q]), den);
+        const float m = (sR * fL[q] - sL * fR[q] + sL * sR * (UR[q] - UL[q])) * rden;
         F[q] = sL >= 0.f ? fL[q] : (sR <= 0.f ? fR[q] : m);
     }
     clo = k.half_g * (L.h * L.h - HL * HL);
     chi = k.half_g * (R.h * R.h - HR * HR);
 }
 
-// VJP of one face: given dL/dF (3), dL/dcorr_lo, dL/dcorr_hi, return dL/d(h, hu, hv)
-// of the lo cell and of the hi cell (after undoing the wall mirroring).
-template <int AXIS>
-__device__ void adj_face_vjp(FaceIn lo, FaceIn hi, const AdjConsts& k, const float lF[3], float lclo,
-                             float lchi, float dlo[3], float dhi[3]) {
-    dlo[0] = dlo[1] = dlo[2] = 0.f;
-    dhi[0] = dhi[1] = dhi[2] = 0.f;
-    if (!(lo.act || hi.act)) return;
-    const bool hi_wall = lo.act && !hi.act, lo_wall = !lo.act && hi.act;
-    FaceIn L = lo, R = hi;
-    if (hi_wall) {
-        R = mirror<AXIS>(lo);
-    } else if (lo_wall) {
-        L = mirror<AXIS>(hi);
-    }
-    // ---- forward, keeping what the reverse needs ----
-    const float zf = fmaxf(L.z, R.z);
-    const float aL = L.h + L.z - zf, aR = R.h + R.z - zf;
-    const float HL = fmaxf(aL, 0.f), HR = fmaxf(aR, 0.f);
-    const bool dL = L.h > k.dry, dR = R.h > k.dry;
-    const float uL = L.u, vL = L.v, uR = R.u, vR = R.v;
-    const float XL = HL * uL, YL = HL * vL, XR = HR * uR, YR = HR * vR;
-    const float nL = AXIS == 1 ? XL : YL, nR = AXIS == 1 ? XR : YR;
-    const bool wL = HL > k.dry, wR = HR > k.dry;
-    const float unL = wL ? adiv(nL, HL) : 0.f, unR = wR ? adiv(nR, HR) : 0.f;
-    const float tL = wL ? adiv(YL, HL) : 0.f, tR = wR ? adiv(YR, HR) : 0.f;
-    const float cL = asqrt(k.g * HL), cR = asqrt(k.g * HR);
-    const float aminL = unL - cL, aminR = unR - cR, amaxL = unL + cL, amaxR = unR + cR;
-    const float sL = fminf(aminL, aminR), sR = fmaxf(amaxL, amaxR);
-    const float pL = k.half_g * HL * HL, pR = k.half_g * HR * HR;
-    float fL[3], fR[3];
-    if (AXIS == 1) {
-        fL[0] = XL; fL[1] = XL * unL + pL; fL[2] = XL * tL;
-        fR[0] = XR; fR[1] = XR * unR + pR; fR[2] = XR * tR;
-    } else {
-        fL[0] = YL; fL[1] = XL * unL; fL[2] = YL * unL + pL;
-        fR[0] = YR; fR[1] = XR * unR; fR[2] = YR * unR + pR;
-    }
-    const float UL[3] = {HL, XL, YL}, UR[3] = {HR, XR, YR};
-    const float spread = sR - sL;
-    const bool use_spread = spread > kHllEps;
-    const float den = use_spread ? spread : 1.f;
-    const bool take_l = sL >= 0.f, take_r = !take_l && sR <= 0.f;
-    // ---- reverse ----
-    float lfL[3] = {0.f, 0.f, 0.f}, lfR[3] = {0.f, 0.f, 0.f};
-    float lUL[3] = {0.f, 0.f, 0.f}, lUR[3] = {0.f, 0.f, 0.f};
-    float lsL = 0.f, lsR = 0.f;
-    if (take_l) {
-        for (int q = 0; q < 3; ++q) lfL[q] = lF[q];
-    } else if (take_r) {
-        for (int q = 0; q < 3; ++q) lfR[q] = lF[q];
-    } else {
-        float lden = 0.f;
-        for (int q = 0; q < 3; ++q) {
-            const float dU = UR[q] - UL[q];
-            const float m = adiv(sR * fL[q] - sL * fR[q] + sL * sR * dU, den);
-            const float lN = adiv(lF[q], den);
-            lden -= m * lN;
-            lsR += (fL[q] + sL * dU) * lN;
-            lsL += (-fR[q] + sR * dU) * lN;
-            lfL[q] += sR * lN;
-            lfR[q] -= sL * lN;
-            lUR[q] += sL * sR * lN;
-            lUL[q] -= sL * sR * lN;
+// One side of a face in the reverse: given the weights of its flux (a0 mass, an
+// normal, at tangential momentum), of its reconstructed state (uH, uN, uT), of its
+// normal velocity and celerity in the wave speeds (lun, lc) and of its pressure
+// correction, dL/d(h, normal momentum, tangential momentum) of the cell.
+//
+// With N = H n and T = H t the momenta of the reconstructed depth H, the flux is
+// (N, N un + g H^2/2, N tt), where un and tt are the cell's velocities n and t
+// where H > dry and zero elsewhere (the forward recomputes them as N/H and T/H).
+// Reversed through (H, n, t) no term is divided by H.
+template <class T>
+struct AdjSide {
+    T h, n, t, rh;     // the cell: depth, normal and tangential velocity, 1/h
+    T H, un, tt, N, c; // reconstructed depth, velocities in the flux, N, celerity
+    Flag<T> up, wet, deep;  // H > 0, H > dry, h > dry
+};
+
+template <class T>
+__device__ __forceinline__ void adj_side(const AdjConsts& k, const AdjSide<T>& s, T a0, T an, T at, T uH, T uN, T uT,
+                                         T lun, T lc, T lcorr, T out[3]) {
+    const T zero = lit<T>(0.f);
+    const T lN = a0 + s.un * an + s.tt * at + uN;
+    const T ln = s.H * lN + sel(s.wet, s.N * an + lun, zero);
+    const T lt = s.H * uT + sel(s.wet, s.N * at, zero);
+    const T lH = uH + s.n * lN + s.t * uT + k.g * (s.H * (an - lcorr)) +
+                 sel(gt(s.c, 0.f), 0.5f * k.g * (arcp(s.c) * lc), zero);
+    const T lh = k.g * (s.h * lcorr) + sel(s.up, lH, zero);  // the bed is held fixed
+    out[1] = sel(s.deep, ln * s.rh, zero);
+    out[2] = sel(s.deep, lt * s.rh, zero);
+    out[0] = lh - (s.n * out[1] + s.t * out[2]);
+}
+
+// VJP of one face (or of a pair of faces): given dL/dF (3), dL/dcorr_lo, dL/dcorr_hi,
+// return dL/d(h, hu, hv) of the lo cell and of the hi cell (after undoing the
+// wall mirroring).  No branch: a supercritical face's weights are those of the
+// flux it takes, selected per cell.
+template <int AXIS, bool MASKED, class T>
+__device__ __forceinline__ void adj_face_vjp(const FaceInT<T>& lo, const FaceInT<T>& hi, const AdjConsts& k,
+                                             const T lF[3], T lclo, T lchi, T dlo[3], T dhi[3]) {
+    constexpr int in = AXIS == 1 ? 1 : 2, it = 3 - in;  // normal and tangential momentum component
+    const T zero = lit<T>(0.f), one = lit<T>(1.f);
+    const Flag<T> hi_wall = lo.act & !hi.act, lo_wall = !lo.act & hi.act, relevant = lo.act | hi.act;
+    auto side = [&](const FaceInT<T>& f, const FaceInT<T>& across, const Flag<T>& wall, T zf) {
+        AdjSide<T> s;
+        s.h = f.h;
+        s.n = AXIS == 1 ? f.u : f.v;
+        s.t = AXIS == 1 ? f.v : f.u;
+        s.rh = f.rh;
+        T z = f.z;
+        if constexpr (MASKED) {  // the mirrored copy of the cell across a wall
+            s.h = sel(wall, across.h, s.h);
+            s.n = sel(wall, -(AXIS == 1 ? across.u : across.v), s.n);
+            s.t = sel(wall, AXIS == 1 ? across.v : across.u, s.t);
+            s.rh = sel(wall, across.rh, s.rh);
+            z = sel(wall, across.z, z);
         }
-        if (use_spread) {
-            lsR += lden;
-            lsL -= lden;
-        }
+        const T a = s.h + z - zf;
+        s.H = vmax(a, zero);
+        s.up = gt(a, 0.f);
+        s.wet = gt(s.H, k.dry);
+        s.deep = gt(s.h, k.dry);
+        s.un = sel(s.wet, s.n, zero);
+        s.tt = sel(s.wet, s.t, zero);
+        s.N = s.H * s.n;
+        s.c = asqrt(k.g * s.H);
+        return s;
+    };
+    T zf = vmax(lo.z, hi.z);
+    if constexpr (MASKED) zf = vmax(sel(lo_wall, hi.z, lo.z), sel(hi_wall, lo.z, hi.z));
+    const AdjSide<T> L = side(lo, hi, lo_wall, zf), R = side(hi, lo, hi_wall, zf);
+    const T aminL = L.un - L.c, aminR = R.un - R.c, amaxL = L.un + L.c, amaxR = R.un + R.c;
+    const T sL = vmin(aminL, aminR), sR = vmax(amaxL, amaxR);
+    const T spread = sR - sL;
+    const Flag<T> use_spread = gt(spread, kHllEps);
+    const T rden = arcp(sel(use_spread, spread, one));
+    const T s01 = sL * sR;
+    const Flag<T> take_l = ge(sL, zero), take_r = !take_l & ge(zero, sR), middle = !(take_l | take_r);
+    // Weights of the two sides' fluxes and of the state jump in the face's flux.
+    const T wl = sel(middle, sR * rden, sel(take_l, one, zero));
+    const T wr = sel(middle, -(sL * rden), sel(take_l, zero, sel(take_r, one, zero)));
+    const T wu = sel(middle, s01 * rden, zero);
+    const T f[3] = {lF[0], lF[in], lF[it]};
+    const T fL[3] = {L.N, L.N * L.un + k.half_g * (L.H * L.H), L.N * L.tt};
+    const T fR[3] = {R.N, R.N * R.un + k.half_g * (R.H * R.H), R.N * R.tt};
+    const T dU[3] = {R.H - L.H, R.N - L.N, R.H * R.t - L.H * L.t};
+    T lsL = zero, lsR = zero, lden = zero;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        lden = lden + (wl * fL[q] + wr * fR[q] + wu * dU[q]) * f[q];
+        lsR = lsR + (fL[q] + sL * dU[q]) * f[q];
+        lsL = lsL + (sR * dU[q] - fR[q]) * f[q];
     }
-    // corrections: half_g (h^2 - H^2) on each side
-    float lLh = k.g * L.h * lclo, lRh = k.g * R.h * lchi;
-    float lHL = lUL[0] - k.g * HL * lclo, lHR = lUR[0] - k.g * HR * lchi;
-    float lXL = lUL[1], lYL = lUL[2], lXR = lUR[1], lYR = lUR[2];
-    float lunL = 0.f, lunR = 0.f, ltL = 0.f, ltR = 0.f, lpL = 0.f, lpR = 0.f;
-    if (AXIS == 1) {
-        lXL += lfL[0] + unL * lfL[1] + tL * lfL[2];
-        lunL += XL * lfL[1];
-        lpL += lfL[1];
-        ltL += XL * lfL[2];
-        lXR += lfR[0] + unR * lfR[1] + tR * lfR[2];
-        lunR += XR * lfR[1];
-        lpR += lfR[1];
-        ltR += XR * lfR[2];
-    } else {
-        lYL += lfL[0] + unL * lfL[2];
-        lXL += unL * lfL[1];
-        lunL += XL * lfL[1] + YL * lfL[2];
-        lpL += lfL[2];
-        lYR += lfR[0] + unR * lfR[2];
-        lXR += unR * lfR[1];
-        lunR += XR * lfR[1] + YR * lfR[2];
-        lpR += lfR[2];
-    }
-    lHL += k.g * HL * lpL;
-    lHR += k.g * HR * lpR;
-    // wave speeds: min/max route to the selected argument
-    float lcL = 0.f, lcR = 0.f;
-    if (aminL <= aminR) { lunL += lsL; lcL -= lsL; } else { lunR += lsL; lcR -= lsL; }
-    if (amaxL >= amaxR) { lunL += lsR; lcL += lsR; } else { lunR += lsR; lcR += lsR; }
-    if (cL > 0.f) lHL += adiv(0.5f * k.g, cL) * lcL;
-    if (cR > 0.f) lHR += adiv(0.5f * k.g, cR) * lcR;
-    // un = n / H, t = Y / H (for H > dry)
-    float lnL = 0.f, lnR = 0.f;
-    if (wL) {
-        lnL += adiv(lunL, HL);
-        lHL -= adiv(unL, HL) * lunL;
-        if (AXIS == 1) {
-            lYL += adiv(ltL, HL);
-            lHL -= adiv(tL, HL) * ltL;
-        }
-    }
-    if (wR) {
-        lnR += adiv(lunR, HR);
-        lHR -= adiv(unR, HR) * lunR;
-        if (AXIS == 1) {
-            lYR += adiv(ltR, HR);
-            lHR -= adiv(tR, HR) * ltR;
-        }
-    }
-    if (AXIS == 1) { lXL += lnL; lXR += lnR; } else { lYL += lnL; lYR += lnR; }
-    // X = H u, Y = H v
-    lHL += uL * lXL + vL * lYL;
-    lHR += uR * lXR + vR * lYR;
-    const float luL = HL * lXL, lvL = HL * lYL, luR = HR * lXR, lvR = HR * lYR;
-    // H = max(h + z - zf, 0) with the bed held fixed
-    if (aL > 0.f) lLh += lHL;
-    if (aR > 0.f) lRh += lHR;
-    // u = hu / h, v = hv / h (for h > dry)
-    float gL[3] = {lLh, 0.f, 0.f}, gR[3] = {lRh, 0.f, 0.f};
-    if (dL) {
-        gL[1] = adiv(luL, L.h);
-        gL[2] = adiv(lvL, L.h);
-        gL[0] -= adiv(uL * luL + vL * lvL, L.h);
-    }
-    if (dR) {
-        gR[1] = adiv(luR, R.h);
-        gR[2] = adiv(lvR, R.h);
-        gR[0] -= adiv(uR * luR + vR * lvR, R.h);
-    }
-    // undo the wall mirroring: the mirrored side's gradient belongs to the active cell
-    const int nq = AXIS == 1 ? 1 : 2;
-    if (hi_wall) {
-        for (int q = 0; q < 3; ++q) dlo[q] = gL[q] + (q == nq ? -gR[q] : gR[q]);
-    } else if (lo_wall) {
-        for (int q = 0; q < 3; ++q) dhi[q] = gR[q] + (q == nq ? -gL[q] : gL[q]);
-    } else {
-        for (int q = 0; q < 3; ++q) {
-            dlo[q] = gL[q];
-            dhi[q] = gR[q];
+    lden = sel(use_spread, lden, zero);
+    const T live = sel(middle, rden, zero);
+    lsR = (lsR - lden) * live;
+    lsL = (lsL + lden) * live;
+    // Wave speeds: min/max route to the selected argument.
+    const Flag<T> minL = ge(aminR, aminL), maxL = ge(amaxL, amaxR);
+    const T lsLL = sel(minL, lsL, zero), lsLR = sel(minL, zero, lsL);
+    const T lsRL = sel(maxL, lsR, zero), lsRR = sel(maxL, zero, lsR);
+    T gL[3], gR[3];
+    adj_side(k, L, wl * f[0], wl * f[1], wl * f[2], -(wu * f[0]), -(wu * f[1]), -(wu * f[2]), lsLL + lsRL, lsRL - lsLL,
+             lclo, gL);
+    adj_side(k, R, wr * f[0], wr * f[1], wr * f[2], wu * f[0], wu * f[1], wu * f[2], lsLR + lsRR, lsRR - lsLR, lchi, gR);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int comp = q == 0 ? 0 : (q == 1 ? in : it);
+        if constexpr (MASKED) {
+            // The mirrored side's gradient belongs to the active cell.
+            const T mR = q == 1 ? -gR[q] : gR[q], mL = q == 1 ? -gL[q] : gL[q];
+            dlo[comp] = sel(relevant, sel(lo_wall, zero, gL[q] + sel(hi_wall, mR, zero)), zero);
+            dhi[comp] = sel(relevant, sel(hi_wall, zero, gR[q] + sel(lo_wall, mL, zero)), zero);
+        } else {
+            dlo[comp] = gL[q];
+            dhi[comp] = gR[q];
         }
     }
 }
@@ -299,7 +301,10 @@ __device__ __forceinline__ Cell adj_load(const DomainDev& d, const StateView& s,
 
 // The forward update of cell (r, c) from its four faces: upd (3) before the
 // pointwise part.
-__device__ void adj_cell_update(const AdjLaunch& p, int r, int c, float upd[3]) {
+struct AdjUpd {
+    float u0, u1, u2;
+};
+__device__ __noinline__ inline AdjUpd adj_cell_update(const AdjLaunch& p, int r, int c) {
     const DomainDev& d = p.d;
     const float dry = p.k.dry;
     const FaceIn C = face_in(adj_load(d, p.in, r, c), dry);
@@ -310,7 +315,9 @@ __device__ void adj_cell_update(const AdjLaunch& p, int r, int c, float upd[3]) 
     adj_face_fwd<1>(C, E, p.k, Fr, cr_lo, cr_hi);
     adj_face_fwd<0>(S, C, p.k, Fb, cb_lo, cb_hi);
     adj_face_fwd<0>(C, N, p.k, Ft, ct_lo, ct_hi);
-    const float U[3] = {C.h, C.hu, C.hv};
+    const Cell own = adj_load(d, p.in, r, c);
+    const float U[3] = {own.h, own.hu, own.hv};
+    float upd[3];
     for (int q = 0; q < 3; ++q) {
         const float xl = Fr[q] + (q == 1 ? cr_lo : 0.f);
         const float xr = Fl[q] + (q == 1 ? cl_hi : 0.f);
@@ -318,76 +325,80 @@ __device__ void adj_cell_update(const AdjLaunch& p, int r, int c, float upd[3]) 
         const float yt = Fb[q] + (q == 2 ? cb_hi : 0.f);
         upd[q] = U[q] - p.s.dt * ((xl - xr) * p.rdx + (yb - yt) * p.rdy);
     }
+    return {upd[0], upd[1], upd[2]};
 }
 
-// The cell update before the pointwise part, rebuilt from the step's own output
-// U_{k+1} = (h1, hu1, hv1) of an active cell instead of from its four faces.
-// The momenta invert the semi-implicit friction: with a = dt g n^2 max(h,dry)^(-7/3),
-// q = upd/(1 + a|upd|) gives upd = q/(1 - a|q|).  Returns false (rebuild from the
-// faces instead) where that inversion loses precision (a|q| > 0.999, i.e. friction
-// dividing the momentum by more than 1000).  For dry or clipped cells only the
-// depth part is needed: the momentum outputs are zero and carry no gradient.
-__device__ __forceinline__ bool adj_upd_from_next(const AdjLaunch& p, int r, int c, float n2, float upd[3]) {
-    const int64_t o = (int64_t)r * p.next.pitch + c;
-    const float h1 = p.next.h[o];
-    upd[0] = h1;  // only the sign of upd0 + rain and h itself are used below
-    upd[1] = upd[2] = 0.f;
-    if (!(h1 > p.k.dry)) return true;
-    const float q1 = p.next.hu[o], q2 = p.next.hv[o];
-    const float aq = p.s.dt_g * n2 * apow(h1, -7.0f / 3.0f) * asqrt(q1 * q1 + q2 * q2);
-    if (!(aq <= 0.999f)) return false;
-    const float den = adiv(1.f, 1.f - aq);
-    upd[1] = q1 * den;
-    upd[2] = q2 * den;
-    return true;
-}
-
-// Reverse of the pointwise part of cell (r, c) (rain, clip, friction, masks):
-// returns lupd = dL/d(upd) (zero for an inactive cell); when `owned`, also adds
-// the cell's dL/d(n^2) to grad_n2 and its rain-scale term to *rain_acc.
-template <bool NEXT>
-__device__ __forceinline__ void adj_cell_at(const AdjLaunch& p, int r, int c, bool owned, double* rain_acc,
-                                            float lu[3]) {
+// Reverse of the pointwise part of an active cell (rain, clip, friction, masks):
+// lu = dL/d(upd); when `owned`, also adds the cell's dL/d(n^2) to grad_n2 and its
+// rain-scale term to *rain_acc.
+//
+// With NEXT the cell update before the pointwise part is rebuilt from the step's
+// own output U_{k+1} = (h1, q1, q2) instead of from the cell's four faces.  The
+// momenta invert the semi-implicit friction: with a = dt g n^2 max(h,dry)^(-7/3),
+// q = upd/(1 + a|upd|) gives upd = q/(1 - a|q|).  Where that inversion loses
+// precision (a|q| > 0.999, i.e. friction dividing the momentum by more than 1000)
+// the update is rebuilt from the faces.  For dry or clipped cells only the depth
+// part is needed: the momentum outputs are zero and carry no gradient.
+template <bool NEXT, bool MASKED>
+__device__ __forceinline__ void adj_pointwise(const AdjLaunch& p, int r, int c, V2 nm, const V2 lam[3], const V2 next[3],
+                                              B2 live, B2 owned, double* rain_acc, V2 lu[3]) {
     const DomainDev& d = p.d;
-    const float nm = d.nm[(int64_t)r * d.spitch + c];
-    lu[0] = lu[1] = lu[2] = 0.f;
-    if (!active(nm)) return;
-    const float mult = d.mult ? d.mult[(int64_t)r * d.spitch + c] : 1.f;
-    float upd[3];
-    // upd[0] below is the depth after the rain (before the clip).
-    if (!(NEXT && adj_upd_from_next(p, r, c, fabsf(nm), upd))) {
-        adj_cell_update(p, r, c, upd);
-        upd[0] += p.s.dt_rain * mult;
+    const V2 zero = lit<V2>(0.f), n2 = MASKED ? vabs(nm) : nm;
+    V2 mult = lit<V2>(1.f);
+    if (d.mult) {
+        if (live.x) mult.v.x = d.mult[(int64_t)r * d.spitch + c];
+        if (live.y) mult.v.y = d.mult[(int64_t)r * d.spitch + c + 1];
     }
-    const float h = fmaxf(upd[0], 0.f);
-    const float norm = asqrt(upd[1] * upd[1] + upd[2] * upd[2]);
-    const float m = fmaxf(h, p.k.dry);
-    const float pw = apow(m, -7.0f / 3.0f);
-    const float n2 = fabsf(nm);
-    const float fr = p.s.dt_g * n2 * norm * pw;
-    const float den = 1.f + fr;
-    const float rden = adiv(1.f, den);
-    const float qx = upd[1] * rden, qy = upd[2] * rden;
-    const bool wet = h > p.k.dry;
-    const int64_t li = (int64_t)r * p.lam.pitch + c;
-    const float lqx = wet ? p.lam.hu[li] : 0.f, lqy = wet ? p.lam.hv[li] : 0.f;
-    float lh = p.lam.h[li];
-    const float lden = -(lqx * qx + lqy * qy) * rden;
-    float lu1 = lqx * rden, lu2 = lqy * rden;
-    if (norm > 0.f) {
-        const float lnorm = lden * p.s.dt_g * n2 * pw;
-        lu1 += adiv(lnorm * upd[1], norm);
-        lu2 += adiv(lnorm * upd[2], norm);
+    V2 u0 = zero, u1 = zero, u2 = zero;  // u0: the depth after the rain (before the clip)
+    B2 rebuild = live;
+    if constexpr (NEXT) {
+        u0 = next[0];
+        const B2 wet = gt(u0, p.k.dry);
+        const V2 pw = apow(vmax(u0, lit<V2>(p.k.dry)), -7.0f / 3.0f);
+        const V2 aq = p.s.dt_g * n2 * pw * asqrt(next[1] * next[1] + next[2] * next[2]);
+        const V2 den = arcp(lit<V2>(1.f) - aq);
+        u1 = sel(wet, next[1] * den, zero);
+        u2 = sel(wet, next[2] * den, zero);
+        rebuild = live & wet & B2{!(aq.v.x <= 0.999f), !(aq.v.y <= 0.999f)};
     }
-    if (h > p.k.dry) lh += adiv(lden * fr * (-7.0f / 3.0f), h);
-    const float lu0 = upd[0] > 0.f ? lh : 0.f;
-    if (owned) {
-        p.grad_n2[(int64_t)r * d.cols + c] += lden * p.s.dt_g * norm * pw;
-        *rain_acc += (double)lu0 * (double)p.dt_rate * (double)mult;
+    if (rebuild.x) {
+        const AdjUpd t = adj_cell_update(p, r, c);
+        u0.v.x = t.u0 + p.s.dt_rain * mult.v.x;
+        u1.v.x = t.u1;
+        u2.v.x = t.u2;
     }
-    lu[0] = lu0;
-    lu[1] = lu1;
-    lu[2] = lu2;
+    if (rebuild.y) {
+        const AdjUpd t = adj_cell_update(p, r, c + 1);
+        u0.v.y = t.u0 + p.s.dt_rain * mult.v.y;
+        u1.v.y = t.u1;
+        u2.v.y = t.u2;
+    }
+    const V2 h = vmax(u0, zero);
+    const V2 pw = apow(vmax(h, lit<V2>(p.k.dry)), -7.0f / 3.0f);
+    const V2 norm = asqrt(u1 * u1 + u2 * u2);
+    const V2 a = p.s.dt_g * n2 * pw;
+    const V2 fr = a * norm;
+    const V2 rden = arcp(lit<V2>(1.f) + fr);
+    const V2 qx = u1 * rden, qy = u2 * rden;
+    const B2 wet = gt(h, p.k.dry);
+    const V2 lqx = sel(wet, lam[1], zero), lqy = sel(wet, lam[2], zero);
+    const V2 lden = -((lqx * qx + lqy * qy) * rden);
+    const V2 ln = sel(gt(norm, 0.f), lden * a * arcp(norm), zero);
+    const V2 lh = lam[0] + sel(wet, (-7.0f / 3.0f) * (lden * fr * arcp(h)), zero);
+    lu[0] = sel(live & gt(u0, 0.f), lh, zero);
+    lu[1] = sel(live, lqx * rden + ln * u1, zero);
+    lu[2] = sel(live, lqy * rden + ln * u2, zero);
+    const B2 add = owned & live;
+    const V2 gn = p.s.dt_g * (lden * norm * pw);
+    float* g = p.grad_n2 + (int64_t)r * d.cols + c;
+    if (add.x) {
+        g[0] += gn.v.x;
+        *rain_acc += (double)lu[0].v.x * (double)p.dt_rate * (double)mult.v.x;
+    }
+    if (add.y) {
+        g[1] += gn.v.y;
+        *rain_acc += (double)lu[0].v.y * (double)p.dt_rate * (double)mult.v.y;
+    }
 }
 
 // Adds a CTA's rain-scale gradient to the device scalar (one atomic per CTA).
@@ -405,18 +416,27 @@ __device__ __forceinline__ void adj_flush_rain(const AdjLaunch& p, double rain_a
 }
 
 template <int THREADS, bool NEXT>
-__global__ void __launch_bounds__(THREADS) adj_cell_kernel(const AdjLaunch p) {
+__global__ void __launch_bounds__(THREADS) adj_cell_kernel(const __grid_constant__ AdjLaunch p) {
     const DomainDev& d = p.d;
     const int64_t n = (int64_t)d.rows * d.cols;
     double rain_acc = 0.0;
     for (int64_t i = (int64_t)blockIdx.x * THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * THREADS) {
         const int r = (int)(i / d.cols), c = (int)(i - (int64_t)r * d.cols);
-        float lu[3];
-        adj_cell_at<NEXT>(p, r, c, true, &rain_acc, lu);
+        const int64_t li = (int64_t)r * p.lam.pitch + c, no = (int64_t)r * p.next.pitch + c;
+        auto one = [](float x) { return V2{{x, x}}; };
+        const float nm = d.nm[(int64_t)r * d.spitch + c];
+        const V2 lam[3] = {one(p.lam.h[li]), one(p.lam.hu[li]), one(p.lam.hv[li])};
+        V2 next[3] = {}, lu[3];
+        if constexpr (NEXT) {
+            next[0] = one(p.next.h[no]);
+            next[1] = one(p.next.hu[no]);
+            next[2] = one(p.next.hv[no]);
+        }
+        adj_pointwise<NEXT, true>(p, r, c, one(nm), lam, next, B2{active(nm), false}, B2{true, false}, &rain_acc, lu);
         const int64_t lo = (int64_t)r * p.lpitch + c;
-        p.lupd[0][lo] = lu[0];
-        p.lupd[1][lo] = lu[1];
-        p.lupd[2][lo] = lu[2];
+        p.lupd[0][lo] = lu[0].v.x;
+        p.lupd[1][lo] = lu[1].v.x;
+        p.lupd[2][lo] = lu[2].v.x;
     }
     adj_flush_rain<THREADS>(p, rain_acc);
 }
@@ -447,7 +467,7 @@ __device__ __forceinline__ void adj_face_at(const AdjLaunch& p, int rl, int cl, 
     for (int q = 0; q < 3; ++q) lF[q] = -a * ll[q] + a * lh[q];
     constexpr int nq = AXIS == 1 ? 1 : 2;
     float lo[3], hi[3];
-    adj_face_vjp<AXIS>(L, H, p.k, lF, -a * ll[nq], a * lh[nq], lo, hi);
+    adj_face_vjp<AXIS, true, float>(L, H, p.k, lF, -a * ll[nq], a * lh[nq], lo, hi);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
         dlo[q] = lo[q];
@@ -522,127 +542,217 @@ __global__ void __launch_bounds__(kAdjTW * kAdjTH) adj_face_tile_kernel(const Ad
     }
 }
 
-// The whole reverse step in one kernel, for lam_out not aliasing lam.  A CTA
-// of 256 threads takes a tile of 32 x 16 cells and stages, for the tile and its
-// one-cell halo ring (34 x 18 cells), each cell's state, velocities and
-// dL/d(upd) in shared memory (phase 0: the pointwise reverse of adj_cell_at;
-// halo cells are recomputed, but only the tile's own cells add to the n^2 and
-// rain-scale gradients).  Phase 1 evaluates every face of the tile once
-// (16 x 33 x-faces and 17 x 32 y-faces over the 256 threads) from the staged
-// cells; phase 2 gathers the four faces of each cell.  Reading the halo cells'
-// lam while neighbouring tiles write lam_out is why the two must not alias.
-constexpr int kFTW = 32, kFTH = 16, kFHW = kFTW + 2, kFHH = kFTH + 2, kFThreads = 256;
+// ---------------------------------------------------------------------------
+// The whole reverse step in one kernel, for lam_out not aliasing lam
+// ---------------------------------------------------------------------------
+// A warp owns 60 columns and marches up a chunk of rows, two cells per lane
+// evaluated together (packed f32x2); lanes 0 and 31 hold the columns either side,
+// so that every face of the strip lies within the warp.  A row's cells are reversed pointwise once
+// (dL/d(upd) in registers), its x-faces are evaluated between neighbouring lanes
+// and their two sides moved by shuffle, and the y-face above it is evaluated once,
+// its upper side carried to the next row.  Only the rows below and above the chunk
+// and the two outer columns are reversed twice; lam is read in a neighbour's rows
+// while that warp writes lam_out, which is why the two must not alias.
+//
+// The step is bound by instructions and their latency, not by memory (56 bytes
+// a cell): 18 warp instructions a cell, issued at 47 % by the 12 warps of an SM.
+// A CTA of 32 x 16 cells staged in shared memory, with a barrier between its three
+// phases and the face loop's last round mostly idle, took 9.9 us on 128^2, 17.2 on
+// 512^2 and 54 on 1024^2; this march takes 4.4, 11.4 and 33.7 us.
+constexpr int kMarchCols = 2 * kWarp - 4;
 
-struct AdjTileSmem {
-    float h[kFHH][kFHW], hu[kFHH][kFHW], hv[kFHH][kFHW], z[kFHH][kFHW], u[kFHH][kFHW], v[kFHH][kFHW];
-    float l[3][kFHH][kFHW];
-    float fx[kFTH][kFTW + 1][6];  // face left of tile column c: dlo (0..2), dhi (3..5)
-    float fy[kFTH + 1][kFTW][6];  // face below tile row r
-    unsigned char act[kFHH][kFHW];
+// What the faces of a pair of cells read of it, and its dL/d(upd).
+struct AdjCells {
+    FaceInT<V2> f;
+    V2 l[3];
 };
 
-__device__ __forceinline__ FaceIn staged(const AdjTileSmem& S, int hr, int hc) {
-    return {S.h[hr][hc], S.hu[hr][hc], S.hv[hr][hc], S.z[hr][hc], S.u[hr][hc], S.v[hr][hc], S.act[hr][hc] != 0};
+// The values a row's cells are built from, loaded one row ahead of their use.
+struct AdjRaw {
+    V2 h, hu, hv, z, nm;
+    V2 h1, q1, q2;  // U_{k+1}
+    V2 l0, l1, l2;  // dL/dU_{k+1}
+};
+
+// Two neighbouring elements of a plane: one 8-byte load where VEC (even column,
+// even pitch, 8-byte aligned plane), else two loads at the clamped columns.
+template <bool VEC>
+__device__ __forceinline__ V2 load2(const float* p, uint32_t row, int c0, int c1) {
+    if constexpr (VEC) return {__ldg(reinterpret_cast<const float2*>(p + row + c0))};
+    return {{__ldg(p + row + c0), __ldg(p + row + c1)}};
 }
 
-template <int AXIS>
-__device__ __forceinline__ void staged_face(const AdjTileSmem& S, const AdjConsts& k, int lr, int lc, int hr, int hc,
-                                            float a, float* out) {
-    constexpr int nq = AXIS == 1 ? 1 : 2;
-    float lF[3], lo[3], hi[3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) lF[q] = -a * S.l[q][lr][lc] + a * S.l[q][hr][hc];
-    adj_face_vjp<AXIS>(staged(S, lr, lc), staged(S, hr, hc), k, lF, -a * S.l[nq][lr][lc], a * S.l[nq][hr][hc], lo, hi);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        out[q] = lo[q];
-        out[3 + q] = hi[q];
-    }
-}
-
-template <bool NEXT>
-__global__ void __launch_bounds__(kFThreads) adj_tile_kernel(const AdjLaunch p) {
-    extern __shared__ __align__(16) unsigned char s_raw[];
-    AdjTileSmem& S = *reinterpret_cast<AdjTileSmem*>(s_raw);
+template <bool NEXT, bool VEC>
+__device__ __forceinline__ AdjRaw adj_raw(const AdjLaunch& p, int r, int c0, int c1) {
     const DomainDev& d = p.d;
-    const int tiles_x = (d.cols + kFTW - 1) / kFTW, tiles_y = (d.rows + kFTH - 1) / kFTH;
-    const float ax = p.s.dt * p.rdx, ay = p.s.dt * p.rdy;
-    double rain_acc = 0.0;
-    for (int tile = blockIdx.x; tile < tiles_x * tiles_y; tile += gridDim.x) {
-        const int c0 = (tile % tiles_x) * kFTW, r0 = (tile / tiles_x) * kFTH;
-        // Phase 0: the tile and its halo ring (ghost cells outside the grid carry no dL/d(upd)).
-        for (int i = threadIdx.x; i < kFHH * kFHW; i += kFThreads) {
-            const int hr = i / kFHW, hc = i - hr * kFHW;
-            const int r = r0 - 1 + hr, c = c0 - 1 + hc;
-            const FaceIn f = face_in(adj_load(d, p.in, r, c), p.k.dry);
-            S.h[hr][hc] = f.h;
-            S.hu[hr][hc] = f.hu;
-            S.hv[hr][hc] = f.hv;
-            S.z[hr][hc] = f.z;
-            S.u[hr][hc] = f.u;
-            S.v[hr][hc] = f.v;
-            S.act[hr][hc] = f.act ? 1 : 0;
-            float lu[3] = {0.f, 0.f, 0.f};
-            if (r >= 0 && r < d.rows && c >= 0 && c < d.cols) {
-                const bool owned = hr >= 1 && hr <= kFTH && hc >= 1 && hc <= kFTW;
-                adj_cell_at<NEXT>(p, r, c, owned, &rain_acc, lu);
-            }
-            S.l[0][hr][hc] = lu[0];
-            S.l[1][hr][hc] = lu[1];
-            S.l[2][hr][hc] = lu[2];
-        }
-        __syncthreads();
-        // Phase 1: x-faces exist for rows [0, rows) and columns [0, cols] (left of
-        // column c), y-faces for columns [0, cols) and rows [0, rows] (below row r).
-        constexpr int NX = kFTH * (kFTW + 1), NY = (kFTH + 1) * kFTW;
-        for (int f = threadIdx.x; f < NX + NY; f += kFThreads) {
-            if (f < NX) {
-                const int ty = f / (kFTW + 1), tx = f - ty * (kFTW + 1);
-                if (r0 + ty < d.rows && c0 + tx <= d.cols)
-                    staged_face<1>(S, p.k, ty + 1, tx, ty + 1, tx + 1, ax, S.fx[ty][tx]);
-            } else {
-                const int g = f - NX, ty = g / kFTW, tx = g - ty * kFTW;
-                if (c0 + tx < d.cols && r0 + ty <= d.rows)
-                    staged_face<0>(S, p.k, ty, tx + 1, ty + 1, tx + 1, ay, S.fy[ty][tx]);
-            }
-        }
-        __syncthreads();
-        // Phase 2: each cell of the tile adds its side of its four faces.
-        for (int i = threadIdx.x; i < kFTH * kFTW; i += kFThreads) {
-            const int ty = i / kFTW, tx = i - ty * kFTW;
-            const int r = r0 + ty, c = c0 + tx;
-            if (r >= d.rows || c >= d.cols) continue;
-            const float* fl = S.fx[ty][tx];
-            const float* fr = S.fx[ty][tx + 1];
-            const float* fb = S.fy[ty][tx];
-            const float* ft = S.fy[ty + 1][tx];
-            float g[3];
+    // 32-bit element offsets: planes hold fewer than 2^31 elements (checked on the host).
+    const uint32_t rr = (uint32_t)min(max(r, 0), d.rows - 1);
+    const uint32_t so = rr * (uint32_t)p.in.pitch, zo = rr * (uint32_t)d.spitch, lo = rr * (uint32_t)p.lam.pitch;
+    AdjRaw a;
+    a.h = load2<VEC>(p.in.h, so, c0, c1);
+    a.hu = load2<VEC>(p.in.hu, so, c0, c1);
+    a.hv = load2<VEC>(p.in.hv, so, c0, c1);
+    a.z = load2<VEC>(d.bed, zo, c0, c1);
+    a.nm = load2<VEC>(d.nm, zo, c0, c1);
+    a.l0 = load2<VEC>(p.lam.h, lo, c0, c1);
+    a.l1 = load2<VEC>(p.lam.hu, lo, c0, c1);
+    a.l2 = load2<VEC>(p.lam.hv, lo, c0, c1);
+    if constexpr (NEXT) {
+        const uint32_t no = rr * (uint32_t)p.next.pitch;
+        a.h1 = load2<VEC>(p.next.h, no, c0, c1);
+        a.q1 = load2<VEC>(p.next.hu, no, c0, c1);
+        a.q2 = load2<VEC>(p.next.hv, no, c0, c1);
+    }
+    return a;
+}
+
+// Cells (r, c) and (r, c + 1) from their loaded values: velocities, and the
+// pointwise reverse (rain, clip, friction, masks) of the cells inside the grid
+// (flags `in`); the others carry no dL/d(upd).  Owned cells add their n^2 and
+// rain-scale gradients.
+template <bool NEXT, bool MASKED, bool VEC>
+__device__ __forceinline__ AdjCells adj_cells(const AdjLaunch& p, AdjRaw a, int r, int c, B2 in, B2 owned,
+                                              double* rain_acc) {
+    const DomainDev& d = p.d;
+    if (VEC && (c < 0 || c >= d.cols)) {
+        auto edge = [&](V2& x) { c < 0 ? x.v.y = x.v.x : x.v.x = x.v.y; };
+        edge(a.h);
+        edge(a.hu);
+        edge(a.hv);
+        edge(a.z);
+        edge(a.nm);
+    }
+    V2 hu = a.hu, hv = a.hv;
+    // Ghost columns and rows (the loads are clamped to the grid): reflective edges mirror the normal momentum.
+    if (d.bnd[0] == 0) hu = {{c < 0 ? -hu.v.x : hu.v.x, c + 1 < 0 ? -hu.v.y : hu.v.y}};
+    if (d.bnd[1] == 0) hu = {{c >= d.cols ? -hu.v.x : hu.v.x, c + 1 >= d.cols ? -hu.v.y : hu.v.y}};
+    if ((r < 0 && d.bnd[2] == 0) || (r >= d.rows && d.bnd[3] == 0)) hv = -hv;
+    const V2 zero = lit<V2>(0.f);
+    AdjCells k;
+    k.f.h = a.h;
+    k.f.z = a.z;
+    k.f.act = MASKED ? act_of(a.nm.v) : B2{true, true};
+    k.f.rh = arcp(a.h);
+    const B2 deep = gt(a.h, p.k.dry);
+    k.f.u = sel(deep, hu * k.f.rh, zero);
+    k.f.v = sel(deep, hv * k.f.rh, zero);
+    k.l[0] = k.l[1] = k.l[2] = zero;
+    if (r >= 0 && r < d.rows) {
+        const B2 live = in & k.f.act;
+        const V2 lam[3] = {a.l0, a.l1, a.l2}, next[3] = {a.h1, a.q1, a.q2};
+        adj_pointwise<NEXT, MASKED>(p, r, c, a.nm, lam, next, live, owned, rain_acc, k.l);
+    }
+    return k;
+}
+
+// The cells one column to the right of a lane's: its own second cell and the
+// first cell of the next lane.
+template <bool MASKED>
+__device__ __forceinline__ AdjCells right_of(const AdjCells& a) {
+    auto next = [](V2 x) { return V2{{x.v.y, __shfl_down_sync(0xffffffffu, x.v.x, 1)}}; };
+    AdjCells b;
+    b.f = {next(a.f.h), next(a.f.z), next(a.f.u), next(a.f.v), next(a.f.rh), {true, true}};
+    if (MASKED) b.f.act = {a.f.act.y, __shfl_down_sync(0xffffffffu, a.f.act.x ? 1 : 0, 1) != 0};
 #pragma unroll
-            for (int q = 0; q < 3; ++q) g[q] = S.l[q][ty + 1][tx + 1] + fl[3 + q] + fr[q] + fb[3 + q] + ft[q];
-            if (c == 0) {
-                const float s = d.bnd[0] == 0 ? -1.f : 1.f;
-                g[0] += fl[0]; g[1] += s * fl[1]; g[2] += fl[2];
+    for (int q = 0; q < 3; ++q) b.l[q] = next(a.l[q]);
+    return b;
+}
+
+// VJP of the faces between two pairs of cells for their dL/d(upd) (s = dt/dx or dt/dy).
+template <int AXIS, bool MASKED>
+__device__ __forceinline__ void adj_faces(const AdjConsts& k, const AdjCells& lo, const AdjCells& hi, float s, V2 dlo[3],
+                                          V2 dhi[3]) {
+    constexpr int nq = AXIS == 1 ? 1 : 2;
+    V2 lF[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) lF[q] = s * (hi.l[q] - lo.l[q]);
+    adj_face_vjp<AXIS, MASKED, V2>(lo.f, hi.f, k, lF, -(s * lo.l[nq]), s * hi.l[nq], dlo, dhi);
+}
+
+template <int THREADS, bool NEXT, bool MASKED, bool VEC>
+__global__ void __launch_bounds__(THREADS) adj_march_kernel(const __grid_constant__ AdjLaunch p, int nstrips,
+                                                            int rows_per_warp) {
+    const DomainDev& d = p.d;
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * (THREADS / kWarp) + (threadIdx.x >> 5);
+    const int r0 = (gw / nstrips) * rows_per_warp, r1 = min(r0 + rows_per_warp, d.rows);
+    const int c = (gw % nstrips) * kMarchCols - 2 + 2 * lane;
+    // Columns clamped to the grid.  With VEC (an even number of columns) a pair
+    // outside the grid loads the nearest pair and keeps the value of its edge column.
+    const int c0 = min(max(c, 0), VEC ? d.cols - 2 : d.cols - 1), c1 = min(max(c + 1, 0), d.cols - 1);
+    const B2 in{c >= 0 && c < d.cols, c + 1 >= 0 && c + 1 < d.cols};
+    const bool strip = lane >= 1 && lane <= kWarp - 2;
+    const B2 mine{strip && in.x, strip && in.y};  // cells this warp writes
+    const float ax = p.s.dt * p.rdx, ay = p.s.dt * p.rdy;
+    const V2 zero = lit<V2>(0.f);
+    double rain_acc = 0.0;
+    if (r0 < d.rows) {
+        AdjRaw raw = adj_raw<NEXT, VEC>(p, r0 - 1, c0, c1), ahead = adj_raw<NEXT, VEC>(p, r0, c0, c1);
+        AdjCells cur = adj_cells<NEXT, MASKED, VEC>(p, raw, r0 - 1, c, in, B2{false, false}, &rain_acc);
+        raw = ahead;
+        ahead = adj_raw<NEXT, VEC>(p, r0 + 1, c0, c1);
+        AdjCells nxt = adj_cells<NEXT, MASKED, VEC>(p, raw, r0, c, in, mine, &rain_acc);
+        V2 below[3];  // the upper side of the y-face below the row
+        {
+            V2 blo[3];
+            adj_faces<0, MASKED>(p.k, cur, nxt, ay, blo, below);
+            // Ghost cells are mirrored copies of their boundary cell: their side of a
+            // boundary face belongs to that cell (normal momentum sign-flipped on reflective edges).
+            if (r0 == 0) {
+                below[0] = below[0] + blo[0];
+                below[1] = below[1] + blo[1];
+                below[2] = below[2] + (d.bnd[2] == 0 ? -blo[2] : blo[2]);
             }
-            if (c == d.cols - 1) {
-                const float s = d.bnd[1] == 0 ? -1.f : 1.f;
-                g[0] += fr[3]; g[1] += s * fr[4]; g[2] += fr[5];
-            }
-            if (r == 0) {
-                const float s = d.bnd[2] == 0 ? -1.f : 1.f;
-                g[0] += fb[0]; g[1] += fb[1]; g[2] += s * fb[2];
+        }
+        for (int r = r0; r < r1; ++r) {
+            cur = nxt;
+            raw = ahead;
+            if (r + 2 <= r1) ahead = adj_raw<NEXT, VEC>(p, r + 2, c0, c1);
+            nxt = adj_cells<NEXT, MASKED, VEC>(p, raw, r + 1, c, in, r + 1 < r1 ? mine : B2{false, false}, &rain_acc);
+            V2 lo[3], hi[3], g[3];
+            adj_faces<0, MASKED>(p.k, cur, nxt, ay, lo, hi);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                g[q] = cur.l[q] + below[q] + lo[q];
+                below[q] = hi[q];
             }
             if (r == d.rows - 1) {
-                const float s = d.bnd[3] == 0 ? -1.f : 1.f;
-                g[0] += ft[3]; g[1] += ft[4]; g[2] += s * ft[5];
+                g[0] = g[0] + hi[0];
+                g[1] = g[1] + hi[1];
+                g[2] = g[2] + (d.bnd[3] == 0 ? -hi[2] : hi[2]);
             }
-            const int64_t o = (int64_t)r * p.lam_out.pitch + c;
-            p.lam_out.h[o] = g[0];
-            p.lam_out.hu[o] = g[1];
-            p.lam_out.hv[o] = g[2];
+            adj_faces<1, MASKED>(p.k, cur, right_of<MASKED>(cur), ax, lo, hi);
+            const float sw = d.bnd[0] == 0 ? -1.f : 1.f, se = d.bnd[1] == 0 ? -1.f : 1.f;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                // hi.x is this lane's second cell's left side, hi.y the next lane's first cell's.
+                const float from_left = __shfl_up_sync(0xffffffffu, hi[q].v.y, 1);
+                g[q] = g[q] + lo[q] + V2{{from_left, hi[q].v.x}};
+                const float west = __shfl_up_sync(0xffffffffu, lo[q].v.y, 1);  // the ghost left of column 0
+                if (c == 0) g[q].v.x += (q == 1 ? sw : 1.f) * west;
+                if (c == d.cols - 1) g[q].v.x += (q == 1 ? se : 1.f) * hi[q].v.x;
+                if (c + 1 == d.cols - 1) g[q].v.y += (q == 1 ? se : 1.f) * hi[q].v.y;
+            }
+            const uint32_t o = (uint32_t)r * (uint32_t)p.lam_out.pitch + (uint32_t)c;
+            if (VEC && mine.y) {
+                *reinterpret_cast<float2*>(p.lam_out.h + o) = g[0].v;
+                *reinterpret_cast<float2*>(p.lam_out.hu + o) = g[1].v;
+                *reinterpret_cast<float2*>(p.lam_out.hv + o) = g[2].v;
+            } else {
+                if (mine.x) {
+                    p.lam_out.h[o] = g[0].v.x;
+                    p.lam_out.hu[o] = g[1].v.x;
+                    p.lam_out.hv[o] = g[2].v.x;
+                }
+                if (mine.y) {
+                    p.lam_out.h[o + 1] = g[0].v.y;
+                    p.lam_out.hu[o + 1] = g[1].v.y;
+                    p.lam_out.hv[o + 1] = g[2].v.y;
+                }
+            }
         }
-        __syncthreads();  // the next tile reuses the shared planes
     }
-    adj_flush_rain<kFThreads>(p, rain_acc);
+    adj_flush_rain<THREADS>(p, rain_acc);
 }
 
 }  // namespace swe

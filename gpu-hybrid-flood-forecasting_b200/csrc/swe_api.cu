@@ -19,6 +19,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "swe_b200.h"
@@ -1312,6 +1313,12 @@ int swe_domain_set_manning(swe_domain_t d, const float* manning_n, int32_t on_ho
 
 namespace {
 
+// adj_march_kernel: resident CTAs per SM (168 registers), and the rows beyond which
+// longer marches in one wave gain nothing over several waves of this height
+// (1024^2 at 4 / 8 / 10 / 14 rows 33.6 / 33.8 / 39.8 / 35.8 us, 1500^2 at 4 / 8 / 16
+// rows 72 / 64 / 72 us; 700^2, one wave at 5 rows, 15.9 us, at 4 rows 20.0 us).
+constexpr int kAdjCtas = 3, kAdjMaxRows = 8;
+
 // One reverse step; `next` (U_{k+1}, or null) lets the cell part skip the face recompute.
 int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const float* hv, int64_t pitch,
                       const float* next, int64_t next_pitch, int64_t next_plane,
@@ -1350,21 +1357,31 @@ int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const floa
     const bool aliased = lam_h_out == lam_h || lam_hu_out == lam_hu || lam_hv_out == lam_hv;
     if (!aliased) {
         // One fused kernel (its halo reads of lam need lam_out elsewhere).
-        static std::once_flag attr_once[2];
-        std::call_once(attr_once[next ? 1 : 0], [&] {
-            if (next)
-                cudaFuncSetAttribute(adj_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(AdjTileSmem));
-            else
-                cudaFuncSetAttribute(adj_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(AdjTileSmem));
-        });
-        const int64_t tiles = (int64_t)((d->dd.cols + kFTW - 1) / kFTW) * ((rows + kFTH - 1) / kFTH);
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(tiles, (int64_t)d->sms * 4));
-        if (next)
-            adj_tile_kernel<true><<<grid, kFThreads, sizeof(AdjTileSmem), st>>>(al);
-        else
-            adj_tile_kernel<false><<<grid, kFThreads, sizeof(AdjTileSmem), st>>>(al);
+        constexpr int wpb = kThreads / kWarp;
+        const int nstrips = (d->dd.cols + kMarchCols - 1) / kMarchCols;
+        auto rows_for = [&](int64_t warps) {
+            const int64_t chunks = std::max<int64_t>(1, warps / nstrips);
+            return (rows + chunks - 1) / chunks;
+        };
+        const int R = march_rows(std::min<int64_t>(rows_for((int64_t)kAdjCtas * wpb * d->sms), kAdjMaxRows),
+                                 rows_for((int64_t)kFewWarps * d->sms));
+        const int64_t warps = (int64_t)nstrips * ((rows + R - 1) / R);
+        const int grid = (int)((warps + wpb - 1) / wpb);
+        // 8-byte accesses where every row of every plane starts on 8 bytes and no pair straddles the right edge.
+        const void* ptrs[12] = {h, hu, hv, lam_h, lam_hu, lam_hv, lam_h_out, lam_hu_out, lam_hv_out, next,
+                                next ? next + next_plane : nullptr, next ? next + 2 * next_plane : nullptr};
+        const bool vec = d->dd.cols % 2 == 0 && choose_vec(ptrs, 12, pitch, lam_pitch) == 2 && out_pitch % 2 == 0 &&
+                         (!next || next_pitch % 2 == 0);
+        auto launch = [&](auto kernel) { kernel<<<grid, kThreads, 0, st>>>(al, nstrips, R); };
+        auto pick = [&](auto nx, auto mk) {
+            constexpr bool N = decltype(nx)::value, M = decltype(mk)::value;
+            if (vec) launch(adj_march_kernel<kThreads, N, M, true>); else launch(adj_march_kernel<kThreads, N, M, false>);
+        };
+        if (next) {
+            if (d->masked) pick(std::true_type{}, std::true_type{}); else pick(std::true_type{}, std::false_type{});
+        } else {
+            if (d->masked) pick(std::false_type{}, std::true_type{}); else pick(std::false_type{}, std::false_type{});
+        }
     } else {
         if (next)
             adj_cell_kernel<kThreads, true><<<blocks, kThreads, 0, st>>>(al);

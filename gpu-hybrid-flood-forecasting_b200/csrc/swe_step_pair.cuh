@@ -481,7 +481,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     // Strip edges for rows rb .. rb+31, one row per lane (the left x-face and the right halo cell).
     auto batch = [&](int rb) {
         __syncwarp();
-        const int rr = min(rb + lane, d.rows - 1);
+        const int rr = min(rb + lane, r1 - 1);  // lanes past the chunk repeat its last row's lines
         Cell L[1], E[1], Q[1];
         const int b = x0w / kEdgeStrip;
         const float* ein = RUN && epar >= 0 ? d.edge[epar] : nullptr;
