@@ -582,27 +582,38 @@ __device__ __forceinline__ V2 load2(const float* p, uint32_t row, int c0, int c1
     return {{__ldg(p + row + c0), __ldg(p + row + c1)}};
 }
 
+// 32-bit element offsets: planes hold fewer than 2^31 elements (checked on the host).
+__device__ __forceinline__ uint32_t adj_row(const DomainDev& d, int r) { return (uint32_t)min(max(r, 0), d.rows - 1); }
+
 template <bool NEXT, bool VEC>
-__device__ __forceinline__ AdjRaw adj_raw(const AdjLaunch& p, int r, int c0, int c1) {
-    const DomainDev& d = p.d;
-    // 32-bit element offsets: planes hold fewer than 2^31 elements (checked on the host).
-    const uint32_t rr = (uint32_t)min(max(r, 0), d.rows - 1);
-    const uint32_t so = rr * (uint32_t)p.in.pitch, zo = rr * (uint32_t)d.spitch, lo = rr * (uint32_t)p.lam.pitch;
-    AdjRaw a;
+__device__ __forceinline__ void load_states(const AdjLaunch& p, int r, int c0, int c1, AdjRaw& a) {
+    const uint32_t rr = adj_row(p.d, r), so = rr * (uint32_t)p.in.pitch, zo = rr * (uint32_t)p.d.spitch;
     a.h = load2<VEC>(p.in.h, so, c0, c1);
     a.hu = load2<VEC>(p.in.hu, so, c0, c1);
     a.hv = load2<VEC>(p.in.hv, so, c0, c1);
-    a.z = load2<VEC>(d.bed, zo, c0, c1);
-    a.nm = load2<VEC>(d.nm, zo, c0, c1);
-    a.l0 = load2<VEC>(p.lam.h, lo, c0, c1);
-    a.l1 = load2<VEC>(p.lam.hu, lo, c0, c1);
-    a.l2 = load2<VEC>(p.lam.hv, lo, c0, c1);
+    a.z = load2<VEC>(p.d.bed, zo, c0, c1);
+    a.nm = load2<VEC>(p.d.nm, zo, c0, c1);
     if constexpr (NEXT) {
         const uint32_t no = rr * (uint32_t)p.next.pitch;
         a.h1 = load2<VEC>(p.next.h, no, c0, c1);
         a.q1 = load2<VEC>(p.next.hu, no, c0, c1);
         a.q2 = load2<VEC>(p.next.hv, no, c0, c1);
     }
+}
+
+template <bool VEC>
+__device__ __forceinline__ void load_lam(const AdjLaunch& p, int r, int c0, int c1, AdjRaw& a) {
+    const uint32_t lo = adj_row(p.d, r) * (uint32_t)p.lam.pitch;
+    a.l0 = load2<VEC>(p.lam.h, lo, c0, c1);
+    a.l1 = load2<VEC>(p.lam.hu, lo, c0, c1);
+    a.l2 = load2<VEC>(p.lam.hv, lo, c0, c1);
+}
+
+template <bool NEXT, bool VEC>
+__device__ __forceinline__ AdjRaw adj_raw(const AdjLaunch& p, int r, int c0, int c1) {
+    AdjRaw a;
+    load_states<NEXT, VEC>(p, r, c0, c1, a);
+    load_lam<VEC>(p, r, c0, c1, a);
     return a;
 }
 
@@ -686,8 +697,16 @@ __global__ void __launch_bounds__(THREADS) adj_march_kernel(const __grid_constan
     const float ax = p.s.dt * p.rdx, ay = p.s.dt * p.rdy;
     const V2 zero = lit<V2>(0.f);
     double rain_acc = 0.0;
+    if (r0 >= d.rows) pdl_enter();
     if (r0 < d.rows) {
-        AdjRaw raw = adj_raw<NEXT, VEC>(p, r0 - 1, c0, c1), ahead = adj_raw<NEXT, VEC>(p, r0, c0, c1);
+        // The states are those of a finished forward pass; only lam (and the gradients)
+        // come from the reverse step before, which is waited for once they are loading.
+        AdjRaw raw, ahead;
+        load_states<NEXT, VEC>(p, r0 - 1, c0, c1, raw);
+        load_states<NEXT, VEC>(p, r0, c0, c1, ahead);
+        pdl_enter();
+        load_lam<VEC>(p, r0 - 1, c0, c1, raw);
+        load_lam<VEC>(p, r0, c0, c1, ahead);
         AdjCells cur = adj_cells<NEXT, MASKED, VEC>(p, raw, r0 - 1, c, in, B2{false, false}, &rain_acc);
         raw = ahead;
         ahead = adj_raw<NEXT, VEC>(p, r0 + 1, c0, c1);

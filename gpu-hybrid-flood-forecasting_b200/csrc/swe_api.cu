@@ -156,16 +156,17 @@ struct swe_domain {
 
 namespace {
 
-// SWE_PDL=1 launches the step kernels with programmatic stream serialisation,
-// so that a step's CTAs are placed while the previous step ends (the kernels
-// wait for their predecessor with griddepcontrol.wait before touching memory;
-// without the attribute that instruction does nothing).  Off by default: the
-// one-wave step grid measured 1.3 % faster with ordinary launches inside the
-// captured graphs.
+// Programmatic stream serialisation of a sequence of steps (SWE_PDL=0 turns it off):
+// a step's CTAs are placed as the previous step's leave, and load what no step
+// writes before they wait for it (griddepcontrol.wait; without the attribute that
+// instruction does nothing).  us a step with it and without: 128^2 4.3 / 5.0, 256^2
+// exact 6.5 / 7.0, 512^2 7.5 / 7.9, 1024^2 14.4 / 15.0, 2048^2 43.5 / 44.1.
+// Only a kernel whose predecessor in the stream writes no bed or n^2 may carry it:
+// the steps of a run or a rollout.
 bool pdl_enabled() {
     static const bool on = [] {
         const char* e = std::getenv("SWE_PDL");
-        return e && e[0] == '1';
+        return !(e && e[0] == '0');
     }();
     return on;
 }
@@ -179,8 +180,8 @@ cudaLaunchConfig_t pdl_config(int blocks, cudaStream_t st) {
     return cfg;
 }
 
-void attach_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
-    if (!pdl_enabled()) return;
+void attach_pdl(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, bool pdl) {
+    if (!pdl || !pdl_enabled()) return;
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
@@ -198,10 +199,10 @@ struct StepK {
         else
             return reinterpret_cast<const void*>(&step_kernel<V, M, kThreads, RUN, MASKED>);
     }
-    static void launch(int blocks, const StepLaunch& sl, cudaStream_t st) {
+    static void launch(int blocks, const StepLaunch& sl, cudaStream_t st, bool pdl) {
         cudaLaunchConfig_t cfg = pdl_config(blocks, st);
         cudaLaunchAttribute attr[1];
-        attach_pdl(cfg, attr);
+        attach_pdl(cfg, attr, pdl);
         if constexpr (V == 2)
             cudaLaunchKernelEx(&cfg, step_kernel_pair<M, kThreads, RUN, MASKED>, sl);
         else
@@ -281,8 +282,8 @@ Plan make_plan(const swe_domain* d, int V, bool run) {
 }
 
 void launch_step(const swe_domain* d, const Plan& pl, const StepLaunch& sl, bool run,
-                 cudaStream_t st) {
-    dispatch(pl.V, d->arith, run, d->masked, [&](auto k) { decltype(k)::launch(pl.blocks, sl, st); });
+                 cudaStream_t st, bool pdl = false) {
+    dispatch(pl.V, d->arith, run, d->masked, [&](auto k) { decltype(k)::launch(pl.blocks, sl, st, pdl); });
 }
 
 // 2-D grid of a per-cell kernel over rows x cols (for_cells): x over the
@@ -551,7 +552,7 @@ int chunk_graph(swe_domain* d, const Plan& pl, int par, int len, cudaGraphExec_t
     }
     if (!d->cap_stream) SWE_CK(cudaStreamCreateWithFlags(&d->cap_stream, cudaStreamNonBlocking));
     SWE_CK(cudaStreamBeginCapture(d->cap_stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < len; ++k) launch_step(d, pl, run_launch(d, pl, par + k), true, d->cap_stream);
+    for (int k = 0; k < len; ++k) launch_step(d, pl, run_launch(d, pl, par + k), true, d->cap_stream, true);
     cudaGraph_t g = nullptr;
     SWE_CK(cudaStreamEndCapture(d->cap_stream, &g));
     const cudaError_t err = cudaGraphInstantiate(&slot, g, 0);
@@ -742,10 +743,10 @@ struct swe_ensemble {
 namespace {
 
 template <class M, bool MASKED>
-void ens_launch_t(const swe_ensemble* e, int parity, cudaStream_t st) {
+void ens_launch_t(const swe_ensemble* e, int parity, cudaStream_t st, bool pdl) {
     cudaLaunchConfig_t cfg = pdl_config(e->grid, st);
     cudaLaunchAttribute attr[1];
-    attach_pdl(cfg, attr);
+    attach_pdl(cfg, attr, pdl);
     if (e->params) {
         e->params->parity = parity;
         cudaLaunchKernelEx(&cfg, ensemble_step_kernel_p<M, kThreads, MASKED>, *e->params);
@@ -755,11 +756,11 @@ void ens_launch_t(const swe_ensemble* e, int parity, cudaStream_t st) {
     }
 }
 
-void ens_launch(const swe_ensemble* e, int parity, cudaStream_t st) {
+void ens_launch(const swe_ensemble* e, int parity, cudaStream_t st, bool pdl = false) {
     if (e->arith == SWE_ARITH_FAST) {
-        if (e->masked) ens_launch_t<FastMath, true>(e, parity, st); else ens_launch_t<FastMath, false>(e, parity, st);
+        if (e->masked) ens_launch_t<FastMath, true>(e, parity, st, pdl); else ens_launch_t<FastMath, false>(e, parity, st, pdl);
     } else {
-        if (e->masked) ens_launch_t<ExactMath, true>(e, parity, st); else ens_launch_t<ExactMath, false>(e, parity, st);
+        if (e->masked) ens_launch_t<ExactMath, true>(e, parity, st, pdl); else ens_launch_t<ExactMath, false>(e, parity, st, pdl);
     }
 }
 
@@ -887,7 +888,7 @@ int ens_graph(swe_ensemble* e, int K) {
     }
     if (!e->cap_stream) SWE_CK(cudaStreamCreateWithFlags(&e->cap_stream, cudaStreamNonBlocking));
     SWE_CK(cudaStreamBeginCapture(e->cap_stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < K; ++k) ens_launch(e, k & 1, e->cap_stream);
+    for (int k = 0; k < K; ++k) ens_launch(e, k & 1, e->cap_stream, true);
     cudaGraph_t g = nullptr;
     SWE_CK(cudaStreamEndCapture(e->cap_stream, &g));
     const cudaError_t err = cudaGraphInstantiate(&e->graph, g, 0);
@@ -1320,11 +1321,14 @@ namespace {
 constexpr int kAdjCtas = 3, kAdjMaxRows = 8;
 
 // One reverse step; `next` (U_{k+1}, or null) lets the cell part skip the face recompute.
+// `chained`: its predecessor in the stream is the reverse step of the next state, and
+// the states were complete before that one (see pdl_enabled).
 int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const float* hv, int64_t pitch,
                       const float* next, int64_t next_pitch, int64_t next_plane,
                       const float* lam_h, const float* lam_hu, const float* lam_hv, int64_t lam_pitch,
                       float* lam_h_out, float* lam_hu_out, float* lam_hv_out, int64_t out_pitch,
-                      float* grad_n2, double* grad_rain_scale, double dt, double time_s, cudaStream_t st) {
+                      float* grad_n2, double* grad_rain_scale, double dt, double time_s, cudaStream_t st,
+                      bool chained = false) {
     const int rows = d->dd.rows;
     if (!d->lupd[0]) {
         d->lpitch = round_up(d->dd.cols, 128);
@@ -1355,7 +1359,9 @@ int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const floa
     const int64_t n = (int64_t)rows * d->dd.cols;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + kThreads - 1) / kThreads, (int64_t)d->sms * 16));
     const bool aliased = lam_h_out == lam_h || lam_hu_out == lam_hu || lam_hv_out == lam_hv;
-    if (!aliased) {
+    // The march addresses a plane with 32-bit element offsets.
+    const bool small = (int64_t)rows * std::max({pitch, lam_pitch, out_pitch, next_pitch}) < (int64_t(1) << 31);
+    if (!aliased && small) {
         // One fused kernel (its halo reads of lam need lam_out elsewhere).
         constexpr int wpb = kThreads / kWarp;
         const int nstrips = (d->dd.cols + kMarchCols - 1) / kMarchCols;
@@ -1372,7 +1378,10 @@ int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const floa
                                 next ? next + next_plane : nullptr, next ? next + 2 * next_plane : nullptr};
         const bool vec = d->dd.cols % 2 == 0 && choose_vec(ptrs, 12, pitch, lam_pitch) == 2 && out_pitch % 2 == 0 &&
                          (!next || next_pitch % 2 == 0);
-        auto launch = [&](auto kernel) { kernel<<<grid, kThreads, 0, st>>>(al, nstrips, R); };
+        cudaLaunchConfig_t cfg = pdl_config(grid, st);
+        cudaLaunchAttribute attr[1];
+        attach_pdl(cfg, attr, chained);
+        auto launch = [&](auto kernel) { cudaLaunchKernelEx(&cfg, kernel, al, nstrips, R); };
         auto pick = [&](auto nx, auto mk) {
             constexpr bool N = decltype(nx)::value, M = decltype(mk)::value;
             if (vec) launch(adj_march_kernel<kThreads, N, M, true>); else launch(adj_march_kernel<kThreads, N, M, false>);
@@ -1413,9 +1422,13 @@ int swe_adjoint_step(swe_domain_t d, const float* h, const float* hu, const floa
                              static_cast<cudaStream_t>(stream));
 }
 
-int swe_step(swe_domain_t d, const float* h, const float* hu, const float* hv, int64_t pitch_in,
-             float* h_out, float* hu_out, float* hv_out, int64_t pitch_out, double dt,
-             double time_s, void* stream) {
+}  // extern "C"
+
+namespace {
+
+// swe_step; `chained`: a step of a rollout (see pdl_enabled).
+int step_impl(swe_domain* d, const float* h, const float* hu, const float* hv, int64_t pitch_in, float* h_out,
+              float* hu_out, float* hv_out, int64_t pitch_out, double dt, double time_s, cudaStream_t st, bool chained) {
     if (!d) return fail(SWE_ERR_INVALID, "null domain");
     int rc = check_state_ptrs(h, hu, hv, pitch_in, d->dd.cols);
     if (rc) return rc;
@@ -1445,9 +1458,20 @@ int swe_step(swe_domain_t d, const float* h, const float* hu, const float* hv, i
     sl.slots = nullptr;
     sl.nstrips = pl.nstrips;
     sl.rows_per_warp = pl.rows_per_warp;
-    launch_step(d, pl, sl, false, static_cast<cudaStream_t>(stream));
+    launch_step(d, pl, sl, false, st, chained);
     SWE_CK(cudaGetLastError());
     return SWE_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int swe_step(swe_domain_t d, const float* h, const float* hu, const float* hv, int64_t pitch_in,
+             float* h_out, float* hu_out, float* hv_out, int64_t pitch_out, double dt,
+             double time_s, void* stream) {
+    return step_impl(d, h, hu, hv, pitch_in, h_out, hu_out, hv_out, pitch_out, dt, time_s,
+                     static_cast<cudaStream_t>(stream), false);
 }
 
 int swe_max_inverse_dt(swe_domain_t d, const float* h, const float* hu, const float* hv,
@@ -1907,8 +1931,8 @@ int swe_rollout_forward(swe_domain_t d, float* h, float* hu, float* hv, int64_t 
                 if (rc) return rc;
             }
         }
-        rc = swe_step(d, d->ping[src][0], d->ping[src][1], d->ping[src][2], d->ppitch, d->ping[src ^ 1][0],
-                      d->ping[src ^ 1][1], d->ping[src ^ 1][2], d->ppitch, dtk, t, stream);
+        rc = step_impl(d, d->ping[src][0], d->ping[src][1], d->ping[src][2], d->ppitch, d->ping[src ^ 1][0],
+                       d->ping[src ^ 1][1], d->ping[src ^ 1][2], d->ppitch, dtk, t, st, k > 0);
         if (rc) return rc;
         if (n_gauges > 0 && (k + 1) % obs_every == 0) {
             gauge_gather_kernel<<<(n_gauges + 127) / 128, 128, 0, st>>>(
@@ -1983,8 +2007,8 @@ int swe_rollout_backward(swe_domain_t d, const float* ckpt, int32_t ckpt_every, 
         for (int k = k0; k < k1; ++k) {
             const float* a = sb + (int64_t)(k - k0) * 3 * plane;
             float* o = k + 1 < k1 ? sb + (int64_t)(k + 1 - k0) * 3 * plane : nxtbuf[b];
-            const int src = swe_step(d, a, a + plane, a + 2 * plane, cols, o, o + plane, o + 2 * plane, cols,
-                                     dts ? dts[k] : dt, step_time(k, dt, t0, dts), aux);
+            const int src = step_impl(d, a, a + plane, a + 2 * plane, cols, o, o + plane, o + 2 * plane, cols,
+                                      dts ? dts[k] : dt, step_time(k, dt, t0, dts), aux, k > k0);
             if (src) return src;
         }
         SWE_CK(cudaEventRecord(ev_rec[b], aux));
@@ -2030,7 +2054,7 @@ int swe_rollout_backward(swe_domain_t d, const float* ckpt, int32_t ckpt_every, 
             const float* nx = k + 1 < k1 ? sb + (int64_t)(k + 1 - k0) * 3 * plane : nxtbuf[b];
             rc = adjoint_step_impl(d, a, a + plane, a + 2 * plane, cols, nx, cols, plane, src[0], src[1], src[2], sp,
                                    dst[0], dst[1], dst[2], dp, grad_n2, grad_rain_scale, dts ? dts[k] : dt,
-                                   step_time(k, dt, t0, dts), st);
+                                   step_time(k, dt, t0, dts), st, k < k1 - 1);
             if (rc) return join(rc);
             cur ^= 1;
         }

@@ -95,9 +95,9 @@ __device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) { return __
 // fast 6.6 us a step instead of 7.5, 300 x 420 7.2 instead of 7.5).
 static_assert(kEdgeStrip == 2 * kWarp, "a paired-march strip is 2 x 32 columns");
 
-template <class M, bool RUN, bool MASKED, bool LAST_CONSUME, class PlanFn>
+template <class M, bool RUN, bool MASKED, bool LAST_CONSUME, class EnterFn, class PlanFn>
 __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& in,
-                                            const StateOut& out, PlanFn&& plan_fn, const Control* ctl,
+                                            const StateOut& out, EnterFn&& enter_fn, PlanFn&& plan_fn, const Control* ctl,
                                             int r0, int r1, int x0w, WarpSmem& sm, StepAccum& acc, int epar = -1) {
     constexpr int kBatch = kWarp;
     using A = P<M>;
@@ -153,19 +153,24 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
 
     // Start the copies of ring row qi (row r0-1+qi, clamped to the grid): one group per row,
     // zero bytes past the chunk or the right edge, so the issue path has no branch.
-    auto issue = [&](int qi) {
-        const int q = r0 - 1 + qi;
-        const int rr = min(max(q, 0), d.rows - 1);
+    // The state's copies close the group.
+    auto issue_static = [&](int qi) {
+        const int rr = min(max(r0 - 1 + qi, 0), d.rows - 1);
         const int sz = qi < nq ? csize : 0;
         const int slot = qi & (kRing - 1);
         // 32-bit element offsets: planes hold fewer than 2^31 elements (checked on the host).
-        const uint32_t so = (uint32_t)rr * (uint32_t)in.pitch + (uint32_t)ccol;
         const uint32_t zo = (uint32_t)rr * (uint32_t)d.spitch + (uint32_t)ccol;
+        cp_async_8z(&sm.ring[slot][3][lane], d.bed + zo, sz);
+        cp_async_8z(&sm.ring[slot][4][lane], d.nm + zo, sz);
+    };
+    auto issue_state = [&](int qi) {
+        const int rr = min(max(r0 - 1 + qi, 0), d.rows - 1);
+        const int sz = qi < nq ? csize : 0;
+        const int slot = qi & (kRing - 1);
+        const uint32_t so = (uint32_t)rr * (uint32_t)in.pitch + (uint32_t)ccol;
         cp_async_8z(&sm.ring[slot][0][lane], in.h + so, sz);
         cp_async_8z(&sm.ring[slot][1][lane], in.hu + so, sz);
         cp_async_8z(&sm.ring[slot][2][lane], in.hv + so, sz);
-        cp_async_8z(&sm.ring[slot][3][lane], d.bed + zo, sz);
-        cp_async_8z(&sm.ring[slot][4][lane], d.nm + zo, sz);
         cp_async_commit();
     };
     // Ring row qi into registers, ghost ring applied; its slot is refilled with row qi+kRing.
@@ -211,7 +216,8 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         } else {
             set_vel_t<M>(c, kp);
         }
-        issue(qi + kRing);
+        issue_static(qi + kRing);
+        issue_state(qi + kRing);
         return big;
     };
 
@@ -239,8 +245,10 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         }
     };
 
+    // What no step writes (bed, n^2, the edges' bed and n^2) is loaded before the
+    // previous step is waited for (enter_fn).
 #pragma unroll
-    for (int qi = 0; qi < kRing; ++qi) issue(qi);
+    for (int qi = 0; qi < kRing; ++qi) issue_static(qi);
 
     CellT<float2> R0, R1;
     float big0 = 0.f, big1 = 0.f;  // their rows' largest depth or speed (exact arithmetic)
@@ -478,27 +486,43 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             }
         }
     };
+    // The cells either side of the strip in the edge array.  At the grid's own edges
+    // the ghost column is the mirrored edge column.  Past a partial strip the last
+    // column's ghost sits in the strip itself (consume), so the cell right of it is
+    // not read: any cell does.
+    const float* ein = RUN && epar >= 0 ? d.edge[epar] : nullptr;
+    const int eb = x0w / kEdgeStrip;
+    const bool west = x0w == 0, full = x0w + kEdgeStrip <= d.cols, east = x0w + kEdgeStrip >= d.cols;
+    struct EdgeStatics {
+        float z[3], nm[3];  // left of the strip, its first column, right of it
+    };
+    auto edge_statics = [&](int rb) -> EdgeStatics {
+        EdgeStatics e{};
+        if (RUN && ein != nullptr) {
+            const int rr = min(rb + lane, r1 - 1);
+            auto at = [&](int i, int bd, int right) {
+                e.z[i] = __ldg(d.edge_static + edge_static_index(d, bd, 2 * right + 0, rr));
+                e.nm[i] = __ldg(d.edge_static + edge_static_index(d, bd, 2 * right + 1, rr));
+            };
+            at(0, eb, west ? 1 : 0);
+            at(1, eb, 1);
+            at(2, full ? eb + 1 : eb, east && full ? 0 : 1);
+        }
+        return e;
+    };
     // Strip edges for rows rb .. rb+31, one row per lane (the left x-face and the right halo cell).
-    auto batch = [&](int rb) {
+    auto batch = [&](int rb, const EdgeStatics& es) {
         __syncwarp();
         const int rr = min(rb + lane, r1 - 1);  // lanes past the chunk repeat its last row's lines
         Cell L[1], E[1], Q[1];
-        const int b = x0w / kEdgeStrip;
-        const float* ein = RUN && epar >= 0 ? d.edge[epar] : nullptr;
         if (RUN && ein != nullptr) {
-            // The grid's own edges: the ghost column is the mirrored edge column.  Past a
-            // partial strip the last column's ghost sits in the strip itself (consume), so
-            // the cell right of it is not read: any cell does.
-            const bool west = x0w == 0, full = x0w + kEdgeStrip <= d.cols, east = x0w + kEdgeStrip >= d.cols;
-            auto side = [&](int bd, int right) -> Cell {
+            auto side = [&](int i, int bd, int right) -> Cell {
                 return {__ldg(ein + edge_index(d, bd, 3 * right + 0, rr)), __ldg(ein + edge_index(d, bd, 3 * right + 1, rr)),
-                        __ldg(ein + edge_index(d, bd, 3 * right + 2, rr)),
-                        __ldg(d.edge_static + edge_static_index(d, bd, 2 * right + 0, rr)),
-                        __ldg(d.edge_static + edge_static_index(d, bd, 2 * right + 1, rr)), 0.f, 0.f};
+                        __ldg(ein + edge_index(d, bd, 3 * right + 2, rr)), es.z[i], es.nm[i], 0.f, 0.f};
             };
-            L[0] = side(b, west ? 1 : 0);
-            E[0] = side(b, 1);
-            Q[0] = side(full ? b + 1 : b, east && full ? 0 : 1);
+            L[0] = side(0, eb, west ? 1 : 0);
+            E[0] = side(1, eb, 1);
+            Q[0] = side(2, full ? eb + 1 : eb, east && full ? 0 : 1);
             if (west && d.bnd[0] == 0) L[0].hu = -L[0].hu;
             if (east && d.bnd[1] == 0) Q[0].hu = -Q[0].hu;
         } else {
@@ -574,7 +598,13 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     // The first batch's strip edges are loaded before the ring's first rows are
     // waited for, and the step is planned while the ring's rows are in flight,
     // so that the latencies of the march's start overlap.
-    batch(r0);
+    {
+        const EdgeStatics es = edge_statics(r0);
+        enter_fn();
+#pragma unroll
+        for (int qi = 0; qi < kRing; ++qi) issue_state(qi);
+        batch(r0, es);
+    }
     {
         const MarchPlan mp = plan_fn();
         if (!mp.go) {
@@ -615,7 +645,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     big1 = consume(2, R1);  // row r0+1
     for (int rb = r0; rb < r1; rb += kBatch) {
         flush_ledger();
-        if (rb != r0) batch(rb);
+        if (rb != r0) batch(rb, edge_statics(rb));
         const int re = min(rb + kBatch, r1);
         for (int r = rb; r < re; r += 2) {
             row(r, r - rb, R0, R1, big0, big1);
@@ -641,7 +671,6 @@ template <class M, int THREADS, bool RUN, bool MASKED>
 __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(const StepLaunch p) {
     constexpr int NW = THREADS / kWarp;
     __shared__ WarpSmem s_warp[NW];
-    pdl_enter();
     const DomainDev& d = p.d;
     const int wib = threadIdx.x >> 5;
     const int gw = blockIdx.x * NW + wib;
@@ -652,11 +681,15 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
     StepAccum acc;
     acc.zero();
     if constexpr (RUN) {
-        // The slot copy and the plan's loads are in flight while the march
-        // starts its own; the plan is made once those are issued.
-        ledger_prefetch(&p.slots[gw], s_warp[wib].old);
-        cp_async_commit();
-        const PlanInputs in = plan_fetch(p.ctl, p.par);
+        // The slot copy and the plan's loads are issued once the previous step is
+        // complete and are in flight while the march starts its own; the plan is
+        // made once those are issued.
+        PlanInputs in;
+        auto enter_fn = [&]() {
+            pdl_enter();
+            ledger_prefetch(&p.slots[gw], s_warp[wib].old);
+            in = plan_fetch(p.ctl, p.par);
+        };
         StepPlan pl;
         auto plan_fn = [&]() -> MarchPlan {
             pl = plan_step(d, in);
@@ -664,10 +697,10 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
             return MarchPlan{pl.s, pl.snap, pl.dt, pl.go};
         };
         const bool went = r0 < d.upd_hi
-                              ? march_pair<M, true, MASKED, true>(d, p.in, p.out, plan_fn, p.ctl, r0, r1,
+                              ? march_pair<M, true, MASKED, true>(d, p.in, p.out, enter_fn, plan_fn, p.ctl, r0, r1,
                                                                   strip * kWarp * 2, s_warp[wib], acc,
                                                                   d.edge[0] ? p.par : -1)
-                              : plan_fn().go != 0;
+                              : (enter_fn(), cp_async_commit(), plan_fn().go != 0);
         if (!went) {  // uniform over the grid: the run has ended
             cp_async_wait<0>();
             return;
@@ -684,7 +717,7 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
         warp_end_step(p.ctl, &p.slots[gw], s_warp[wib].old, p.par, in.pos.steps, gw % kMaxStripes, a);
     } else {
         if (r0 < d.upd_hi)
-            march_pair<M, false, MASKED, true>(d, p.in, p.out, [&]() { return MarchPlan{p.s, -1, 0.0, 1}; }, nullptr, r0,
+            march_pair<M, false, MASKED, true>(d, p.in, p.out, pdl_enter, [&]() { return MarchPlan{p.s, -1, 0.0, 1}; }, nullptr, r0,
                                          r1, strip * kWarp * 2, s_warp[wib], acc);
     }
 }
@@ -710,16 +743,20 @@ struct MemberDev {
     int nstrips, rows_per_warp, ncta;
 };
 
-// One item of a batched step: warp `wib` of slot `slot` of member `md`.
+// One item of a batched step: warp `wib` of slot `slot` of member `md`.  A CTA's
+// first item waits for the previous step (pdl_enter) once its static loads are issued.
 template <class M, int THREADS, bool MASKED>
-__device__ __forceinline__ void ensemble_item(const MemberDev& md, int slot, int par, WarpSmem& sm) {
+__device__ __forceinline__ void ensemble_item(const MemberDev& md, int slot, int par, WarpSmem& sm, bool first) {
     constexpr int NW = THREADS / kWarp;
     const int wib = threadIdx.x >> 5;
     const int gw = slot * NW + wib;
     __syncwarp();  // the previous item's slot copy has been read
-    ledger_prefetch(&md.slots[gw], sm.old);
-    cp_async_commit();
-    const PlanInputs pin = plan_fetch(md.ctl, par);
+    PlanInputs pin;
+    auto enter_fn = [&]() {
+        if (first) pdl_enter();
+        ledger_prefetch(&md.slots[gw], sm.old);
+        pin = plan_fetch(md.ctl, par);
+    };
     StepPlan pl;
     auto plan_fn = [&]() -> MarchPlan {
         pl = plan_step(md.d, pin);
@@ -734,10 +771,10 @@ __device__ __forceinline__ void ensemble_item(const MemberDev& md, int slot, int
     const StateOut out{md.buf[par ^ 1][0], md.buf[par ^ 1][1], md.buf[par ^ 1][2], md.pitch};
     StepAccum acc;
     acc.zero();
-    const bool went = r0 < md.d.rows ? march_pair<M, true, MASKED, false>(md.d, in, out, plan_fn, md.ctl,
+    const bool went = r0 < md.d.rows ? march_pair<M, true, MASKED, false>(md.d, in, out, enter_fn, plan_fn, md.ctl,
                                                                    r0, r1, strip * kWarp * 2, sm, acc,
                                                                    md.d.edge[0] ? par : -1)
-                                     : plan_fn().go != 0;
+                                     : (enter_fn(), cp_async_commit(), plan_fn().go != 0);
     if (!went) {
         cp_async_wait<0>();
         return;
@@ -768,14 +805,13 @@ ensemble_step_kernel(const MemberDev* __restrict__ members, const int2* __restri
     constexpr int NW = THREADS / kWarp;
     __shared__ WarpSmem s_warp[NW];
     __shared__ MemberDev s_md;
-    pdl_enter();
     const int wib = threadIdx.x >> 5;
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const int2 item = items[it];
         __syncthreads();  // the previous item is done with s_md
         if (threadIdx.x == 0) s_md = members[item.x];
         __syncthreads();
-        ensemble_item<M, THREADS, MASKED>(s_md, item.y, parity, s_warp[wib]);
+        ensemble_item<M, THREADS, MASKED>(s_md, item.y, parity, s_warp[wib], it == (int)blockIdx.x);
     }
 }
 
@@ -799,12 +835,12 @@ __global__ void __launch_bounds__(THREADS, SWE_ENS_MINBLOCKS)
 ensemble_step_kernel_p(const __grid_constant__ EnsParams p) {
     constexpr int NW = THREADS / kWarp;
     __shared__ WarpSmem s_warp[NW];
-    pdl_enter();
     const int wib = threadIdx.x >> 5;
     int member = 0;
     for (int it = blockIdx.x; it < p.n_items; it += gridDim.x) {
         while (it >= p.cta_begin[member + 1]) ++member;
-        ensemble_item<M, THREADS, MASKED>(p.m[member], it - p.cta_begin[member], p.parity, s_warp[wib]);
+        ensemble_item<M, THREADS, MASKED>(p.m[member], it - p.cta_begin[member], p.parity, s_warp[wib],
+                                          it == (int)blockIdx.x);
     }
 }
 
