@@ -25,6 +25,7 @@
 #include "swe_b200.h"
 #include "swe_step.cuh"
 #include "swe_step_pair.cuh"
+#include "swe_begin.cuh"
 #include "swe_adjoint.cuh"
 #include "swe_hybrid.cuh"
 #include "swe_nn.cuh"
@@ -88,6 +89,13 @@ struct Plan {
 
 }  // namespace
 
+// Page-locked words of a domain that its kernels write and the host reads after
+// waiting for the stream.
+struct HostSlots {
+    RunSummary run;
+    float max_inverse_dt;
+};
+
 struct swe_domain {
     DomainDev dd{};
     int arith = SWE_ARITH_EXACT;
@@ -101,9 +109,10 @@ struct swe_domain {
     Control* ctl = nullptr;          // run control (device)
     Control* ctl_scratch = nullptr;  // standalone reductions (device)
     Control* ctl_host = nullptr;     // pinned poll slots [2]
+    HostSlots* host = nullptr;       // pinned words that kernels write (after the poll slots)
     LedgerSlot* slots = nullptr;  // step warps' ledger slots (kept over a run)
     int slots_cap = 0;            // in CTAs (kWarpsPerCta slots each)
-    Partial* rparts = nullptr;     // partials of the standalone CFL/volume reductions
+    StartPartial* rparts = nullptr;  // partials of the start reductions
     int rparts_cap = 0;
     float* ping[2][3] = {{nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr}};
     int64_t ppitch = 0;
@@ -134,7 +143,6 @@ struct swe_domain {
     cudaEvent_t seg_ev[6] = {};  // start, recomputed[2], reversed[2], end
     double* corr_sums = nullptr;    // volume sums of the residual correction
     float* corr_prov = nullptr;     // provisional-depth plane of the correction
-    unsigned* done_counter = nullptr;  // set by an ensemble: shared completion counter
     // swe_run_host: device staging of the recorded outputs and the copy stream.
     float* snap_dev = nullptr;
     int64_t snap_cap = 0;  // floats
@@ -297,21 +305,41 @@ dim3 cell_grid(int rows, int cols, int threads, int sms, int per_thread = 1) {
     return dim3((unsigned)gx, (unsigned)gy);
 }
 
-dim3 reduce_grid(const swe_domain* d) {
-    return cell_grid(d->dd.upd_hi - d->dd.upd_lo, d->dd.cols, kThreads, d->sms, 8);
-}
+// CTAs of a load or store of a domain's rows on `sms` SMs' share of the GPU.
+dim3 load_grid(const swe_domain* d, int sms) { return cell_grid(d->dd.rows, d->dd.cols, kThreads, sms); }
 
 int reduce_blocks(const swe_domain* d) {
-    const dim3 g = reduce_grid(d);
+    const dim3 g = load_grid(d, d->sms);
     return (int)(g.x * g.y);
 }
 
-void launch_reduce(const swe_domain* d, const StateView& s, Control* ctl, cudaStream_t st) {
-    const dim3 grid = reduce_grid(d);
-    if (d->arith == SWE_ARITH_FAST)
-        reduce_kernel<FastMath, kThreads><<<grid, kThreads, 0, st>>>(d->dd, s, ctl, d->rparts);
+template <int ND>
+void launch_load(const LoadBatch<ND>& b, int ctas, int arith, cudaStream_t st) {
+    if (arith == SWE_ARITH_FAST)
+        load_kernel<FastMath, kThreads, ND><<<ctas, kThreads, 0, st>>>(b);
     else
-        reduce_kernel<ExactMath, kThreads><<<grid, kThreads, 0, st>>>(d->dd, s, ctl, d->rparts);
+        load_kernel<ExactMath, kThreads, ND><<<ctas, kThreads, 0, st>>>(b);
+}
+
+// The reduction of state `s` of domain `d` on `sms` SMs' share, as part `cta0` of a load.
+LoadDomain load_part(const swe_domain* d, const StateView& s, Control* ctl, int cta0, int sms) {
+    const dim3 g = load_grid(d, sms);
+    LoadDomain q{};
+    q.rows = d->dd.rows;
+    q.cols = d->dd.cols;
+    q.upd_lo = d->dd.upd_lo;
+    q.upd_hi = d->dd.upd_hi;
+    q.gx = (int)g.x;
+    q.gy = (int)g.y;
+    q.cta0 = cta0;
+    q.k = d->dd.k;
+    q.area = d->dd.dx * d->dd.dy;
+    q.nm = d->nm;
+    q.spitch = d->dd.spitch;
+    q.in = s;
+    q.ctl = ctl;
+    q.parts = d->rparts;
+    return q;
 }
 
 int choose_vec(const void* const* ptrs, int n, int64_t pitch_a, int64_t pitch_b) {
@@ -324,14 +352,14 @@ int choose_vec(const void* const* ptrs, int n, int64_t pitch_a, int64_t pitch_b)
     return 1;
 }
 
-// Partials of the reductions (reduce_kernel); separate from the step slots so that
+// Partials of the start reductions; separate from the step slots so that
 // a CFL query in the middle of a resident run leaves its ledger intact.
 int ensure_rparts(swe_domain* d) {
     const int blocks = reduce_blocks(d);
     if (blocks <= d->rparts_cap) return SWE_OK;
     if (d->rparts) cudaFree(d->rparts);
     d->rparts = nullptr;
-    SWE_CK(cudaMalloc(&d->rparts, sizeof(Partial) * (size_t)blocks));
+    SWE_CK(cudaMalloc(&d->rparts, sizeof(StartPartial) * (size_t)blocks));
     d->rparts_cap = blocks;
     return SWE_OK;
 }
@@ -354,18 +382,7 @@ int ensure_parts(swe_domain* d, int blocks) {
 int fill_edge_statics(swe_domain* d, cudaStream_t st) {
     if (!d->edge_stat) return SWE_OK;
     const int nb = (d->dd.cols + kEdgeStrip - 1) / kEdgeStrip + 1;
-    edge_fill_kernel<<<dim3((unsigned)((d->dd.rows + 127) / 128), (unsigned)nb), 128, 0, st>>>(
-        d->dd, StateView{nullptr, nullptr, nullptr, 0}, nullptr, d->edge_stat);
-    SWE_CK(cudaGetLastError());
-    return SWE_OK;
-}
-
-// The strip-boundary columns of the state in ping buffer 0 (a run's start).
-int fill_edges(swe_domain* d, cudaStream_t st) {
-    if (!d->edge_buf[0]) return SWE_OK;
-    const int nb = (d->dd.cols + kEdgeStrip - 1) / kEdgeStrip + 1;
-    edge_fill_kernel<<<dim3((unsigned)((d->dd.rows + 127) / 128), (unsigned)nb), 128, 0, st>>>(
-        d->dd, StateView{d->ping[0][0], d->ping[0][1], d->ping[0][2], d->ppitch}, d->edge_buf[0], nullptr);
+    edge_fill_kernel<<<dim3((unsigned)((d->dd.rows + 127) / 128), (unsigned)nb), 128, 0, st>>>(d->dd, d->edge_stat);
     SWE_CK(cudaGetLastError());
     return SWE_OK;
 }
@@ -418,91 +435,162 @@ int copy_plane(float* dst, int64_t dpitch, const float* src, int64_t spitch, int
     return SWE_OK;
 }
 
-// Load the initial state into ping buffer 0, upload the output times, write
-// snapshot 0, reset the run control and launch the reduction that sets the
-// clock, the first CFL dt and volume0.  Shared by swe_run, swe_advance and the
-// ensemble.
-int begin_run(swe_domain* d, StateView init, const float* times_host, int n_times, double t_start,
-              int n_out, int max_steps, float* out_h, float* out_hu, float* out_hv, cudaStream_t st,
-              const double* times64_host = nullptr, double* dt_log = nullptr, int defer_plan = 0) {
-    const int rows = d->dd.rows, cols = d->dd.cols;
+// A run of one domain as its start needs it: the initial state, clock, targets,
+// step cap and the buffers of its outputs.
+struct RunStart {
+    StateView init;
+    double t_start;
+    int n_out, max_steps;
+    const float* times;               // HOST, n_times
+    int n_times;
+    const double* times64 = nullptr;  // HOST float64 targets (n_times <= 2), or null
+    float* out[3] = {nullptr, nullptr, nullptr};
+    double* dt_log = nullptr;
+    unsigned* done_counter = nullptr;
+    int defer_plan = 0;
+};
+
+constexpr int kInlineTimes = 64;  // output times of one run carried in launch parameters
+
+// Buffers of a run and its parts of the start launches: the control block with up
+// to NT targets, and the load on `sms` SMs' share from CTA `cta0` on.
+template <int NT>
+int prepare_start(swe_domain* d, const RunStart& r, int cta0, int sms, InitDomain<NT>& in, LoadDomain& ld, cudaStream_t st) {
     d->resident = false;  // any run replaces a resident state
     int rc = ensure_ping(d);
     if (rc) return rc;
     rc = ensure_parts(d, reduce_blocks(d));
     if (rc) return rc;
-    for (int f = 0; f < 3; ++f) {
-        const float* src = f == 0 ? init.h : (f == 1 ? init.hu : init.hv);
-        rc = copy_plane(d->ping[0][f], d->ppitch, src, init.pitch, rows, cols, st);
-        if (rc) return rc;
-    }
-    rc = fill_edges(d, st);
-    if (rc) return rc;
-    if (n_times > d->times_cap) {
+    if (r.n_times > d->times_cap) {
         if (d->times_dev) cudaFree(d->times_dev);
         d->times_dev = nullptr;
-        SWE_CK(cudaMalloc(&d->times_dev, sizeof(float) * (size_t)n_times));
-        d->times_cap = n_times;
+        SWE_CK(cudaMalloc(&d->times_dev, sizeof(float) * (size_t)r.n_times));
+        d->times_cap = r.n_times;
     }
-    // Output times (up to kInlineTimes: every advance, ensemble interval and
-    // ordinary run) travel with the control block's launch parameters; longer
-    // output lists are copied.
-    static_assert(kInlineTimes <= 128, "one thread of control_init_kernel per inline time");
-    RunTargets tg{};
-    if (n_times <= kInlineTimes) {
-        tg.n = n_times;
-        tg.times = d->times_dev;
-        for (int i = 0; i < n_times; ++i) tg.t[i] = times_host[i];
+    in = InitDomain<NT>{};
+    in.ctl = d->ctl;
+    if (r.n_times <= NT) {
+        in.n = r.n_times;
+        in.times = d->times_dev;
+        for (int i = 0; i < r.n_times; ++i) in.t[i] = r.times[i];
     } else {
-        SWE_CK(cudaMemcpyAsync(d->times_dev, times_host, sizeof(float) * (size_t)n_times,
-                               cudaMemcpyHostToDevice, st));
+        SWE_CK(cudaMemcpyAsync(d->times_dev, r.times, sizeof(float) * (size_t)r.n_times, cudaMemcpyHostToDevice, st));
     }
-    if (times64_host) {
-        if (n_times > 2) return fail(SWE_ERR_INVALID, "float64 targets support one interval");
+    if (r.times64) {
+        if (r.n_times > 2) return fail(SWE_ERR_INVALID, "float64 targets support one interval");
         if (!d->times64_dev) SWE_CK(cudaMalloc(&d->times64_dev, 2 * sizeof(double)));
-        tg.times64 = d->times64_dev;
-        for (int i = 0; i < n_times; ++i) tg.t64[i] = times64_host[i];
-    }
-    if (out_h) {
-        float* outs[3] = {out_h, out_hu, out_hv};
-        for (int f = 0; f < 3; ++f) {
-            const float* src = f == 0 ? init.h : (f == 1 ? init.hu : init.hv);
-            rc = copy_plane(outs[f], cols, src, init.pitch, rows, cols, st);
-            if (rc) return rc;
-        }
+        in.times64 = d->times64_dev;
+        for (int i = 0; i < r.n_times; ++i) in.t64[i] = r.times64[i];
     }
     Control c0;
     std::memset(&c0, 0, sizeof(c0));
-    c0.n_out = n_out;
-    c0.max_steps = max_steps;
-    c0.t_start = t_start;
+    c0.n_out = r.n_out;
+    c0.max_steps = r.max_steps;
+    c0.t_start = r.t_start;
     c0.times = d->times_dev;
-    c0.times64 = times64_host ? d->times64_dev : nullptr;
-    c0.done_counter = d->done_counter;
-    c0.dt_log = dt_log;
-    c0.defer_plan = defer_plan;
-    c0.out_h = out_h;
-    c0.out_hu = out_hu;
-    c0.out_hv = out_hv;
-    c0.out_plane = (int64_t)rows * cols;
-    ControlHeadImage img;
-    std::memcpy(&img, &c0, sizeof(img));
-    control_init_kernel<<<1, 128, 0, st>>>(d->ctl, img, tg);
-    SWE_CK(cudaGetLastError());
-    StateView v0{d->ping[0][0], d->ping[0][1], d->ping[0][2], d->ppitch};
-    launch_reduce(d, v0, d->ctl, st);
-    SWE_CK(cudaGetLastError());
-    // The step warps' ledger slots start the run at zero.
-    SWE_CK(cudaMemsetAsync(d->slots, 0, sizeof(LedgerSlot) * kWarpsPerCta * (size_t)d->slots_cap, st));
+    c0.times64 = r.times64 ? d->times64_dev : nullptr;
+    c0.done_counter = r.done_counter;
+    c0.dt_log = r.dt_log;
+    c0.defer_plan = r.defer_plan;
+    c0.out_h = r.out[0];
+    c0.out_hu = r.out[1];
+    c0.out_hv = r.out[2];
+    c0.out_plane = (int64_t)d->dd.rows * d->dd.cols;
+    std::memcpy(&in.head, &c0, sizeof(in.head));
+    ld = load_part(d, r.init, d->ctl, cta0, sms);
+    ld.out = StateOut{d->ping[0][0], d->ping[0][1], d->ping[0][2], d->ppitch};
+    for (int f = 0; f < 3; ++f) ld.snap[f] = r.out[f];
+    ld.edge = d->edge_buf[0];
+    ld.edge_rows = d->dd.edge_rows;
+    ld.slots = d->slots;
+    ld.nslots = d->slots_cap * kWarpsPerCta;
     return SWE_OK;
 }
 
-// The run's ledger into the control block from the slots of the step warps of
-// `ncta` CTAs.
-int fold_ledger(swe_domain* d, int ncta, cudaStream_t st) {
-    ledger_fold_kernel<kThreads><<<1, kThreads, 0, st>>>(d->dd, d->ctl, d->slots, ncta * kWarpsPerCta);
+// Start of one run: control block, state, first CFL maximum and volume (two launches).
+int begin_run(swe_domain* d, const RunStart& r, cudaStream_t st) {
+    InitBatch<1, kInlineTimes> ib;
+    LoadBatch<1> lb;
+    lb.n = 1;
+    const int rc = prepare_start(d, r, 0, d->sms, ib.d[0], lb.d[0], st);
+    if (rc) return rc;
+    control_init_kernel<1, kInlineTimes><<<1, 128, 0, st>>>(ib);
+    launch_load(lb, lb.d[0].gx * lb.d[0].gy, d->arith, st);
     SWE_CK(cudaGetLastError());
     return SWE_OK;
+}
+
+// Start of the members' runs of an ensemble (two launches per kBatchDomains members).
+int begin_runs(const std::vector<swe_domain*>& doms, const std::vector<RunStart>& runs, int sms, cudaStream_t st) {
+    for (size_t m0 = 0; m0 < doms.size(); m0 += kBatchDomains) {
+        const int n = (int)std::min<size_t>(kBatchDomains, doms.size() - m0);
+        InitBatch<kBatchDomains, 2> ib;
+        LoadBatch<kBatchDomains> lb;
+        lb.n = n;
+        int ctas = 0;
+        for (int i = 0; i < n; ++i) {
+            const int rc = prepare_start(doms[m0 + i], runs[m0 + i], ctas, std::max(1, sms / n), ib.d[i], lb.d[i], st);
+            if (rc) return rc;
+            ctas += lb.d[i].gx * lb.d[i].gy;
+        }
+        control_init_kernel<kBatchDomains, 2><<<n, 128, 0, st>>>(ib);
+        launch_load(lb, ctas, doms[0]->arith, st);
+        SWE_CK(cudaGetLastError());
+    }
+    return SWE_OK;
+}
+
+// End of runs: their ledgers from the slots of the step warps of ncta[i] CTAs and
+// their summaries into host memory (doms[i]->host->run, valid once the stream has
+// been waited for), and, where dst is given, the final states into the callers' planes.
+struct RunPlanes {
+    float* p[3];
+    int64_t pitch;
+};
+
+template <int ND>
+int end_batch(swe_domain* const* doms, const int* ncta, const RunPlanes* dst, int n, int sms, cudaStream_t st) {
+    FoldBatch<ND> fb;
+    StoreBatch<ND> sb;
+    sb.n = n;
+    int ctas = 0;
+    for (int i = 0; i < n; ++i) {
+        swe_domain* d = doms[i];
+        fb.d[i] = FoldDomain{d->dd.dx * d->dd.dy, d->ctl, d->slots, ncta[i] * kWarpsPerCta, &d->host->run};
+        if (!dst) continue;
+        const dim3 g = load_grid(d, std::max(1, sms / n));
+        StoreDomain& q = sb.d[i];
+        q.rows = d->dd.rows;
+        q.cols = d->dd.cols;
+        q.gx = (int)g.x;
+        q.gy = (int)g.y;
+        q.cta0 = ctas;
+        ctas += q.gx * q.gy;
+        for (int b = 0; b < 2; ++b)
+            for (int f = 0; f < 3; ++f) q.src[b][f] = d->ping[b][f];
+        q.spitch = d->ppitch;
+        for (int f = 0; f < 3; ++f) q.dst[f] = dst[i].p[f];
+        q.dpitch = dst[i].pitch;
+        q.ctl = d->ctl;
+    }
+    ledger_fold_kernel<256, ND><<<n, 256, 0, st>>>(fb);
+    if (dst) store_kernel<kThreads, ND><<<ctas, kThreads, 0, st>>>(sb);
+    SWE_CK(cudaGetLastError());
+    return SWE_OK;
+}
+
+int end_run(swe_domain* d, int ncta, const RunPlanes* dst, cudaStream_t st) {
+    return end_batch<1>(&d, &ncta, dst, 1, d->sms, st);
+}
+
+void fill_result(const swe_domain* d, swe_run_result* r) {
+    const RunSummary& c = d->host->run;
+    r->final_time_s = c.t;
+    r->outputs_written = c.idx;
+    r->steps_used = c.steps;
+    r->status = c.status;
+    r->reserved = 0;
+    for (int i = 0; i < 6; ++i) r->ledger[i] = c.ledger[i];
 }
 
 // Steps per poll of the run driver and at most per captured step graph.
@@ -590,18 +678,15 @@ int enqueue_run_steps(swe_domain* d, int64_t k0, int64_t n, cudaStream_t st, boo
     return SWE_OK;
 }
 
-// Shared run driver for swe_run and swe_advance.
-int run_driver(swe_domain* d, StateView init, const float* times_host, int n_times,
-               double t_start, int n_out, int max_steps, float* out_h, float* out_hu,
-               float* out_hv, swe_run_result* res, cudaStream_t st, int* final_buf,
-               const double* times64_host = nullptr, double* dt_log = nullptr) {
+// Shared run driver for swe_run, swe_advance and swe_advance_to; the final state goes to `dst` (or nowhere).
+int run_driver(swe_domain* d, const RunStart& r, const RunPlanes* dst, swe_run_result* res, cudaStream_t st) {
+    const int max_steps = r.max_steps;
     int rc = ensure_ping(d);
     if (rc) return rc;
     const Plan pl = make_plan(d, d->run_vec, true);
     rc = ensure_parts(d, std::max(pl.blocks, reduce_blocks(d)));
     if (rc) return rc;
-    rc = begin_run(d, init, times_host, n_times, t_start, n_out, max_steps, out_h, out_hu, out_hv, st,
-                   times64_host, dt_log);
+    rc = begin_run(d, r, st);
     if (rc) return rc;
     int64_t launched = 0;
     d->launches = 1;
@@ -632,18 +717,11 @@ int run_driver(swe_domain* d, StateView init, const float* times_host, int n_tim
         d->timed_steps = launched;
         d->timed_valid = true;
     }
-    rc = fold_ledger(d, pl.blocks, st);
+    rc = end_run(d, pl.blocks, dst, st);
     if (rc) return rc;
     SWE_CK(cudaStreamSynchronize(st));
-    SWE_CK(cudaMemcpy(&d->ctl_host[0], d->ctl, kControlHead, cudaMemcpyDeviceToHost));
-    const Control& c = d->ctl_host[0];
-    res->final_time_s = c.t;
-    res->outputs_written = c.idx;
-    res->steps_used = c.steps;
-    res->status = c.status ? c.status : (c.idx >= n_out ? SWE_OK : SWE_ERR_MAX_STEPS);
-    res->reserved = 0;
-    for (int i = 0; i < 6; ++i) res->ledger[i] = c.ledger[i];
-    if (final_buf) *final_buf = c.steps & 1;
+    fill_result(d, res);
+    if (!res->status && res->outputs_written < r.n_out) res->status = SWE_ERR_MAX_STEPS;
     return SWE_OK;
 }
 
@@ -898,40 +976,26 @@ int ens_graph(swe_ensemble* e, int K) {
     return SWE_OK;
 }
 
-// Reads every member's Control block, fills its run result and copies its
-// final planes to the caller's buffers.  Error statuses: any member's, the
+// Fills every member's run result and copies its final planes to the caller's buffers.  Error statuses: any member's, the
 // first one met; a member short of its target counts only when need_target.
 int ens_collect(swe_ensemble* e, float* const* h, float* const* hu, float* const* hv, const int64_t* pitch,
                 swe_run_result* results, cudaStream_t st, bool need_target) {
     const int n = (int)e->doms.size();
-    // Every member's ledger fold and control-block read are queued first and
-    // waited for once; the final states are then copied out in stream order.
-    for (int m = 0; m < n; ++m) {
-        swe_domain* d = e->doms[m];
-        const int rc = fold_ledger(d, e->member_ncta[m], st);
+    // Every member's ledger fold and final state are queued, then waited for once.
+    std::vector<RunPlanes> dst(n);
+    for (int m = 0; m < n; ++m) dst[m] = RunPlanes{{h[m], hu[m], hv[m]}, pitch[m]};
+    for (int m0 = 0; m0 < n; m0 += kBatchDomains) {
+        const int rc = end_batch<kBatchDomains>(e->doms.data() + m0, e->member_ncta.data() + m0, dst.data() + m0,
+                                                std::min(kBatchDomains, n - m0), e->sms, st);
         if (rc) return rc;
-        SWE_CK(cudaMemcpyAsync(&d->ctl_host[0], d->ctl, kControlHead, cudaMemcpyDeviceToHost, st));
     }
     SWE_CK(cudaStreamSynchronize(st));
     int status = SWE_OK;
     for (int m = 0; m < n; ++m) {
         swe_domain* d = e->doms[m];
-        const Control& c = d->ctl_host[0];
-        swe_run_result& r = results[m];
-        r.final_time_s = c.t;
-        r.outputs_written = c.idx;
-        r.steps_used = c.steps;
-        r.status = c.status;
-        r.reserved = 0;
-        for (int i = 0; i < 6; ++i) r.ledger[i] = c.ledger[i];
-        if (c.status && !status) status = c.status;
-        if (need_target && !c.done && !status) status = SWE_ERR_MAX_STEPS;
-        float* outs[3] = {h[m], hu[m], hv[m]};
-        const int fb = c.steps & 1;
-        for (int f = 0; f < 3; ++f) {
-            const int rc = copy_plane(outs[f], pitch[m], d->ping[fb][f], d->ppitch, d->dd.rows, d->dd.cols, st);
-            if (rc) return rc;
-        }
+        fill_result(d, &results[m]);
+        if (results[m].status && !status) status = results[m].status;
+        if (need_target && !d->host->run.done && !status) status = SWE_ERR_MAX_STEPS;
     }
     if (status == SWE_ERR_NONFINITE) return fail(SWE_ERR_NONFINITE, "non-finite values reached a member's CFL reduction");
     if (status == SWE_ERR_MAX_STEPS) return fail(status, "an ensemble member did not reach its target time");
@@ -1216,7 +1280,8 @@ int swe_domain_create(const swe_domain_desc* desc, swe_domain_t* out) {
     SWE_CK2(cudaMalloc(&d->ctl_scratch, sizeof(Control)));
     SWE_CK2(cudaMemset(d->ctl, 0, sizeof(Control)));
     SWE_CK2(cudaMemset(d->ctl_scratch, 0, sizeof(Control)));
-    SWE_CK2(cudaMallocHost(&d->ctl_host, 2 * sizeof(Control)));
+    SWE_CK2(cudaMallocHost(&d->ctl_host, 2 * sizeof(Control) + sizeof(HostSlots)));
+    d->host = reinterpret_cast<HostSlots*>(d->ctl_host + 2);
     for (int i = 0; i < 2; ++i) SWE_CK2(cudaEventCreateWithFlags(&d->poll_ev[i], cudaEventDisableTiming));
 #undef SWE_CK2
 
@@ -1482,12 +1547,15 @@ int swe_max_inverse_dt(swe_domain_t d, const float* h, const float* hu, const fl
     rc = ensure_parts(d, reduce_blocks(d));
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    SWE_CK(cudaMemsetAsync(d->ctl_scratch, 0, sizeof(Control), st));
-    launch_reduce(d, StateView{h, hu, hv, pitch}, d->ctl_scratch, st);
+    // The scratch control block stays zero but for what the reduction itself sets.
+    LoadBatch<1> lb;
+    lb.n = 1;
+    lb.d[0] = load_part(d, StateView{h, hu, hv, pitch}, d->ctl_scratch, 0, d->sms);
+    lb.d[0].host_max = &d->host->max_inverse_dt;
+    launch_load(lb, lb.d[0].gx * lb.d[0].gy, d->arith, st);
     SWE_CK(cudaGetLastError());
-    SWE_CK(cudaMemcpyAsync(&d->ctl_host[0], d->ctl_scratch, kControlHead, cudaMemcpyDeviceToHost, st));
     SWE_CK(cudaStreamSynchronize(st));
-    *max_inverse_dt_out = d->ctl_host[0].maxinv;
+    *max_inverse_dt_out = d->host->max_inverse_dt;
     return SWE_OK;
 }
 
@@ -1522,9 +1590,11 @@ int swe_run(swe_domain_t d, const float* h0, const float* hu0, const float* hv0,
             return fail(SWE_ERR_INVALID, "Output times must be one-dimensional, start at zero, and increase.");
     if (max_steps < 0) return fail(SWE_ERR_INVALID, "max_steps must be >= 0");
     if (!out_h || !out_hu || !out_hv) return fail(SWE_ERR_INVALID, "output buffers are required");
-    rc = run_driver(d, StateView{h0, hu0, hv0, pitch_in}, output_times, n_out,
-                    (double)output_times[0], n_out, max_steps, out_h, out_hu, out_hv, result,
-                    static_cast<cudaStream_t>(stream), nullptr);
+    RunStart r{StateView{h0, hu0, hv0, pitch_in}, (double)output_times[0], n_out, max_steps, output_times, n_out};
+    r.out[0] = out_h;
+    r.out[1] = out_hu;
+    r.out[2] = out_hv;
+    rc = run_driver(d, r, nullptr, result, static_cast<cudaStream_t>(stream));
     if (rc) return rc;
     if (result->status == SWE_ERR_MAX_STEPS) {
         char msg[256];
@@ -1576,8 +1646,12 @@ int swe_run_host(swe_domain_t d, const float* h0, const float* hu0, const float*
     float* sh = d->snap_dev;
     float* shu = sh + (int64_t)n_out * plane;
     float* shv = shu + (int64_t)n_out * plane;
-    rc = begin_run(d, StateView{d->ping[1][0], d->ping[1][1], d->ping[1][2], d->ppitch}, output_times, n_out,
-                   (double)output_times[0], n_out, max_steps, sh, shu, shv, st);
+    RunStart r{StateView{d->ping[1][0], d->ping[1][1], d->ping[1][2], d->ppitch}, (double)output_times[0], n_out,
+               max_steps, output_times, n_out};
+    r.out[0] = sh;
+    r.out[1] = shu;
+    r.out[2] = shv;
+    rc = begin_run(d, r, st);
     if (rc) return rc;
     float* host[3] = {out_h, out_hu, out_hv};
     float* dev[3] = {sh, shu, shv};
@@ -1621,21 +1695,15 @@ int swe_run_host(swe_domain_t d, const float* h0, const float* hu0, const float*
         }
         ++chunk;
     }
-    rc = fold_ledger(d, pl.blocks, st);
+    rc = end_run(d, pl.blocks, nullptr, st);
     if (rc) return rc;
     SWE_CK(cudaStreamSynchronize(st));
-    SWE_CK(cudaMemcpy(&d->ctl_host[0], d->ctl, kControlHead, cudaMemcpyDeviceToHost));
-    const Control& c = d->ctl_host[0];
+    fill_result(d, result);
     SWE_CK(cudaEventRecord(d->snap_ev, st));
-    rc = copy_out(std::min(c.idx, n_out), d->snap_ev);
+    rc = copy_out(std::min(result->outputs_written, n_out), d->snap_ev);
     if (rc) return rc;
     SWE_CK(cudaStreamSynchronize(d->copy_stream));
-    result->final_time_s = c.t;
-    result->outputs_written = c.idx;
-    result->steps_used = c.steps;
-    result->status = c.status ? c.status : (c.idx >= n_out ? SWE_OK : SWE_ERR_MAX_STEPS);
-    result->reserved = 0;
-    for (int i = 0; i < 6; ++i) result->ledger[i] = c.ledger[i];
+    if (!result->status && result->outputs_written < n_out) result->status = SWE_ERR_MAX_STEPS;
     if (result->status == SWE_ERR_MAX_STEPS) {
         char msg[256];
         std::snprintf(msg, sizeof msg, "max_steps=%d wrote %d/%d outputs; last time=%.3f s.", max_steps,
@@ -1654,19 +1722,12 @@ int swe_advance(swe_domain_t d, float* h, float* hu, float* hv, int64_t pitch, i
     if (n_steps < 0) return fail(SWE_ERR_INVALID, "n_steps must be >= 0");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float times[2] = {(float)start_s, INFINITY};
-    int fb = 0;
-    rc = run_driver(d, StateView{h, hu, hv, pitch}, times, 2, start_s, 2, n_steps, nullptr,
-                    nullptr, nullptr, result, st, &fb);
+    const RunPlanes dst{{h, hu, hv}, pitch};
+    rc = run_driver(d, RunStart{StateView{h, hu, hv, pitch}, start_s, 2, n_steps, times, 2}, &dst, result, st);
     if (rc) return rc;
     if (result->status == SWE_ERR_NONFINITE)
         return fail(SWE_ERR_NONFINITE, "non-finite values reached the CFL reduction");
     result->status = SWE_OK;
-    float* outs[3] = {h, hu, hv};
-    for (int f = 0; f < 3; ++f) {
-        rc = copy_plane(outs[f], pitch, d->ping[fb][f], d->ppitch, d->dd.rows, d->dd.cols, st);
-        if (rc) return rc;
-    }
-    SWE_CK(cudaStreamSynchronize(st));
     return SWE_OK;
 }
 
@@ -1685,7 +1746,7 @@ int swe_resident_load(swe_domain_t d, const float* h, const float* hu, const flo
     // An open-ended run: no output target within reach and no step cap, so the
     // control block stops the steps only on a non-finite CFL maximum.
     const float times[2] = {(float)start_s, INFINITY};
-    rc = begin_run(d, StateView{h, hu, hv, pitch}, times, 2, start_s, 2, INT32_MAX, nullptr, nullptr, nullptr,
+    rc = begin_run(d, RunStart{StateView{h, hu, hv, pitch}, start_s, 2, INT32_MAX, times, 2},
                    static_cast<cudaStream_t>(stream));
     if (rc) return rc;
     d->resident = true;
@@ -1722,24 +1783,13 @@ int swe_resident_store(swe_domain_t d, float* h, float* hu, float* hv, int64_t p
     int rc = check_state_ptrs(h, hu, hv, pitch, d->dd.cols);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int fb = (int)(d->resident_steps & 1);
-    float* outs[3] = {h, hu, hv};
-    for (int f = 0; f < 3; ++f) {
-        rc = copy_plane(outs[f], pitch, d->ping[fb][f], d->ppitch, d->dd.rows, d->dd.cols, st);
-        if (rc) return rc;
-    }
-    rc = fold_ledger(d, make_plan(d, d->run_vec, true).blocks, st);
+    const RunPlanes dst{{h, hu, hv}, pitch};
+    rc = end_run(d, make_plan(d, d->run_vec, true).blocks, &dst, st);
     if (rc) return rc;
-    SWE_CK(cudaMemcpyAsync(&d->ctl_host[0], d->ctl, kControlHead, cudaMemcpyDeviceToHost, st));
     SWE_CK(cudaStreamSynchronize(st));
-    const Control& c = d->ctl_host[0];
-    result->final_time_s = c.t;
+    fill_result(d, result);
     result->outputs_written = 0;
-    result->steps_used = c.steps;
-    result->status = c.status;
-    result->reserved = 0;
-    for (int i = 0; i < 6; ++i) result->ledger[i] = c.ledger[i];
-    if (c.status == SWE_ERR_NONFINITE) return fail(SWE_ERR_NONFINITE, "non-finite values reached the CFL reduction");
+    if (result->status == SWE_ERR_NONFINITE) return fail(SWE_ERR_NONFINITE, "non-finite values reached the CFL reduction");
     return SWE_OK;
 }
 
@@ -1752,16 +1802,12 @@ int swe_advance_to(swe_domain_t d, float* h, float* hu, float* hv, int64_t pitch
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float times[2] = {(float)t_start, (float)t_target};
     const double times64[2] = {t_start, t_target};
-    int fb = 0;
-    rc = run_driver(d, StateView{h, hu, hv, pitch}, times, 2, t_start, 2, max_steps, nullptr, nullptr, nullptr,
-                    result, st, &fb, times64, dt_log);
+    RunStart r{StateView{h, hu, hv, pitch}, t_start, 2, max_steps, times, 2};
+    r.times64 = times64;
+    r.dt_log = dt_log;
+    const RunPlanes dst{{h, hu, hv}, pitch};
+    rc = run_driver(d, r, &dst, result, st);
     if (rc) return rc;
-    float* outs[3] = {h, hu, hv};
-    for (int f = 0; f < 3; ++f) {
-        rc = copy_plane(outs[f], pitch, d->ping[fb][f], d->ppitch, d->dd.rows, d->dd.cols, st);
-        if (rc) return rc;
-    }
-    SWE_CK(cudaStreamSynchronize(st));
     if (result->status == SWE_ERR_NONFINITE) return fail(SWE_ERR_NONFINITE, "non-finite values reached the CFL reduction");
     if (result->status == SWE_ERR_MAX_STEPS) {
         char msg[160];
@@ -2136,16 +2182,18 @@ int swe_ensemble_advance(swe_ensemble_t e, float* const* h, float* const* hu, fl
     if (n_steps < 0) return fail(SWE_ERR_INVALID, "n_steps must be >= 0");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int n = (int)e->doms.size();
+    std::vector<RunStart> runs(n);
+    std::vector<float> times(2 * n);
     for (int m = 0; m < n; ++m) {
-        swe_domain* d = e->doms[m];
-        int rc = check_state_ptrs(h[m], hu[m], hv[m], pitch[m], d->dd.cols);
+        const int rc = check_state_ptrs(h[m], hu[m], hv[m], pitch[m], e->doms[m]->dd.cols);
         if (rc) return rc;
         const double t0 = start_s ? start_s[m] : 0.0;
-        const float times[2] = {(float)t0, INFINITY};
-        rc = begin_run(d, StateView{h[m], hu[m], hv[m], pitch[m]}, times, 2, t0, 2, n_steps, nullptr,
-                       nullptr, nullptr, st);
-        if (rc) return rc;
+        times[2 * m] = (float)t0;
+        times[2 * m + 1] = INFINITY;
+        runs[m] = RunStart{StateView{h[m], hu[m], hv[m], pitch[m]}, t0, 2, n_steps, &times[2 * m], 2};
     }
+    const int brc = begin_runs(e->doms, runs, e->sms, st);
+    if (brc) return brc;
     const int K = 50;
     e->timed_valid = false;
     if (e->timing) {
@@ -2186,19 +2234,25 @@ int swe_ensemble_advance_to(swe_ensemble_t e, float* const* h, float* const* hu,
         SWE_CK(cudaEventCreateWithFlags(&e->poll_ev[1], cudaEventDisableTiming));
     }
     SWE_CK(cudaMemsetAsync(e->done_counter, 0, sizeof(unsigned), st));
+    std::vector<RunStart> runs(n);
+    std::vector<float> times(2 * n);
+    std::vector<double> times64(2 * n);
     for (int m = 0; m < n; ++m) {
-        swe_domain* d = e->doms[m];
-        int rc = check_state_ptrs(h[m], hu[m], hv[m], pitch[m], d->dd.cols);
+        const int rc = check_state_ptrs(h[m], hu[m], hv[m], pitch[m], e->doms[m]->dd.cols);
         if (rc) return rc;
         if (!(target_s >= start_s[m])) return fail(SWE_ERR_INVALID, "every start time must be <= the target");
-        const float times[2] = {(float)start_s[m], (float)target_s};
-        const double times64[2] = {start_s[m], target_s};
-        d->done_counter = e->done_counter;
-        rc = begin_run(d, StateView{h[m], hu[m], hv[m], pitch[m]}, times, 2, start_s[m], 2, max_steps, nullptr,
-                       nullptr, nullptr, st, times64, dt_logs ? dt_logs[m] : nullptr);
-        d->done_counter = nullptr;
-        if (rc) return rc;
+        times64[2 * m] = start_s[m];
+        times64[2 * m + 1] = target_s;
+        times[2 * m] = (float)start_s[m];
+        times[2 * m + 1] = (float)target_s;
+        RunStart& r = runs[m];
+        r = RunStart{StateView{h[m], hu[m], hv[m], pitch[m]}, start_s[m], 2, max_steps, &times[2 * m], 2};
+        r.times64 = &times64[2 * m];
+        r.dt_log = dt_logs ? dt_logs[m] : nullptr;
+        r.done_counter = e->done_counter;
     }
+    int rc = begin_runs(e->doms, runs, e->sms, st);
+    if (rc) return rc;
     // K-step graphs until every member is done.  The counter is read one
     // graph late so the host never waits on the graph just queued.
     const int K = 50;
@@ -2210,7 +2264,7 @@ int swe_ensemble_advance_to(swe_ensemble_t e, float* const* h, float* const* hu,
         }
         SWE_CK(cudaEventRecord(e->time_ev[0], st));
     }
-    int rc = ens_graph(e, K);
+    rc = ens_graph(e, K);
     if (rc) return rc;
     const int64_t max_graphs = ((int64_t)max_steps + K - 1) / K;
     int64_t g = 0;
@@ -2650,8 +2704,9 @@ int strip_begin(swe_domain* d, float* h, float* hu, float* hv, int64_t pitch, do
     rc = ensure_parts(d, std::max(make_plan(d, d->run_vec, true).blocks, reduce_blocks(d)));
     if (rc) return rc;
     const float times[2] = {(float)t0, INFINITY};
-    return begin_run(d, StateView{h, hu, hv, pitch}, times, 2, t0, 2, n_steps, nullptr, nullptr, nullptr, st,
-                     nullptr, nullptr, 1);
+    RunStart r{StateView{h, hu, hv, pitch}, t0, 2, n_steps, times, 2};
+    r.defer_plan = 1;
+    return begin_run(d, r, st);
 }
 
 void strip_step(swe_domain* d, int k, cudaStream_t st) {
@@ -2659,25 +2714,12 @@ void strip_step(swe_domain* d, int k, cudaStream_t st) {
     launch_step(d, pl, run_launch(d, pl, k), true, st);
 }
 
-int strip_finish(swe_domain* d, float* h, float* hu, float* hv, int64_t pitch, int n_steps, swe_run_result* r,
-                 cudaStream_t st) {
-    const int lrc = fold_ledger(d, make_plan(d, d->run_vec, true).blocks, st);
-    if (lrc) return lrc;
-    const int fb = n_steps & 1;
-    float* outs[3] = {h, hu, hv};
-    for (int f = 0; f < 3; ++f) {
-        const int rc = copy_plane(outs[f], pitch, d->ping[fb][f], d->ppitch, d->dd.rows, d->dd.cols, st);
-        if (rc) return rc;
-    }
-    SWE_CK(cudaMemcpyAsync(&d->ctl_host[0], d->ctl, kControlHead, cudaMemcpyDeviceToHost, st));
+int strip_finish(swe_domain* d, float* h, float* hu, float* hv, int64_t pitch, swe_run_result* r, cudaStream_t st) {
+    const RunPlanes dst{{h, hu, hv}, pitch};
+    const int rc = end_run(d, make_plan(d, d->run_vec, true).blocks, &dst, st);
+    if (rc) return rc;
     SWE_CK(cudaStreamSynchronize(st));
-    const Control& c = d->ctl_host[0];
-    r->final_time_s = c.t;
-    r->outputs_written = c.idx;
-    r->steps_used = c.steps;
-    r->status = c.status;
-    r->reserved = 0;
-    for (int i = 0; i < 6; ++i) r->ledger[i] = c.ledger[i];
+    fill_result(d, r);
     return SWE_OK;
 }
 
@@ -2903,7 +2945,7 @@ int swe_strips_advance(const swe_domain_t* strips, int32_t n, float* const* h, f
         }
     }
     if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(SWE_ERR_CUDA, "strip step launch failed");
-    for (int i = 0; i < n && !rc; ++i) rc = strip_finish(strips[i], h[i], hu[i], hv[i], pitch[i], n_steps, &results[i], st);
+    for (int i = 0; i < n && !rc; ++i) rc = strip_finish(strips[i], h[i], hu[i], hv[i], pitch[i], &results[i], st);
     cudaStreamSynchronize(st);
     if (rc) return rc;
     for (int i = 0; i < n; ++i)
@@ -2989,7 +3031,7 @@ int swe_strip_advance_nccl(swe_domain_t d, swe_comm_t comm, int32_t rank_below, 
     }
     if (!rc && cudaGetLastError() != cudaSuccess) rc = fail(SWE_ERR_CUDA, "strip step launch failed");
     if (!rc) rc = nccl_wait(api, comm, st);
-    if (!rc) rc = strip_finish(d, h, hu, hv, pitch, n_steps, result, st);
+    if (!rc) rc = strip_finish(d, h, hu, hv, pitch, result, st);
     if (rc) return rc;
     if (result->status) return fail(result->status, "the strip stopped with an error status");
     return SWE_OK;

@@ -176,59 +176,19 @@ struct Control {
 // Bytes of the control block the host reads back (everything before the maxima).
 constexpr size_t kControlHead = offsetof(Control, maxk);
 
-// The strip-boundary columns of state `s` into `edge` and, when `stat` is not
-// null, of the bed and n^2 into `stat` (the layouts of DomainDev::edge and
-// edge_static).  Grid: x over the rows, y over the boundaries.  Cells outside
-// the grid (left of boundary 0, right of the last) are left as they are.
-__global__ void edge_fill_kernel(const DomainDev d, const StateView s, float* edge, float* stat) {
+// The bed and n^2 of the strip-boundary columns into `stat` (the layout of
+// DomainDev::edge_static).  Grid: x over the rows, y over the boundaries.  Cells
+// outside the grid (left of boundary 0, right of the last) are left as they are.
+__global__ void edge_fill_kernel(const DomainDev d, float* stat) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     if (r >= d.rows) return;
     for (int side = 0; side < 2; ++side) {
         const int x = kEdgeStrip * b - 1 + side;
         if (x < 0 || x >= d.cols) continue;
-        if (edge) {
-            const int64_t so = (int64_t)r * s.pitch + x;
-            edge[edge_index(d, b, 3 * side + 0, r)] = s.h[so];
-            edge[edge_index(d, b, 3 * side + 1, r)] = s.hu[so];
-            edge[edge_index(d, b, 3 * side + 2, r)] = s.hv[so];
-        }
-        if (stat) {
-            const int64_t zo = (int64_t)r * d.spitch + x;
-            stat[edge_static_index(d, b, 2 * side + 0, r)] = d.bed[zo];
-            stat[edge_static_index(d, b, 2 * side + 1, r)] = d.nm[zo];
-        }
-    }
-}
-
-// A run's control block written from launch parameters: the head as the host
-// built it, the stripe maxima zeroed and up to two target times.  Parameters
-// are captured when the launch is queued, so the host needs no staging buffer,
-// and the queue never waits for the stream as a copy from pageable host memory
-// may.
-struct ControlHeadImage {
-    unsigned long long w[kControlHead / 8];
-};
-static_assert(kControlHead % 8 == 0 && sizeof(ControlHeadImage) <= 2048, "control head must fit the launch parameters");
-
-constexpr int kInlineTimes = 64;  // output times carried in the launch parameters
-
-struct RunTargets {
-    int n;              // entries of t (and of t64, at most 2, when times64 is set) written
-    float t[kInlineTimes];
-    double t64[2];
-    float* times;       // device arrays receiving them (times64 may be null)
-    double* times64;
-};
-
-__global__ void control_init_kernel(Control* ctl, const ControlHeadImage head, const RunTargets tg) {
-    auto* dst = reinterpret_cast<unsigned long long*>(ctl);
-    for (int i = threadIdx.x; i < (int)(kControlHead / 8); i += blockDim.x) dst[i] = head.w[i];
-    unsigned long long* mk = &ctl->maxk[0][0];
-    for (int i = threadIdx.x; i < 2 * kMaxStripes * kStripeWords; i += blockDim.x) mk[i] = 0ull;
-    if ((int)threadIdx.x < tg.n) {
-        tg.times[threadIdx.x] = tg.t[threadIdx.x];
-        if (tg.times64 && threadIdx.x < 2) tg.times64[threadIdx.x] = tg.t64[threadIdx.x];
+        const int64_t zo = (int64_t)r * d.spitch + x;
+        stat[edge_static_index(d, b, 2 * side + 0, r)] = d.bed[zo];
+        stat[edge_static_index(d, b, 2 * side + 1, r)] = d.nm[zo];
     }
 }
 
@@ -640,86 +600,6 @@ __device__ __forceinline__ Partial cta_reduce(Accum acc) {
     return p;
 }
 
-// End of the reduction that starts a run (reduce_kernel): the CTA partials are
-// folded by the last CTA to arrive, in a fixed order, into the initial volume
-// and CFL maximum, and the run's first position is set: clock at t_start,
-// output 0 taken as the initial state, the first target loaded, the maximum
-// stored for step 0 (step count 0 in the high word of stripe 0).
-//
-// PER: partials a thread of the last CTA loads before folding them.
-template <int THREADS, int PER = 8>
-__device__ void finish_start(const DomainDev& d, Control* ctl, Partial* parts, Accum acc) {
-    const int nparts = (int)(gridDim.x * gridDim.y);
-    __shared__ bool s_last;
-    const Partial p = cta_reduce<THREADS>(acc);
-    if (threadIdx.x == 0) {
-        parts[blockIdx.y * gridDim.x + blockIdx.x] = p;
-        __threadfence();
-        const unsigned ticket = atomicAdd(&ctl->counter, 1u);
-        s_last = (ticket == (unsigned)nparts - 1);
-    }
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // Fixed-order fold of all CTA partials: thread t folds partials t, t+T, ...,
-    // a batch of them loaded from the L2 (.cg: the other CTAs' writes are
-    // visible there after the fence) with every load in flight at once.
-    Accum a;
-    a.zero();
-    constexpr int kPer = PER;
-    for (int base = threadIdx.x; base < nparts; base += kPer * THREADS) {
-        Partial buf[kPer];
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            const int b = base + j * THREADS;
-            if (b < nparts) {
-                buf[j].maxinv = __ldcg(&parts[b].maxinv);
-                buf[j].vol = __ldcg(&parts[b].vol);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < kPer; ++j) {
-            if (base + j * THREADS < nparts) {
-                a.maxinv = nan_max(a.maxinv, buf[j].maxinv);
-                a.vol += buf[j].vol;
-            }
-        }
-    }
-    const Partial t = cta_reduce<THREADS>(a);
-    if (threadIdx.x != 0) return;
-    float mx = t.maxinv;
-    // A NaN volume means a non-finite state somewhere: report it as a NaN CFL
-    // maximum, the form plan_step tests.
-    if (!(t.vol == t.vol)) mx = __int_as_float(0x7fffffff);
-    const double area = d.dx * d.dy;
-    const int n_out = ctl->n_out;
-    RunPos p0;
-    p0.t = ctl->t_start;
-    p0.target = n_out > 1 ? output_time(ctl, 1) : 0.0;
-    p0.rain = RainSeg{0.0, 0.0, 0.0, 0.0, 0.0, -1};
-    p0.steps = 0;
-    p0.idx = 1;
-    p0.done = (1 >= n_out || ctl->max_steps <= 0) ? 1 : 0;
-    p0.status = 0;
-    ctl->pos[0] = p0;
-    ctl->t = p0.t;
-    ctl->dt = 0.0;
-    ctl->idx = 1;
-    ctl->steps = 0;
-    ctl->done = p0.done;
-    ctl->status = 0;
-    ctl->ledger[0] = t.vol * area;
-    ctl->ledger[1] = t.vol * area;
-    ctl->ledger[2] = ctl->ledger[3] = ctl->ledger[4] = ctl->ledger[5] = 0.0;
-    // A row strip plans from the maximum across strips: NaN is kept as +inf
-    // there, so that a maximum carries it.
-    ctl->maxinv = (ctl->defer_plan && !(mx == mx)) ? INFINITY : mx;
-    ctl->maxk[0][0] = (unsigned long long)(__float_as_uint(mx) & 0x7fffffffu);
-    ctl->counter = 0;
-    if (p0.done && ctl->done_counter) atomicAdd(ctl->done_counter, 1u);
-    __threadfence();
-}
-
 // The CFL maximum of the state with `steps` steps taken, from the words of
 // parity `par` (one load per lane).
 __device__ __forceinline__ float stripes_maxinv(const Control* c, int par, int steps) {
@@ -819,28 +699,6 @@ __device__ __forceinline__ void warp_end_step(Control* c, LedgerSlot* slot, cons
     slot->clip = old[2] + clip;
     slot->mask = old[3] + mask;
     atomicMax(&c->maxk[par ^ 1][stripe * kStripeWords], ((unsigned long long)(steps + 1) << 32) | m);
-}
-
-// The run's ledger from the warps' slots (one CTA, fixed order): the stored
-// volume of the last step and the rain, outflow, clip and mask terms summed over
-// the run.  With no step taken the volume stays the initial one.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS) ledger_fold_kernel(const DomainDev d, Control* ctl, const LedgerSlot* slots,
-                                                             int nslots) {
-    Accum a;
-    a.zero();
-    for (int b = threadIdx.x; b < nslots; b += THREADS) {
-        a.vol += slots[b].vol; a.rain += slots[b].rain; a.outflow += slots[b].outflow;
-        a.clip += slots[b].clip; a.mask += slots[b].mask;
-    }
-    const Partial t = cta_reduce<THREADS>(a);
-    if (threadIdx.x != 0) return;
-    const double area = d.dx * d.dy;
-    ctl->ledger[1] = ctl->steps > 0 ? t.vol * area : ctl->ledger[0];
-    ctl->ledger[2] = t.rain * area;
-    ctl->ledger[3] = t.outflow;
-    ctl->ledger[4] = t.clip * area;
-    ctl->ledger[5] = t.mask * area;
 }
 
 // A row strip's CFL maximum after its step, from the stripes of the step's
@@ -1157,30 +1015,6 @@ __device__ __forceinline__ void for_cells(int r0, int r1, int cols, F&& body) {
     for (int r = r0 + (int)blockIdx.y; r < r1; r += (int)gridDim.y)
         for (int c = (int)(blockIdx.x * blockDim.x + threadIdx.x); c < cols; c += (int)(gridDim.x * blockDim.x))
             body(r, c);
-}
-
-// Max inverse CFL dt and stored volume of a state (the reduction of
-// compute_cfl_dt, shallow_water_2d.py:269-273); initialises the run control.
-// A 2-D launch: each CTA's partial is slot blockIdx.y * gridDim.x + blockIdx.x.
-template <class M, int THREADS>
-__global__ void __launch_bounds__(THREADS) reduce_kernel(const DomainDev d, const StateView s,
-                                                         Control* ctl, Partial* parts) {
-    const Consts& k = d.k;
-    Accum acc;
-    acc.zero();
-    for_cells(d.upd_lo, d.upd_hi, d.cols, [&](int r, int c) {
-        const float h = s.h[(int64_t)r * s.pitch + c];
-        const float hu = s.hu[(int64_t)r * s.pitch + c];
-        const float hv = s.hv[(int64_t)r * s.pitch + c];
-        const bool act = active(d.nm[(int64_t)r * d.spitch + c]);
-        float u, v;
-        M::vel2(hu, hv, h, k.dry, u, v);
-        const float w = M::sqrt(M::mul(k.g, fmaxf(h, 0.0f)));
-        const float inv = M::add(M::div(M::add(fabsf(u), w), k.dx), M::div(M::add(fabsf(v), w), k.dy));
-        acc.maxinv = nan_max(acc.maxinv, act ? inv : 0.0f);
-        if (act) acc.vol += (double)h;
-    });
-    finish_start<THREADS>(d, ctl, parts, acc);
 }
 
 }  // namespace swe
