@@ -93,6 +93,7 @@ struct Plan {
 // waiting for the stream.
 struct HostSlots {
     RunSummary run;
+    RunProgress progress[2];  // polls of a run
     float max_inverse_dt;
 };
 
@@ -108,8 +109,7 @@ struct swe_domain {
     std::vector<double> rain_t, rain_r;
     Control* ctl = nullptr;          // run control (device)
     Control* ctl_scratch = nullptr;  // standalone reductions (device)
-    Control* ctl_host = nullptr;     // pinned poll slots [2]
-    HostSlots* host = nullptr;       // pinned words that kernels write (after the poll slots)
+    HostSlots* host = nullptr;       // pinned words that kernels write
     LedgerSlot* slots = nullptr;  // step warps' ledger slots (kept over a run)
     int slots_cap = 0;            // in CTAs (kWarpsPerCta slots each)
     StartPartial* rparts = nullptr;  // partials of the start reductions
@@ -446,7 +446,6 @@ struct RunStart {
     const double* times64 = nullptr;  // HOST float64 targets (n_times <= 2), or null
     float* out[3] = {nullptr, nullptr, nullptr};
     double* dt_log = nullptr;
-    unsigned* done_counter = nullptr;
     int defer_plan = 0;
 };
 
@@ -489,7 +488,6 @@ int prepare_start(swe_domain* d, const RunStart& r, int cta0, int sms, InitDomai
     c0.t_start = r.t_start;
     c0.times = d->times_dev;
     c0.times64 = r.times64 ? d->times64_dev : nullptr;
-    c0.done_counter = r.done_counter;
     c0.dt_log = r.dt_log;
     c0.defer_plan = r.defer_plan;
     c0.out_h = r.out[0];
@@ -678,9 +676,82 @@ int enqueue_run_steps(swe_domain* d, int64_t k0, int64_t n, cudaStream_t st, boo
     return SWE_OK;
 }
 
+// Steps k0 .. k0+n-1 of the current run one launch at a time (fewer than a graph's).
+void launch_run_steps(swe_domain* d, const Plan& pl, int64_t k0, int64_t n, cudaStream_t st) {
+    for (int64_t k = k0; k < k0 + n; ++k) launch_step(d, pl, run_launch(d, pl, k), true, st, true);
+}
+
+// Steps the run takes by an estimate from its position: the time left at the
+// current dt, and one more step for every output that shortens one.
+int64_t steps_expected(double t, double dt, double t_end, int steps, int outputs_left) {
+    const double left = dt > 0.0 ? std::ceil((t_end - t) / dt) + outputs_left : 1.0;
+    return steps + (int64_t)std::min(std::max(left, 1.0), 1.0e9);
+}
+
+// Steps a run until it is done or max_steps are queued.  The host polls the run's
+// position: on_poll(progress, event) is called with each, the event having
+// passed.  A run to a known end time is paced: after kProbe steps the host knows
+// dt, and it queues no more than the steps expected to be left, polling one chunk
+// late while more are, so that the stream neither runs dry in the middle nor works
+// off launches past the end (a launch that finds its run ended still takes 3 us on
+// 512^2; a 22-step interval used to queue 64).
+template <class OnPoll>
+int run_steps(swe_domain* d, const Plan& pl, int64_t max_steps, double t_end, int n_out, cudaStream_t st, OnPoll&& on_poll) {
+    constexpr int kProbe = 4;
+    const bool paced = std::isfinite(t_end);
+    int64_t launched = 0, expected = paced ? 2 * kProbe : max_steps;
+    bool finished = false;
+    int pending = -1, slot = 0;
+    auto poll = [&]() -> int {
+        run_progress_kernel<<<1, 32, 0, st>>>(d->ctl, &d->host->progress[slot]);
+        SWE_CK(cudaEventRecord(d->poll_ev[slot], st));
+        return SWE_OK;
+    };
+    auto consume = [&](int s) -> int {
+        SWE_CK(cudaEventSynchronize(d->poll_ev[s]));
+        const RunProgress c = d->host->progress[s];
+        finished = c.done != 0;
+        if (paced) expected = steps_expected(c.t, c.dt, t_end, c.steps, std::max(0, n_out - 1 - c.idx));
+        return on_poll(c, d->poll_ev[s]);
+    };
+    while (!finished && launched < max_steps) {
+        int rc = SWE_OK;
+        if (launched < expected) {
+            const int64_t most = paced && launched < 2 * kProbe ? kProbe : kChunk;
+            const int64_t n = std::min({most, expected - launched, max_steps - launched});
+            if (n == kChunk || !paced) {
+                rc = enqueue_run_steps(d, launched, n, st);
+                if (rc) return rc;
+            } else {
+                launch_run_steps(d, pl, launched, n, st);
+            }
+            launched += n;
+            d->launches += n;
+            rc = poll();
+            if (rc) return rc;
+            const int queued = slot;
+            slot ^= 1;
+            if (pending >= 0) rc = consume(pending);
+            pending = queued;
+        } else {
+            // Everything expected is queued: look where it got.
+            rc = consume(pending);
+            pending = -1;
+            if (!finished && expected <= launched) expected = launched + 1;
+        }
+        if (rc) return rc;
+    }
+    SWE_CK(cudaGetLastError());
+    return SWE_OK;
+}
+
+// The last target of a run in float64.
+double end_time(const RunStart& r) {
+    return r.times64 ? r.times64[r.n_times - 1] : (double)r.times[r.n_times - 1];
+}
+
 // Shared run driver for swe_run, swe_advance and swe_advance_to; the final state goes to `dst` (or nowhere).
 int run_driver(swe_domain* d, const RunStart& r, const RunPlanes* dst, swe_run_result* res, cudaStream_t st) {
-    const int max_steps = r.max_steps;
     int rc = ensure_ping(d);
     if (rc) return rc;
     const Plan pl = make_plan(d, d->run_vec, true);
@@ -688,33 +759,15 @@ int run_driver(swe_domain* d, const RunStart& r, const RunPlanes* dst, swe_run_r
     if (rc) return rc;
     rc = begin_run(d, r, st);
     if (rc) return rc;
-    int64_t launched = 0;
     d->launches = 1;
     d->timed_valid = false;
     if (d->timing) SWE_CK(cudaEventRecord(d->time_ev[0], st));
-    const int K = kChunk;
-    int chunk = 0;
-    bool finished = false;
-    while (!finished) {
-        const int64_t todo = std::min<int64_t>(K, (int64_t)max_steps - launched);
-        rc = enqueue_run_steps(d, launched, todo, st);
-        if (rc) return rc;
-        launched += todo;
-        d->launches += todo;
-        const int slot = chunk & 1;
-        SWE_CK(cudaMemcpyAsync(&d->ctl_host[slot], d->ctl, kControlHead, cudaMemcpyDeviceToHost, st));
-        SWE_CK(cudaEventRecord(d->poll_ev[slot], st));
-        if (launched >= max_steps) break;
-        if (chunk > 0) {
-            SWE_CK(cudaEventSynchronize(d->poll_ev[slot ^ 1]));
-            if (d->ctl_host[slot ^ 1].done) finished = true;
-        }
-        ++chunk;
-    }
+    rc = run_steps(d, pl, r.max_steps, end_time(r), r.n_out, st, [](const RunProgress&, cudaEvent_t) { return SWE_OK; });
+    if (rc) return rc;
     if (d->timing) {
         // The end event follows the last step kernel; poll copies in between are ~1 us each.
         SWE_CK(cudaEventRecord(d->time_ev[1], st));
-        d->timed_steps = launched;
+        d->timed_steps = d->launches - 1;
         d->timed_valid = true;
     }
     rc = end_run(d, pl.blocks, dst, st);
@@ -733,7 +786,7 @@ void free_domain(swe_domain* d) {
     cudaFree(d->rain);
     cudaFree(d->ctl);
     cudaFree(d->ctl_scratch);
-    if (d->ctl_host) cudaFreeHost(d->ctl_host);
+    if (d->host) cudaFreeHost(d->host);
     cudaFree(d->slots);
     cudaFree(d->rparts);
     for (int b = 0; b < 2; ++b)
@@ -809,8 +862,7 @@ struct swe_ensemble {
     bool timed_valid = false;
     int64_t timed_steps = 0;
     int64_t launches = 0;
-    unsigned* done_counter = nullptr;       // device: members finished in advance_to
-    unsigned* done_host = nullptr;          // pinned: two polled copies of it
+    EnsProgress* progress = nullptr;        // pinned: two polls of an advance_to
     cudaEvent_t poll_ev[2] = {nullptr, nullptr};
     // Member table in the kernel's parameter space (up to kEnsParamMembers
     // members; SWE_ENS_PARAM_TABLE=0 keeps the table in global memory).
@@ -1015,8 +1067,7 @@ void free_ensemble(swe_ensemble* e) {
         if (e->time_ev[i]) cudaEventDestroy(e->time_ev[i]);
         if (e->poll_ev[i]) cudaEventDestroy(e->poll_ev[i]);
     }
-    cudaFree(e->done_counter);
-    cudaFreeHost(e->done_host);
+    cudaFreeHost(e->progress);
     delete e;
 }
 
@@ -1280,8 +1331,7 @@ int swe_domain_create(const swe_domain_desc* desc, swe_domain_t* out) {
     SWE_CK2(cudaMalloc(&d->ctl_scratch, sizeof(Control)));
     SWE_CK2(cudaMemset(d->ctl, 0, sizeof(Control)));
     SWE_CK2(cudaMemset(d->ctl_scratch, 0, sizeof(Control)));
-    SWE_CK2(cudaMallocHost(&d->ctl_host, 2 * sizeof(Control) + sizeof(HostSlots)));
-    d->host = reinterpret_cast<HostSlots*>(d->ctl_host + 2);
+    SWE_CK2(cudaMallocHost(&d->host, sizeof(HostSlots)));
     for (int i = 0; i < 2; ++i) SWE_CK2(cudaEventCreateWithFlags(&d->poll_ev[i], cudaEventDisableTiming));
 #undef SWE_CK2
 
@@ -1672,29 +1722,10 @@ int swe_run_host(swe_domain_t d, const float* h0, const float* hu0, const float*
     if (rc) return rc;
     d->launches = 1;
     d->timed_valid = false;
-    int64_t launched = 0;
-    int chunk = 0;
-    for (;;) {
-        const int64_t todo = std::min<int64_t>(kChunk, (int64_t)max_steps - launched);
-        rc = enqueue_run_steps(d, launched, todo, st);
-        if (rc) return rc;
-        launched += todo;
-        d->launches += todo;
-        const int slot = chunk & 1;
-        SWE_CK(cudaMemcpyAsync(&d->ctl_host[slot], d->ctl, kControlHead, cudaMemcpyDeviceToHost, st));
-        SWE_CK(cudaEventRecord(d->poll_ev[slot], st));
-        if (launched >= max_steps) break;
-        if (chunk > 0) {
-            // The previous chunk has finished: outputs it recorded go to the host
-            // while the chunk just queued runs.
-            SWE_CK(cudaEventSynchronize(d->poll_ev[slot ^ 1]));
-            const Control& c = d->ctl_host[slot ^ 1];
-            rc = copy_out(std::min(c.idx, n_out), d->poll_ev[slot ^ 1]);
-            if (rc) return rc;
-            if (c.done) break;
-        }
-        ++chunk;
-    }
+    // Outputs a poll finds recorded go to the host while the later steps run.
+    rc = run_steps(d, pl, max_steps, end_time(r), n_out, st,
+                   [&](const RunProgress& c, cudaEvent_t ev) { return copy_out(std::min(c.idx, n_out), ev); });
+    if (rc) return rc;
     rc = end_run(d, pl.blocks, nullptr, st);
     if (rc) return rc;
     SWE_CK(cudaStreamSynchronize(st));
@@ -2227,13 +2258,11 @@ int swe_ensemble_advance_to(swe_ensemble_t e, float* const* h, float* const* hu,
     if (max_steps < 0) return fail(SWE_ERR_INVALID, "max_steps must be >= 0");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int n = (int)e->doms.size();
-    if (!e->done_counter) {
-        SWE_CK(cudaMalloc(&e->done_counter, sizeof(unsigned)));
-        SWE_CK(cudaHostAlloc(&e->done_host, 2 * sizeof(unsigned), cudaHostAllocDefault));
+    if (!e->progress) {
+        SWE_CK(cudaHostAlloc(&e->progress, 2 * sizeof(EnsProgress), cudaHostAllocDefault));
         SWE_CK(cudaEventCreateWithFlags(&e->poll_ev[0], cudaEventDisableTiming));
         SWE_CK(cudaEventCreateWithFlags(&e->poll_ev[1], cudaEventDisableTiming));
     }
-    SWE_CK(cudaMemsetAsync(e->done_counter, 0, sizeof(unsigned), st));
     std::vector<RunStart> runs(n);
     std::vector<float> times(2 * n);
     std::vector<double> times64(2 * n);
@@ -2249,13 +2278,12 @@ int swe_ensemble_advance_to(swe_ensemble_t e, float* const* h, float* const* hu,
         r = RunStart{StateView{h[m], hu[m], hv[m], pitch[m]}, start_s[m], 2, max_steps, &times[2 * m], 2};
         r.times64 = &times64[2 * m];
         r.dt_log = dt_logs ? dt_logs[m] : nullptr;
-        r.done_counter = e->done_counter;
     }
     int rc = begin_runs(e->doms, runs, e->sms, st);
     if (rc) return rc;
-    // K-step graphs until every member is done.  The counter is read one
-    // graph late so the host never waits on the graph just queued.
-    const int K = 50;
+    // K-step graphs, or single launches, until every member is done, paced as
+    // run_steps paces a run: by the largest number of steps a member is expected to need.
+    const int K = 50, kProbe = 4;
     e->timed_valid = false;
     if (e->timing) {
         if (!e->time_ev[0]) {
@@ -2264,27 +2292,45 @@ int swe_ensemble_advance_to(swe_ensemble_t e, float* const* h, float* const* hu,
         }
         SWE_CK(cudaEventRecord(e->time_ev[0], st));
     }
-    rc = ens_graph(e, K);
-    if (rc) return rc;
-    const int64_t max_graphs = ((int64_t)max_steps + K - 1) / K;
-    int64_t g = 0;
-    e->done_host[0] = e->done_host[1] = 0;
-    for (; g < max_graphs; ++g) {
-        SWE_CK(cudaGraphLaunch(e->graph, st));
-        SWE_CK(cudaMemcpyAsync(&e->done_host[g & 1], e->done_counter, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-        SWE_CK(cudaEventRecord(e->poll_ev[g & 1], st));
-        if (g > 0) {
-            SWE_CK(cudaEventSynchronize(e->poll_ev[(g - 1) & 1]));
-            if (e->done_host[(g - 1) & 1] >= (unsigned)n) {
-                ++g;
-                break;
+    int64_t launched = 0, expected = 2 * kProbe;
+    bool finished = false;
+    int pending = -1, slot = 0;
+    auto consume = [&](int s) -> int {
+        SWE_CK(cudaEventSynchronize(e->poll_ev[s]));
+        finished = e->progress[s].done >= n;
+        expected = e->progress[s].expected;
+        return SWE_OK;
+    };
+    while (!finished && launched < max_steps) {
+        if (launched < expected) {
+            const int64_t most = launched < 2 * kProbe ? kProbe : K;
+            const int64_t k = std::min({most, expected - launched, (int64_t)max_steps - launched});
+            if (k == K && launched % 2 == 0) {
+                rc = ens_graph(e, K);
+                if (rc) return rc;
+                SWE_CK(cudaGraphLaunch(e->graph, st));
+            } else {
+                for (int64_t i = launched; i < launched + k; ++i) ens_launch(e, (int)(i & 1), st, true);
             }
+            launched += k;
+            ens_progress_kernel<<<1, 128, 0, st>>>(e->members_dev, n, target_s, &e->progress[slot]);
+            SWE_CK(cudaEventRecord(e->poll_ev[slot], st));
+            const int queued = slot;
+            slot ^= 1;
+            if (pending >= 0) rc = consume(pending);
+            pending = queued;
+        } else {
+            rc = consume(pending);
+            pending = -1;
+            if (!finished && expected <= launched) expected = launched + 1;
         }
+        if (rc) return rc;
     }
-    e->launches = n + g * K;
+    SWE_CK(cudaGetLastError());
+    e->launches = n + launched;
     if (e->timing) {
         SWE_CK(cudaEventRecord(e->time_ev[1], st));
-        e->timed_steps = g * K;
+        e->timed_steps = launched;
         e->timed_valid = true;
     }
     return ens_collect(e, h, hu, hv, pitch, results, st, true);

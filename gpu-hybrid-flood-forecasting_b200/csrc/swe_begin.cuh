@@ -16,6 +16,7 @@
 
 #include "swe_exact.cuh"
 #include "swe_step.cuh"
+#include "swe_step_pair.cuh"
 
 namespace swe {
 
@@ -215,7 +216,6 @@ __device__ void finish_start(const LoadDomain& q, int cta, float maxinv, double 
     ctl->maxinv = shown;
     ctl->maxk[0][0] = (unsigned long long)(__float_as_uint(mx) & 0x7fffffffu);
     ctl->counter = 0;
-    if (p0.done && ctl->done_counter) atomicAdd(ctl->done_counter, 1u);
     if (q.host_max) *q.host_max = shown;
     __threadfence_system();
 }
@@ -392,6 +392,49 @@ __global__ void __launch_bounds__(THREADS) store_kernel(const __grid_constant__ 
                 q.dst[2][o] = x[j][2];
             }
         }
+}
+
+// A run's position, in host memory.  Written by a kernel and not copied: a copy of
+// a few words waits behind the outputs on their way to the host (0.9 ms for a
+// 2048^2 state), and the steps queued behind it with it.
+struct RunProgress {
+    double t, dt;
+    int idx, steps, done;
+};
+
+__global__ void run_progress_kernel(const Control* c, RunProgress* host) {
+    if (threadIdx.x) return;
+    *host = RunProgress{c->t, c->dt, c->idx, c->steps, c->done};
+    __threadfence_system();
+}
+
+// How far an ensemble's advance to a target time has come, in host memory: the
+// members that are done and the largest number of steps one is expected to take
+// (the time left at its current dt).
+struct EnsProgress {
+    int done;
+    long long expected;
+};
+
+__global__ void ens_progress_kernel(const MemberDev* members, int n, double target, EnsProgress* host) {
+    __shared__ int s_done, s_expected;
+    if (threadIdx.x == 0) s_done = s_expected = 0;
+    __syncthreads();
+    for (int m = threadIdx.x; m < n; m += blockDim.x) {
+        const Control* c = members[m].ctl;
+        if (c->done) {
+            atomicAdd(&s_done, 1);
+            continue;
+        }
+        const double left = c->dt > 0.0 ? fmin(fmax(ceil((target - c->t) / c->dt), 1.0), 1.0e9) : 1.0;
+        atomicMax(&s_expected, c->steps + (int)left);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        host->done = s_done;
+        host->expected = s_expected;
+        __threadfence_system();
+    }
 }
 
 }  // namespace swe

@@ -161,7 +161,6 @@ struct Control {
     double t_start;               // clock value set by the start reduction
     const float* times;           // device copy of the float32 output times
     const double* times64;        // float64 targets instead of `times` (advance_to), or null
-    unsigned* done_counter;       // incremented once when this run finishes (ensembles), or null
     double* dt_log;               // dt of every step (index = step number), or null
     float* out_h;                 // n_out x rows x cols snapshots (may be null)
     float* out_hu;
@@ -173,7 +172,7 @@ struct Control {
     alignas(128) unsigned long long maxk[2][kMaxStripes * kStripeWords];
 };
 
-// Bytes of the control block the host reads back (everything before the maxima).
+// Bytes of the control block the host writes (everything before the maxima).
 constexpr size_t kControlHead = offsetof(Control, maxk);
 
 // The bed and n^2 of the strip-boundary columns into `stat` (the layout of
@@ -441,7 +440,6 @@ struct PlanInputs {
     int defer, n_out, max_steps;
     const float* out_h;
     double* dt_log;
-    unsigned* done_counter;
 };
 
 // Issues the loads of a step's plan (every lane).  They are plain loads: the
@@ -462,7 +460,6 @@ __device__ __forceinline__ PlanInputs plan_fetch(const Control* c, int par) {
     in.max_steps = c->max_steps;
     in.out_h = c->out_h;
     in.dt_log = c->dt_log;
-    in.done_counter = c->done_counter;
     return in;
 }
 
@@ -617,20 +614,18 @@ __device__ __forceinline__ StepPlan warp_plan(const DomainDev& d, const Control*
 // The lead warp of a run (one per run and step) advances the run position into
 // the other parity's copy and publishes it: clock, step count, next output,
 // completion (set as soon as the last output is written or the step cap is
-// reached, so the host sees it after the step that ends the run), the dt log
-// and an ensemble's completion counter.  A finished run's position is copied
-// forward unchanged, so every later step of either parity sees it finished.
+// reached, so the host sees it after the step that ends the run) and the dt log.
+// A finished run's position is copied forward unchanged, so every later step of
+// either parity sees it finished.
 // Stores only, except the time of the next output when the step records one.
 __device__ __forceinline__ void lead_advance(Control* c, int par, const PlanInputs& in, const StepPlan& p) {
     if ((threadIdx.x & 31) != 0) return;
     const RunPos& pos = in.pos;
     RunPos q = pos;
-    int newly_done = 0;
     if (!pos.done) {
         if (!p.go) {
             q.done = 1;
             q.status = p.status;
-            newly_done = 1;
         } else {
             q.t = __dadd_rn(pos.t, p.dt);
             q.steps = pos.steps + 1;
@@ -640,7 +635,6 @@ __device__ __forceinline__ void lead_advance(Control* c, int par, const PlanInpu
                 if (q.idx < in.n_out) q.target = output_time(c, q.idx);
             }
             q.done = (q.idx >= in.n_out || q.steps >= in.max_steps) ? 1 : 0;
-            newly_done = q.done;
             if (in.dt_log) in.dt_log[pos.steps] = p.dt;  // steps < max_steps while not done
             c->dt = p.dt;
         }
@@ -651,7 +645,6 @@ __device__ __forceinline__ void lead_advance(Control* c, int par, const PlanInpu
     c->steps = q.steps;
     c->done = q.done;
     c->status = q.status;
-    if (newly_done && in.done_counter) atomicAdd(in.done_counter, 1u);
 }
 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
