@@ -847,6 +847,8 @@ struct swe_ensemble {
     int arith = SWE_ARITH_FAST;
     bool masked = false;
     int rows_per_warp = 128;  // provisional: swe_ensemble_create sets ens_auto_rows (B200Ensemble.autotune measures)
+    bool tuned = false;       // rows_per_warp was set by the caller (or SWE_ENSEMBLE_ROWS)
+    bool lead = false;        // the marches are a split of rows_per_warp that keeps its bits
     int sms = 148;
     MemberDev* members_dev = nullptr;
     int members_cap = 0;
@@ -879,7 +881,13 @@ void ens_launch_t(const swe_ensemble* e, int parity, cudaStream_t st, bool pdl) 
     attach_pdl(cfg, attr, pdl);
     if (e->params) {
         e->params->parity = parity;
-        cudaLaunchKernelEx(&cfg, ensemble_step_kernel_p<M, kThreads, MASKED>, *e->params);
+        if constexpr (!M::kExact) {
+            if (e->lead) {
+                cudaLaunchKernelEx(&cfg, ensemble_step_kernel_p<M, kThreads, MASKED, true>, *e->params);
+                return;
+            }
+        }
+        cudaLaunchKernelEx(&cfg, ensemble_step_kernel_p<M, kThreads, MASKED, false>, *e->params);
     } else {
         cudaLaunchKernelEx(&cfg, ensemble_step_kernel<M, kThreads, MASKED>, (const MemberDev*)e->members_dev,
                            (const int2*)e->items_dev, e->n_items, parity);
@@ -898,11 +906,11 @@ int ens_occupancy(const swe_ensemble* e) {
     const void* fn = nullptr;
     if (e->params) {
         if (e->arith == SWE_ARITH_FAST)
-            fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel_p<FastMath, kThreads, true>)
-                           : reinterpret_cast<const void*>(&ensemble_step_kernel_p<FastMath, kThreads, false>);
+            fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel_p<FastMath, kThreads, true, false>)
+                           : reinterpret_cast<const void*>(&ensemble_step_kernel_p<FastMath, kThreads, false, false>);
         else
-            fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel_p<ExactMath, kThreads, true>)
-                           : reinterpret_cast<const void*>(&ensemble_step_kernel_p<ExactMath, kThreads, false>);
+            fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel_p<ExactMath, kThreads, true, false>)
+                           : reinterpret_cast<const void*>(&ensemble_step_kernel_p<ExactMath, kThreads, false, false>);
     } else if (e->arith == SWE_ARITH_FAST)
         fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel<FastMath, kThreads, true>)
                        : reinterpret_cast<const void*>(&ensemble_step_kernel<FastMath, kThreads, false>);
@@ -914,37 +922,67 @@ int ens_occupancy(const swe_ensemble* e) {
     return n;
 }
 
+// Whether the member table travels in the launch parameters.
+bool ens_param_table(const swe_ensemble* e) {
+    const char* pt = std::getenv("SWE_ENS_PARAM_TABLE");
+    return (int)e->doms.size() <= kEnsParamMembers && !(pt && pt[0] == '0');
+}
+
+int64_t ens_items(const swe_ensemble* e, int R) {
+    int64_t n = 0;
+    for (const swe_domain* d : e->doms) {
+        const int64_t nstrips = (d->dd.cols + 2 * kWarp - 1) / (2 * kWarp);
+        const int64_t chunks = (d->dd.rows + R - 1) / R;
+        n += (chunks * nstrips + kWarpsPerCta - 1) / kWarpsPerCta;
+    }
+    return n;
+}
+
+// The smallest march of at least `lo` rows whose items fit `slots` (hi when none below it does).
+int ens_fit_rows(const swe_ensemble* e, int64_t slots, int lo, int hi) {
+    if (ens_items(e, lo) <= slots) return lo;
+    while (hi - lo > 1) {  // the item count does not grow with R
+        const int mid = (lo + hi) / 2;
+        if (ens_items(e, mid) <= slots) hi = mid; else lo = mid;
+    }
+    return hi;
+}
+
+constexpr int kEnsMinRows = kEnsSeam;  // the default's smallest value
+
 // Default rows per warp: the step of a batch that fits the persistent grid in
 // one round takes about as long as its longest march, so the default is the
 // smallest march (at least 32 rows) whose work items all fit in one round of
 // the grid; when even 1024-row marches need more than one round, 256.
-int ens_occupancy(const swe_ensemble* e);
 int ens_auto_rows(const swe_ensemble* e) {
-    const int wpb = kThreads / kWarp;
     const int64_t slots = (int64_t)ens_occupancy(e) * e->sms;
-    auto items = [&](int R) {
-        int64_t n = 0;
-        for (const swe_domain* d : e->doms) {
-            const int64_t nstrips = (d->dd.cols + 2 * kWarp - 1) / (2 * kWarp);
-            const int64_t chunks = (d->dd.rows + R - 1) / R;
-            n += (chunks * nstrips + wpb - 1) / wpb;
-        }
-        return n;
-    };
-    if (items(1024) > slots) return 256;
-    int lo = 32, hi = 1024;  // items(hi) <= slots; items is non-increasing in R
-    if (items(lo) <= slots) return lo;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) / 2;
-        if (items(mid) <= slots) hi = mid; else lo = mid;
-    }
-    return hi;
+    if (ens_items(e, 1024) > slots) return 256;
+    return ens_fit_rows(e, slots, kEnsMinRows, 1024);
+}
+
+// Rows the warps march.  An untuned batch that leaves CTA slots of the grid idle
+// at the default's smallest value is split further, as a single small grid is
+// (march_rows).  In fast arithmetic the split is a power of two of rows whose
+// marches, where they do not start on a seam of the 32-row ones, lead in with two
+// dropped rows, and the results keep every bit (march_pair).  us a step, fast, at
+// 32 rows and split: 4 x 512^2 28.1 and 18.6, 2 x 200^2 28.6 and 7.5; a batch that
+// fills most of the grid gains little (eight of 280^2 to 640^2: 32.0 and 29.2).
+int ens_march_rows(const swe_ensemble* e) {
+    if (e->tuned || e->rows_per_warp != kEnsMinRows || !ens_param_table(e)) return e->rows_per_warp;
+    const int one_wave = ens_fit_rows(e, (int64_t)ens_occupancy(e) * e->sms, 1, kEnsMinRows);
+    const int two_a_scheduler = ens_fit_rows(e, (int64_t)kFewWarps / kWarpsPerCta * e->sms, 1, kEnsMinRows);
+    const int rows = march_rows(one_wave, two_a_scheduler);
+    if (e->arith != SWE_ARITH_FAST) return rows;
+    int R = 2;
+    while (R < rows) R *= 2;
+    return R;
 }
 
 // Member table and work list for the current rows-per-warp.
 int ens_rebuild(swe_ensemble* e) {
     const int wpb = kThreads / kWarp;
-    const int R = e->rows_per_warp;
+    const int R = ens_march_rows(e);
+    e->lead = R < e->rows_per_warp && e->arith == SWE_ARITH_FAST;
     std::vector<MemberDev> md(e->doms.size());
     std::vector<int2> items;
     for (size_t m = 0; m < e->doms.size(); ++m) {
@@ -985,9 +1023,8 @@ int ens_rebuild(swe_ensemble* e) {
     SWE_CK(cudaMemcpy(e->members_dev, md.data(), sizeof(MemberDev) * md.size(), cudaMemcpyHostToDevice));
     SWE_CK(cudaMemcpy(e->items_dev, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice));
     e->n_items = (int)items.size();
-    const char* pt = std::getenv("SWE_ENS_PARAM_TABLE");
     e->params.reset();
-    if ((int)md.size() <= kEnsParamMembers && !(pt && pt[0] == '0')) {
+    if (ens_param_table(e)) {
         e->params.reset(new EnsParams());
         std::memset(e->params.get(), 0, sizeof(EnsParams));
         int b = 0;
@@ -2159,7 +2196,10 @@ int swe_ensemble_create(const swe_domain_desc* descs, int32_t n_members, swe_ens
     e->arith = descs[0].arithmetic;
     if (const char* v = std::getenv("SWE_ENSEMBLE_ROWS")) {
         const int r = std::atoi(v);
-        if (r > 0) e->rows_per_warp = r;
+        if (r > 0) {
+            e->rows_per_warp = r;
+            e->tuned = true;
+        }
     }
     for (int m = 0; m < n_members; ++m) {
         swe_domain_t d = nullptr;
@@ -2203,6 +2243,7 @@ int swe_ensemble_set_rows_per_warp(swe_ensemble_t e, int32_t rows_per_warp) {
     if (!e || rows_per_warp < 1) return fail(SWE_ERR_INVALID, "rows_per_warp must be >= 1");
     cudaDeviceSynchronize();
     e->rows_per_warp = rows_per_warp;
+    e->tuned = true;
     return ens_rebuild(e);
 }
 

@@ -82,6 +82,13 @@ __device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) { return __
 // values unused), which keeps the row body free of that branch; the plain step
 // measured 0.6 % faster with it, the ensemble kernel spills with it.
 //
+// LEAD: the first lead_rows rows (0 or 2) are a lead-in whose updates are dropped (the
+// chunk's own rows start at r0 + lead_rows): the face below its first row is then the
+// one a longer march evaluates there, by the same instructions, so that marches
+// cut shorter give the same bits.  (Which product of a flux and its pressure
+// correction the assembler fuses with their sum differs between a march's first
+// face and its rows, and between the two copies of a row in the loop.)
+//
 // Run mode, with epar >= 0: the domain keeps its strip-boundary columns
 // (DomainDev::edge) and `in` is ping-pong buffer epar.  The strip edges are then
 // read from edge[epar] (one coalesced access per quantity for 32 rows, where the
@@ -95,11 +102,13 @@ __device__ __forceinline__ float2 lfma(float2 a, float2 b, float2 c) { return __
 // fast 6.6 us a step instead of 7.5, 300 x 420 7.2 instead of 7.5).
 static_assert(kEdgeStrip == 2 * kWarp, "a paired-march strip is 2 x 32 columns");
 
-template <class M, bool RUN, bool MASKED, bool LAST_CONSUME, class EnterFn, class PlanFn>
+template <class M, bool RUN, bool MASKED, bool LAST_CONSUME, bool LEAD, class EnterFn, class PlanFn>
 __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& in,
                                             const StateOut& out, EnterFn&& enter_fn, PlanFn&& plan_fn, const Control* ctl,
-                                            int r0, int r1, int x0w, WarpSmem& sm, StepAccum& acc, int epar = -1) {
+                                            int r0, int r1, int x0w, WarpSmem& sm, StepAccum& acc, int epar = -1,
+                                            int lead_rows = 0) {
     constexpr int kBatch = kWarp;
+    const int lead = LEAD ? lead_rows : 0;
     using A = P<M>;
     const Consts& k = d.k;
     const KPair kp = make_kpair(k);
@@ -553,7 +562,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         sm.left[0][lane] = f.f0;
         sm.left[1][lane] = A::add(f.f1, f.corr_hi);
         sm.left[2][lane] = f.f2;
-        if (RUN && x0w == 0 && rb + lane < r1) lg.out_x.x -= f.f0;
+        if (RUN && x0w == 0 && rb + lane < r1 && (lead == 0 || rb + lane >= r0 + lead)) lg.out_x.x -= f.f0;
         sm.right[0][lane] = q.h;
         sm.right[1][lane] = q.z;
         sm.right[2][lane] = q.nm;
@@ -585,14 +594,14 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
                 evaluate(M{}, c, n);
             }
         }
-        account(cur, w, x);
+        if (lead == 0 || r >= r0 + lead) account(cur, w, x);
         if constexpr (RUN) {
             if (r == d.rows - 1) lg.out_y = lfma(fy.f0, vmask, lg.out_y);
         }
         yT0 = fy.f0;
         yT1 = fy.f1;
         yT2 = A::add(fy.f2, fy.corr_hi);
-        store(r, w.o);
+        if (lead == 0 || r >= r0 + lead) store(r, w.o);
         if (LAST_CONSUME || r + 1 < r1) big_cur = consume(r + 3 - r0, cur);
     };
     // The first batch's strip edges are loaded before the ring's first rows are
@@ -639,7 +648,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         yT1 = f.f1;
         yT2 = A::add(f.f2, f.corr_hi);
         if constexpr (RUN) {
-            if (r0 == 0) lg.out_y = lfma(neg(f.f0), vmask, lg.out_y);
+            if (r0 + lead == 0) lg.out_y = lfma(neg(f.f0), vmask, lg.out_y);
         }
     }
     big1 = consume(2, R1);  // row r0+1
@@ -665,7 +674,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         acc.outflow += sm.led[4][lane];
         acc.maxinv = nan_max(acc.maxinv, maxinv);
         // Without a mask every in-grid cell of every row received dt*rate.
-        if (!MASKED && d.mult == nullptr) acc.rain_cells += (unsigned)((valid.x ? 1 : 0) + (valid.y ? 1 : 0)) * (unsigned)(r1 - r0);
+        if (!MASKED && d.mult == nullptr) acc.rain_cells += (unsigned)((valid.x ? 1 : 0) + (valid.y ? 1 : 0)) * (unsigned)(r1 - r0 - lead);
     }
     cp_async_wait<0>();  // nothing may land after the warp is done
     return true;
@@ -701,7 +710,7 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
             return MarchPlan{pl.s, pl.snap, pl.dt, pl.go};
         };
         const bool went = r0 < d.upd_hi
-                              ? march_pair<M, true, MASKED, true>(d, p.in, p.out, enter_fn, plan_fn, p.ctl, r0, r1,
+                              ? march_pair<M, true, MASKED, true, false>(d, p.in, p.out, enter_fn, plan_fn, p.ctl, r0, r1,
                                                                   strip * kWarp * 2, s_warp[wib], acc,
                                                                   d.edge[0] ? p.par : -1)
                               : (enter_fn(), cp_async_commit(), plan_fn().go != 0);
@@ -721,7 +730,7 @@ __global__ void __launch_bounds__(THREADS, SWE_PAIR_MINBLOCKS) step_kernel_pair(
         warp_end_step(p.ctl, &p.slots[gw], s_warp[wib].old, p.par, in.pos.steps, gw % kMaxStripes, a);
     } else {
         if (r0 < d.upd_hi)
-            march_pair<M, false, MASKED, true>(d, p.in, p.out, pdl_enter, [&]() { return MarchPlan{p.s, -1, 0.0, 1}; }, nullptr, r0,
+            march_pair<M, false, MASKED, true, false>(d, p.in, p.out, pdl_enter, [&]() { return MarchPlan{p.s, -1, 0.0, 1}; }, nullptr, r0,
                                          r1, strip * kWarp * 2, s_warp[wib], acc);
     }
 }
@@ -747,9 +756,12 @@ struct MemberDev {
     int nstrips, rows_per_warp, ncta;
 };
 
+// LEAD: the marches are a split of kEnsSeam-row ones, whose results they keep (march_pair).
+constexpr int kEnsSeam = 32;
+
 // One item of a batched step: warp `wib` of slot `slot` of member `md`.  A CTA's
 // first item waits for the previous step (pdl_enter) once its static loads are issued.
-template <class M, int THREADS, bool MASKED>
+template <class M, int THREADS, bool MASKED, bool LEAD>
 __device__ __forceinline__ void ensemble_item(const MemberDev& md, int slot, int par, WarpSmem& sm, bool first) {
     constexpr int NW = THREADS / kWarp;
     const int wib = threadIdx.x >> 5;
@@ -769,15 +781,17 @@ __device__ __forceinline__ void ensemble_item(const MemberDev& md, int slot, int
     };
     const int strip = gw % md.nstrips;
     const int chunk = gw / md.nstrips;
-    const int r0 = chunk * md.rows_per_warp;
-    const int r1 = min(r0 + md.rows_per_warp, md.d.rows);
+    const int c0 = chunk * md.rows_per_warp;
+    const int r1 = min(c0 + md.rows_per_warp, md.d.rows);
+    const int lead = LEAD && c0 % kEnsSeam != 0 ? 2 : 0;
+    const int r0 = c0 - lead;
     const StateView in{md.buf[par][0], md.buf[par][1], md.buf[par][2], md.pitch};
     const StateOut out{md.buf[par ^ 1][0], md.buf[par ^ 1][1], md.buf[par ^ 1][2], md.pitch};
     StepAccum acc;
     acc.zero();
-    const bool went = r0 < md.d.rows ? march_pair<M, true, MASKED, false>(md.d, in, out, enter_fn, plan_fn, md.ctl,
+    const bool went = c0 < md.d.rows ? march_pair<M, true, MASKED, false, LEAD>(md.d, in, out, enter_fn, plan_fn, md.ctl,
                                                                    r0, r1, strip * kWarp * 2, sm, acc,
-                                                                   md.d.edge[0] ? par : -1)
+                                                                   md.d.edge[0] ? par : -1, lead)
                                      : (enter_fn(), cp_async_commit(), plan_fn().go != 0);
     if (!went) {
         cp_async_wait<0>();
@@ -815,7 +829,7 @@ ensemble_step_kernel(const MemberDev* __restrict__ members, const int2* __restri
         __syncthreads();  // the previous item is done with s_md
         if (threadIdx.x == 0) s_md = members[item.x];
         __syncthreads();
-        ensemble_item<M, THREADS, MASKED>(s_md, item.y, parity, s_warp[wib], it == (int)blockIdx.x);
+        ensemble_item<M, THREADS, MASKED, false>(s_md, item.y, parity, s_warp[wib], it == (int)blockIdx.x);
     }
 }
 
@@ -834,7 +848,7 @@ struct EnsParams {
 };
 static_assert(sizeof(EnsParams) <= 32764, "the member table must fit the kernel parameters");
 
-template <class M, int THREADS, bool MASKED>
+template <class M, int THREADS, bool MASKED, bool LEAD>
 __global__ void __launch_bounds__(THREADS, SWE_ENS_MINBLOCKS)
 ensemble_step_kernel_p(const __grid_constant__ EnsParams p) {
     constexpr int NW = THREADS / kWarp;
@@ -843,8 +857,7 @@ ensemble_step_kernel_p(const __grid_constant__ EnsParams p) {
     int member = 0;
     for (int it = blockIdx.x; it < p.n_items; it += gridDim.x) {
         while (it >= p.cta_begin[member + 1]) ++member;
-        ensemble_item<M, THREADS, MASKED>(p.m[member], it - p.cta_begin[member], p.parity, s_warp[wib],
-                                          it == (int)blockIdx.x);
+        ensemble_item<M, THREADS, MASKED, LEAD>(p.m[member], it - p.cta_begin[member], p.parity, s_warp[wib], it == (int)blockIdx.x);
     }
 }
 
