@@ -142,7 +142,6 @@ struct swe_domain {
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t seg_ev[6] = {};  // start, recomputed[2], reversed[2], end
     double* corr_sums = nullptr;    // volume sums of the residual correction
-    float* corr_prov = nullptr;     // provisional-depth plane of the correction
     // swe_run_host: device staging of the recorded outputs and the copy stream.
     float* snap_dev = nullptr;
     int64_t snap_cap = 0;  // floats
@@ -302,6 +301,14 @@ dim3 cell_grid(int rows, int cols, int threads, int sms, int per_thread = 1) {
     const int64_t want = std::max<int64_t>(1, ((int64_t)rows * cols + (int64_t)threads * per_thread - 1) /
                                                   ((int64_t)threads * per_thread) / gx);
     const int64_t gy = std::max<int64_t>(1, std::min<int64_t>({(int64_t)rows, want, ((int64_t)sms * 8 + gx - 1) / gx}));
+    return dim3((unsigned)gx, (unsigned)gy);
+}
+
+// Grid of for_pieces.
+dim3 piece_grid(int rows, int cols, int sms) {
+    const int64_t most = (int64_t)sms * 64;
+    const int64_t gx = std::min<int64_t>((cols + kPiece - 1) / kPiece, most);
+    const int64_t gy = std::min<int64_t>({(rows + kPieceWarps - 1) / kPieceWarps, std::max<int64_t>(1, most / gx), 65535});
     return dim3((unsigned)gx, (unsigned)gy);
 }
 
@@ -804,7 +811,6 @@ void free_domain(swe_domain* d) {
         if (e) cudaEventDestroy(e);
     if (d->aux_stream) cudaStreamDestroy(d->aux_stream);
     cudaFree(d->corr_sums);
-    cudaFree(d->corr_prov);
     for (int i = 0; i < 2; ++i) {
         if (d->poll_ev[i]) cudaEventDestroy(d->poll_ev[i]);
         if (d->time_ev[i]) cudaEventDestroy(d->time_ev[i]);
@@ -1912,11 +1918,13 @@ int swe_network_features(swe_domain_t d, const float* h, const float* hu, const 
     }
     a.rain_feature = rain_feature;
     a.dry = d->dd.k.dry;
-    a.layout = layout;
-    a.channels = layout == kFeatRef6 ? 6 : 5;
     a.out = out;
-    a.out_bf16 = out_bf16 ? 1 : 0;
-    features_kernel<<<cell_grid(a.rows, a.cols, 256, d->sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    const dim3 grid = piece_grid(a.rows, a.cols, d->sms);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const auto kernel = layout == kFeatRef6
+                            ? (out_bf16 ? features_kernel<kFeatRef6, __nv_bfloat16> : features_kernel<kFeatRef6, float>)
+                            : (out_bf16 ? features_kernel<kFeatState5, __nv_bfloat16> : features_kernel<kFeatState5, float>);
+    kernel<<<grid, kPieceWarps * kWarp, 0, st>>>(a);
     SWE_CK(cudaGetLastError());
     return SWE_OK;
 }
@@ -1940,7 +1948,7 @@ int swe_output_fields(swe_domain_t d, const float* h, const float* hu, const flo
     a.v = y_velocity;
     a.speed = speed;
     a.out_pitch = out_pitch;
-    schema_kernel<<<cell_grid(a.rows, a.cols, 256, d->sms), 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    schema_kernel<<<piece_grid(a.rows, a.cols, d->sms), kPieceWarps * kWarp, 0, static_cast<cudaStream_t>(stream)>>>(a);
     SWE_CK(cudaGetLastError());
     return SWE_OK;
 }
@@ -1984,15 +1992,12 @@ int swe_apply_correction(swe_domain_t d, const float* h, const float* hu, const 
     if (res_channels != 1 && res_channels != 3) return fail(SWE_ERR_INVALID, "residual must have 1 or 3 channels");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (!d->corr_sums) SWE_CK(cudaMalloc(&d->corr_sums, 2 * sizeof(double)));
-    if (!d->corr_prov) SWE_CK(cudaMalloc(&d->corr_prov, sizeof(float) * (size_t)d->dd.spitch * d->dd.rows));
     SWE_CK(cudaMemsetAsync(d->corr_sums, 0, 2 * sizeof(double), st));
     CorrectionArgs a{};
     a.rows = d->dd.rows;
     a.cols = d->dd.cols;
     a.s = StateView{h, hu, hv, pitch};
     a.out = StateOut{h_out, hu_out, hv_out, out_pitch};
-    a.prov = d->corr_prov;
-    a.prov_pitch = d->dd.spitch;
     a.nm = d->nm;
     a.spitch = d->dd.spitch;
     a.res = residual;
@@ -2009,9 +2014,9 @@ int swe_apply_correction(swe_domain_t d, const float* h, const float* hu, const 
     a.dry = d->dd.k.dry;
     a.eps = 1.1920929e-07f;  // float32 machine epsilon (jnp.finfo(float32).eps)
     a.sums = d->corr_sums;
-    const dim3 grid = cell_grid(a.rows, a.cols, 256, d->sms);
-    correction_sums_kernel<<<grid, 256, 0, st>>>(a);
-    correction_apply_kernel<<<grid, 256, 0, st>>>(a);
+    const dim3 grid = piece_grid(a.rows, a.cols, d->sms);
+    correction_sums_kernel<<<grid, kPieceWarps * kWarp, 0, st>>>(a);
+    correction_apply_kernel<<<grid, kPieceWarps * kWarp, 0, st>>>(a);
     SWE_CK(cudaGetLastError());
     return SWE_OK;
 }

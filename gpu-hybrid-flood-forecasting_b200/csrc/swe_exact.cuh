@@ -79,6 +79,19 @@ __device__ __forceinline__ T quick_div(const O& o, T a, T b, T y) {
     return o.fma(o.fma(o.minus(b), q, a), y, q);
 }
 
+// a / b, rounded once, for any a and b: the quotient above where no operand comes
+// near the ends of the float range (its remainder is then a float) and for a
+// zero numerator, which keeps its sign; the IEEE division otherwise.
+__device__ __forceinline__ float ranged_div(float a, float b) {
+    constexpr float lo = 0x1p-60f, hi = 0x1p60f;
+    const float m = fabsf(a);
+    if (!(b > lo && b < hi && (m == 0.f || (m > lo && m < hi)))) return __fdiv_rn(a, b);
+    float y = rcp_approx(b);
+    y = __fmaf_rn(y, __fmaf_rn(-b, y, 1.f), y);
+    const float q = __fmul_rn(a, y);
+    return m == 0.f ? q : __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+
 // Correctly rounded square root of x >= 0; `xr` is x, or any positive value where x is zero.
 template <class O, class T>
 __device__ __forceinline__ T quick_sqrt(const O& o, T x, T xr) {
