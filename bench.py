@@ -57,7 +57,7 @@ BYTES_PER_CELL = 32  # h, hu, hv, bed, n^2 read (20 B) + h, hu, hv written (12 B
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one fast-arithmetic
 # step_kernel_pair launch on the default 2048x2048 workload, per cell-update, from an
 # ncu capture of that launch: reported as roofline.traffic for that configuration only.
-NCU_TRAFFIC_PER_CELL = (92.77184e6 + 17.041664e6) / 4194304
+NCU_TRAFFIC_PER_CELL = (92.006144e6 + 17.599232e6) / 4194304
 REFERENCE_MAX_STEPS = 200  # whole-grid steps the CPU reference arm times at most
 
 
@@ -541,8 +541,8 @@ def _aux(args, dev):
     state = solver.initial_state(depth_m=street_depth_device(member))
     solver.advance_(state, 20, 0.0)
     ms = timed(lambda: solver.max_inverse_dt(state), 10)
-    entry("reduce_kernel", ms, 16, "run-start CFL maximum and volume: h, hu, hv and n^2 read; "
-                                   "the call returns the value to the host")
+    entry("load_kernel", ms, 16, "CFL maximum of a state: h, hu, hv and n^2 read; "
+                                 "the call returns the value to the host")
     lib = _lib.load()
     mask = torch.ones((n, n), dtype=torch.uint8, device=dev)
     res = torch.empty(1, dtype=torch.float32, device=dev)
@@ -566,9 +566,9 @@ def _aux(args, dev):
     resid = torch.zeros((n, n, 3), dtype=torch.bfloat16, device=dev)
     corr = type(state)(*(torch.empty_like(t) for t in state))
     entry("correction", timed(lambda: apply_residual_correction(solver, state, resid, correction_relaxation=0.5,
-                                                                out=corr), 10), 56,
-          "sums pass: n^2, h and the bf16 residual's sectors read, provisional depth written (18 B); "
-          "apply pass: n^2, h, hu, hv, provisional depth and the residual read, new state written (38 B)")
+                                                                out=corr), 10), 48,
+          "sums pass: n^2, h and the bf16 residual's sectors read (14 B); "
+          "apply pass: n^2, h, hu, hv and the residual read, new state written (34 B)")
     return {"size": [n, n], "peak_gbs": peak, "peak_kind": kind, "kernels": out,
             "timing": "CUDA events around back-to-back calls of the public API (host work between calls included)"}
 

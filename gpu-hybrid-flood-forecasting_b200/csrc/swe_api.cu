@@ -3,8 +3,8 @@
 // Host side: argument validation with the reference's error conventions,
 // packing of the static fields, launch planning, and the run driver.  The run
 // driver keeps the float64 clock, dt, output bookkeeping and mass ledger on
-// the device (swe::Control); the host enqueues step kernels in chunks and only
-// polls a pinned copy of the control block to learn when the run is done.
+// the device (swe::Control); the host enqueues step kernels in chunks, as many as
+// the run is expected to need, and polls its position in pinned memory.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 #include <time.h>

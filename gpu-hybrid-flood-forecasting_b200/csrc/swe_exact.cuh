@@ -7,8 +7,9 @@
 // 2048 x 1024 urban step executed 41.9 warp instructions per cell with 21.5 of
 // 32 lanes active, and waited for instruction fetches and branches in 2.8 of
 // 6.9 cycles between issues.  With the form below the step of the 2048^2 urban
-// grid takes 85 us (325 us before) and that of a masked 517 x 551 grid 16 us (62 us).  QuickExact computes the same values from the
-// published sequences for a machine with fused multiply-add (P. Markstein,
+// grid takes 76 us (304 us before) and that of a masked 517 x 551 grid 12.5 us (62
+// us), of which strip-edge arrays and split marches are part.  QuickExact computes
+// the same values from the published sequences for a machine with fused multiply-add (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
 // IBM J. Res. Dev. 34(1), 1990):
 //

@@ -9,7 +9,7 @@ sequence of fixed-dt steps of
 dt is held fixed (a stop-gradient).  The forward pass keeps one state per
 ``checkpoint_every`` steps.  The backward pass walks the segments in reverse:
 it recomputes a segment's states from its checkpoint and applies the
-hand-written reverse step (``swe_adjoint_step``, two sm_100a kernels) to each
+hand-written reverse step (``swe_adjoint_step``, sm_100a kernels) to each
 of them, injecting the gauge-loss gradient at each observation step.
 """
 

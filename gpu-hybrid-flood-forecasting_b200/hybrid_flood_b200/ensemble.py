@@ -168,8 +168,8 @@ class B200Ensemble:
                     max_steps: int, dt_logs: list | None = None) -> list[tuple]:
         """Advance every member IN PLACE from its start time to ``target_time_s``.
 
-        At most ``max_steps`` CFL-limited steps per member; 50-step graphs are
-        replayed until every member is done.  Returns one
+        At most ``max_steps`` CFL-limited steps per member, queued as the
+        steps the members are expected to need.  Returns one
         ``(final_time_s, steps_used, ledger)`` per member; a member stopped
         short by the cap reports where it stopped.  ``dt_logs``: one device
         float64 tensor of at least ``max_steps`` per member, receiving its dts.

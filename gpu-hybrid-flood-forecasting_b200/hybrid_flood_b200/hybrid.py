@@ -482,7 +482,7 @@ def run_coupled_ensemble(ensemble, initial_states, model, hybrid_inputs: HybridI
 
     All members must share one grid shape (the corrector runs on one
     ``[M, C, rows, cols]`` batch).  Per interval: features of every member
-    into one NHWC batch, one ensemble ``advance_to`` (50-step graphs of the
+    into one NHWC batch, one ensemble ``advance_to`` (queued steps of the
     persistent multi-member kernel), one batched corrector call, and the
     correction of each member.  Returns ``(states, physics_steps_per_member)``
     where ``states[m]`` is that member's ``[T, rows, cols]`` trajectory (or its

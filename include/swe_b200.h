@@ -310,8 +310,8 @@ int swe_ensemble_advance(swe_ensemble_t e, float *const *h, float *const *hu, fl
 
 /* Advance every member IN PLACE from start_s[m] to target_s with CFL-limited
  * steps, at most max_steps each: advance_physics_to_time
- * (hybrid/coupled_forecast.py:123-161) for a batch of members, as 50-step
- * graphs until all members are done.  dt_logs: NULL, or per member a device
+ * (hybrid/coupled_forecast.py:123-161) for a batch of members, queued as the
+ * steps they are expected to need (50-step graphs or single launches).  dt_logs: NULL, or per member a device
  * float64 [max_steps] log of its dts (as swe_advance_to).  SWE_ERR_MAX_STEPS
  * when a member did not reach the target (its result says which).
  * Both advances return with their results final and the members' new states
