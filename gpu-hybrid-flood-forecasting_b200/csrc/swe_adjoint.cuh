@@ -576,10 +576,16 @@ struct AdjRaw {
 
 // Two neighbouring elements of a plane: one 8-byte load where VEC (even column,
 // even pitch, 8-byte aligned plane), else two loads at the clamped columns.
-template <bool VEC>
+// FINISHED: a plane that no kernel writes while this one runs (non-coherent loads;
+// see pdl_enter).
+template <bool VEC, bool FINISHED>
 __device__ __forceinline__ V2 load2(const float* p, uint32_t row, int c0, int c1) {
-    if constexpr (VEC) return {__ldg(reinterpret_cast<const float2*>(p + row + c0))};
-    return {{__ldg(p + row + c0), __ldg(p + row + c1)}};
+    auto get = [](const auto* q) {
+        if constexpr (FINISHED) return __ldg(q);
+        else return state_load(q);
+    };
+    if constexpr (VEC) return {get(reinterpret_cast<const float2*>(p + row + c0))};
+    return {{get(p + row + c0), get(p + row + c1)}};
 }
 
 // 32-bit element offsets: planes hold fewer than 2^31 elements (checked on the host).
@@ -588,25 +594,26 @@ __device__ __forceinline__ uint32_t adj_row(const DomainDev& d, int r) { return 
 template <bool NEXT, bool VEC>
 __device__ __forceinline__ void load_states(const AdjLaunch& p, int r, int c0, int c1, AdjRaw& a) {
     const uint32_t rr = adj_row(p.d, r), so = rr * (uint32_t)p.in.pitch, zo = rr * (uint32_t)p.d.spitch;
-    a.h = load2<VEC>(p.in.h, so, c0, c1);
-    a.hu = load2<VEC>(p.in.hu, so, c0, c1);
-    a.hv = load2<VEC>(p.in.hv, so, c0, c1);
-    a.z = load2<VEC>(p.d.bed, zo, c0, c1);
-    a.nm = load2<VEC>(p.d.nm, zo, c0, c1);
+    a.h = load2<VEC, true>(p.in.h, so, c0, c1);
+    a.hu = load2<VEC, true>(p.in.hu, so, c0, c1);
+    a.hv = load2<VEC, true>(p.in.hv, so, c0, c1);
+    a.z = load2<VEC, true>(p.d.bed, zo, c0, c1);
+    a.nm = load2<VEC, true>(p.d.nm, zo, c0, c1);
     if constexpr (NEXT) {
         const uint32_t no = rr * (uint32_t)p.next.pitch;
-        a.h1 = load2<VEC>(p.next.h, no, c0, c1);
-        a.q1 = load2<VEC>(p.next.hu, no, c0, c1);
-        a.q2 = load2<VEC>(p.next.hv, no, c0, c1);
+        a.h1 = load2<VEC, true>(p.next.h, no, c0, c1);
+        a.q1 = load2<VEC, true>(p.next.hu, no, c0, c1);
+        a.q2 = load2<VEC, true>(p.next.hv, no, c0, c1);
     }
 }
 
+// dL/dU_{k+1}: written by the reverse step before, which may still be running when this kernel starts.
 template <bool VEC>
 __device__ __forceinline__ void load_lam(const AdjLaunch& p, int r, int c0, int c1, AdjRaw& a) {
     const uint32_t lo = adj_row(p.d, r) * (uint32_t)p.lam.pitch;
-    a.l0 = load2<VEC>(p.lam.h, lo, c0, c1);
-    a.l1 = load2<VEC>(p.lam.hu, lo, c0, c1);
-    a.l2 = load2<VEC>(p.lam.hv, lo, c0, c1);
+    a.l0 = load2<VEC, false>(p.lam.h, lo, c0, c1);
+    a.l1 = load2<VEC, false>(p.lam.hu, lo, c0, c1);
+    a.l2 = load2<VEC, false>(p.lam.hv, lo, c0, c1);
 }
 
 template <bool NEXT, bool VEC>

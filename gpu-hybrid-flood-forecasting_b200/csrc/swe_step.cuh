@@ -219,6 +219,10 @@ __device__ __forceinline__ void set_vel(Cell& c, float dry) {
     M::vel2(c.hu, c.hv, c.h, dry, c.u, c.v);
 }
 
+// What the step before writes (states, strip edges, dL/dU) is read with ordinary loads: see pdl_enter.
+template <class T>
+__device__ __forceinline__ T state_load(const T* p) { return *p; }
+
 // Load V cells of row r starting at column c0 (r in [-1, rows], c0 in [-V, cols]),
 // applying the ghost ring: clamp to the nearest interior cell, negate hu on
 // reflective left/right ghosts and hv on reflective bottom/top ghosts.
@@ -231,9 +235,9 @@ __device__ __forceinline__ void load_cells(const DomainDev& d, const StateView& 
     const int64_t zo = (int64_t)rr * d.spitch;
     if (c0 >= 0 && c0 + V <= d.cols) {
         if constexpr (V == 4) {
-            const float4 h = __ldg(reinterpret_cast<const float4*>(s.h + so + c0));
-            const float4 hu = __ldg(reinterpret_cast<const float4*>(s.hu + so + c0));
-            const float4 hv = __ldg(reinterpret_cast<const float4*>(s.hv + so + c0));
+            const float4 h = state_load(reinterpret_cast<const float4*>(s.h + so + c0));
+            const float4 hu = state_load(reinterpret_cast<const float4*>(s.hu + so + c0));
+            const float4 hv = state_load(reinterpret_cast<const float4*>(s.hv + so + c0));
             const float4 z = __ldg(reinterpret_cast<const float4*>(d.bed + zo + c0));
             const float4 nm = __ldg(reinterpret_cast<const float4*>(d.nm + zo + c0));
             out[0] = {h.x, hu.x, hv.x, z.x, nm.x, 0.f, 0.f};
@@ -241,9 +245,9 @@ __device__ __forceinline__ void load_cells(const DomainDev& d, const StateView& 
             out[2] = {h.z, hu.z, hv.z, z.z, nm.z, 0.f, 0.f};
             out[3] = {h.w, hu.w, hv.w, z.w, nm.w, 0.f, 0.f};
         } else if constexpr (V == 2) {
-            const float2 h = __ldg(reinterpret_cast<const float2*>(s.h + so + c0));
-            const float2 hu = __ldg(reinterpret_cast<const float2*>(s.hu + so + c0));
-            const float2 hv = __ldg(reinterpret_cast<const float2*>(s.hv + so + c0));
+            const float2 h = state_load(reinterpret_cast<const float2*>(s.h + so + c0));
+            const float2 hu = state_load(reinterpret_cast<const float2*>(s.hu + so + c0));
+            const float2 hv = state_load(reinterpret_cast<const float2*>(s.hv + so + c0));
             const float2 z = __ldg(reinterpret_cast<const float2*>(d.bed + zo + c0));
             const float2 nm = __ldg(reinterpret_cast<const float2*>(d.nm + zo + c0));
             out[0] = {h.x, hu.x, hv.x, z.x, nm.x, 0.f, 0.f};
@@ -251,9 +255,8 @@ __device__ __forceinline__ void load_cells(const DomainDev& d, const StateView& 
         } else {
 #pragma unroll
             for (int i = 0; i < V; ++i) {
-                out[i] = {__ldg(s.h + so + c0 + i), __ldg(s.hu + so + c0 + i),
-                          __ldg(s.hv + so + c0 + i), __ldg(d.bed + zo + c0 + i),
-                          __ldg(d.nm + zo + c0 + i), 0.f, 0.f};
+                out[i] = {state_load(s.h + so + c0 + i), state_load(s.hu + so + c0 + i), state_load(s.hv + so + c0 + i),
+                          __ldg(d.bed + zo + c0 + i), __ldg(d.nm + zo + c0 + i), 0.f, 0.f};
             }
         }
 #pragma unroll
@@ -264,7 +267,7 @@ __device__ __forceinline__ void load_cells(const DomainDev& d, const StateView& 
         for (int i = 0; i < V; ++i) {
             const int c = c0 + i;
             const int cc = c < 0 ? 0 : (c >= d.cols ? d.cols - 1 : c);
-            Cell x = {__ldg(s.h + so + cc), __ldg(s.hu + so + cc), __ldg(s.hv + so + cc),
+            Cell x = {state_load(s.h + so + cc), state_load(s.hu + so + cc), state_load(s.hv + so + cc),
                       __ldg(d.bed + zo + cc), __ldg(d.nm + zo + cc), 0.f, 0.f};
             if ((c < 0 && d.bnd[0] == 0) || (c >= d.cols && d.bnd[1] == 0)) x.hu = -x.hu;
             if (flip_v) x.hv = -x.hv;
@@ -510,11 +513,16 @@ __device__ __forceinline__ double output_time(const Control* c, int i) {
 }
 
 // Programmatic dependent launch: a step kernel launched with the programmatic
-// stream-serialisation attribute may be scheduled while the previous step is
-// still running.  It lets its own successor launch at once and then waits,
-// before it reads or writes anything, until the previous grid has completed
-// and its memory is visible (a hardware wait, not a spin).  Launched without
-// the attribute both instructions do nothing.
+// stream-serialisation attribute may start while the previous step is still
+// running.  It waits until that grid has completed and its memory is visible (a
+// hardware wait, not a spin), and only then lets its own successor start: a step
+// therefore starts after the one two before it is complete, and at most two
+// overlap.  Ahead of the wait a kernel may read only what neither of its two
+// predecessors writes (bed, n^2, the strip edges' statics, finished states of a
+// rollout).  What the predecessor writes changes within this kernel's lifetime, so
+// it is never read with a non-coherent load (__ldg: read-only for the whole kernel,
+// not ordered by the wait), only with ordinary loads or cp.async after the wait.
+// Launched without the attribute both instructions do nothing.
 __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

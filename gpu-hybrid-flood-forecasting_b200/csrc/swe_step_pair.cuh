@@ -526,8 +526,8 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         Cell L[1], E[1], Q[1];
         if (RUN && ein != nullptr) {
             auto side = [&](int i, int bd, int right) -> Cell {
-                return {__ldg(ein + edge_index(d, bd, 3 * right + 0, rr)), __ldg(ein + edge_index(d, bd, 3 * right + 1, rr)),
-                        __ldg(ein + edge_index(d, bd, 3 * right + 2, rr)), es.z[i], es.nm[i], 0.f, 0.f};
+                return {state_load(ein + edge_index(d, bd, 3 * right + 0, rr)), state_load(ein + edge_index(d, bd, 3 * right + 1, rr)),
+                        state_load(ein + edge_index(d, bd, 3 * right + 2, rr)), es.z[i], es.nm[i], 0.f, 0.f};
             };
             L[0] = side(0, eb, west ? 1 : 0);
             E[0] = side(1, eb, 1);
