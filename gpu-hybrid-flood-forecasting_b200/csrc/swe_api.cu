@@ -551,6 +551,7 @@ int begin_runs(const std::vector<swe_domain*>& doms, const std::vector<RunStart>
 struct RunPlanes {
     float* p[3];
     int64_t pitch;
+    bool unless_failed = false;  // a run that stops with an error status does not write them
 };
 
 template <int ND>
@@ -577,6 +578,7 @@ int end_batch(swe_domain* const* doms, const int* ncta, const RunPlanes* dst, in
         for (int f = 0; f < 3; ++f) q.dst[f] = dst[i].p[f];
         q.dpitch = dst[i].pitch;
         q.ctl = d->ctl;
+        q.unless_failed = dst[i].unless_failed;
     }
     ledger_fold_kernel<256, ND><<<n, 256, 0, st>>>(fb);
     if (dst) store_kernel<kThreads, ND><<<ctas, kThreads, 0, st>>>(sb);
@@ -1796,7 +1798,7 @@ int swe_advance(swe_domain_t d, float* h, float* hu, float* hv, int64_t pitch, i
     if (n_steps < 0) return fail(SWE_ERR_INVALID, "n_steps must be >= 0");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const float times[2] = {(float)start_s, INFINITY};
-    const RunPlanes dst{{h, hu, hv}, pitch};
+    const RunPlanes dst{{h, hu, hv}, pitch, true};
     rc = run_driver(d, RunStart{StateView{h, hu, hv, pitch}, start_s, 2, n_steps, times, 2}, &dst, result, st);
     if (rc) return rc;
     if (result->status == SWE_ERR_NONFINITE)

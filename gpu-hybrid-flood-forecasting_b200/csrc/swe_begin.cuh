@@ -352,6 +352,7 @@ struct StoreDomain {
     float* dst[3];
     int64_t dpitch;
     const Control* ctl;
+    int unless_failed;  // 1: a run that stopped with an error status leaves dst as it was
 };
 
 template <int ND>
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(THREADS) store_kernel(const __grid_constant__ 
     int m = 0;
     while (m + 1 < b.n && (int)blockIdx.x >= b.d[m + 1].cta0) ++m;
     const StoreDomain& q = b.d[m];
+    if (q.unless_failed && q.ctl->status) return;
     const int cta = (int)blockIdx.x - q.cta0, bx = cta % q.gx, by = cta / q.gx;
     const int par = q.ctl->steps & 1;
     const float* h = q.src[par][0];

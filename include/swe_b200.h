@@ -134,7 +134,8 @@ int swe_run_host(swe_domain_t d, const float *h0, const float *hu0, const float 
                  float *out_hv, swe_run_result *result, void *stream);
 
 /* Advance (h, hu, hv) in place by exactly n_steps CFL-limited steps starting at
- * time start_s; the state, final time and ledger are returned in `result`. */
+ * time start_s; the final time and ledger are returned in `result`.  A run that
+ * fails (SWE_ERR_NONFINITE) leaves (h, hu, hv) as they were. */
 int swe_advance(swe_domain_t d, float *h, float *hu, float *hv, int64_t pitch, int32_t n_steps,
                 double start_s, swe_run_result *result, void *stream);
 
