@@ -855,7 +855,8 @@ struct swe_ensemble {
     int arith = SWE_ARITH_FAST;
     bool masked = false;
     int rows_per_warp = 128;  // provisional: swe_ensemble_create sets ens_auto_rows (B200Ensemble.autotune measures)
-    bool tuned = false;       // rows_per_warp was set by the caller (or SWE_ENSEMBLE_ROWS)
+    int auto_rows = 0;        // the default of rows_per_warp
+    bool tuned = false;       // rows_per_warp is the caller's (or SWE_ENSEMBLE_ROWS), not the default
     bool lead = false;        // the marches are a split of rows_per_warp that keeps its bits
     int sms = 148;
     MemberDev* members_dev = nullptr;
@@ -975,6 +976,9 @@ int ens_auto_rows(const swe_ensemble* e) {
 // dropped rows, and the results keep every bit (march_pair).  us a step, fast, at
 // 32 rows and split: 4 x 512^2 28.1 and 18.6, 2 x 200^2 28.6 and 7.5; a batch that
 // fills most of the grid gains little (eight of 280^2 to 640^2: 32.0 and 29.2).
+// Setting the default's own value keeps (or restores) the default's plan, so that a
+// caller who sets what swe_ensemble_rows_per_warp returned, or a tuner that tries it,
+// does not lose the split.
 int ens_march_rows(const swe_ensemble* e) {
     if (e->tuned || e->rows_per_warp != kEnsMinRows || !ens_param_table(e)) return e->rows_per_warp;
     const int one_wave = ens_fit_rows(e, (int64_t)ens_occupancy(e) * e->sms, 1, kEnsMinRows);
@@ -2221,7 +2225,7 @@ int swe_ensemble_create(const swe_domain_desc* descs, int32_t n_members, swe_ens
     }
     int rc = ens_rebuild(e);
     if (!rc && !std::getenv("SWE_ENSEMBLE_ROWS")) {
-        const int R = ens_auto_rows(e);
+        const int R = e->auto_rows = ens_auto_rows(e);
         if (R != e->rows_per_warp) {
             e->rows_per_warp = R;
             rc = ens_rebuild(e);
@@ -2250,7 +2254,7 @@ int swe_ensemble_set_rows_per_warp(swe_ensemble_t e, int32_t rows_per_warp) {
     if (!e || rows_per_warp < 1) return fail(SWE_ERR_INVALID, "rows_per_warp must be >= 1");
     cudaDeviceSynchronize();
     e->rows_per_warp = rows_per_warp;
-    e->tuned = true;
+    e->tuned = rows_per_warp != e->auto_rows;
     return ens_rebuild(e);
 }
 

@@ -206,6 +206,8 @@ class B200Ensemble:
                     raise ValueError("ensemble states must be device float32 [rows, cols] tensors per member")
 
     def set_rows_per_warp(self, rows: int) -> None:
+        """Rows each warp marches per work item.  The value the ensemble started with stands for its
+        default plan, which splits the marches of a small batch further."""
         with torch.cuda.device(self.device):
             _lib.check(self._lib.swe_ensemble_set_rows_per_warp(self._handle, int(rows)), "set_rows_per_warp")
         self.rows_per_warp = int(rows)
@@ -224,7 +226,9 @@ class B200Ensemble:
         return int(self._lib.swe_ensemble_last_launch_count(self._handle))
 
     def shape_key(self) -> str:
-        text = json.dumps({"shapes": sorted(self.shapes), "arith": self.arithmetic,
+        # "plan" numbers what a rows value stands for: 2, the default's value is the default plan with
+        # its split.  Winners timed under another meaning are not reused.
+        text = json.dumps({"shapes": sorted(self.shapes), "arith": self.arithmetic, "plan": 2,
                            "device": torch.cuda.get_device_name(self.device)})
         return hashlib.sha1(text.encode()).hexdigest()[:16]
 
@@ -232,6 +236,7 @@ class B200Ensemble:
                  cache: pathlib.Path | None = DEFAULT_CACHE) -> int:
         """Pick the rows-per-warp of the work list by timing ``steps`` steps per candidate.
 
+        A candidate equal to the ensemble's default (32 for a small batch) is the default plan.
         The members' states are advanced by the tuning steps (pass copies to
         keep them).  The winner is cached in ``cache`` (JSON) per member-shape
         set and device, and reused without timing on later calls.

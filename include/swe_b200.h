@@ -297,8 +297,10 @@ int swe_ensemble_size(swe_ensemble_t e);
  * The default, chosen at creation, is the smallest march of at least 32 rows
  * whose work items fit the persistent grid in one round (256 when none does);
  * SWE_ENSEMBLE_ROWS overrides it.  A batch that leaves part of the grid idle at
- * the default of 32 rows is split further; rows set by the caller are kept.  swe_ensemble_rows_per_warp returns the
- * current value (-1 for a null handle). */
+ * the default of 32 rows is split further, with the same results; other rows set by
+ * the caller are marched as they are, and setting the default's value again restores
+ * the default with its split.  swe_ensemble_rows_per_warp returns the value in
+ * effect, before any split (-1 for a null handle). */
 int swe_ensemble_set_rows_per_warp(swe_ensemble_t e, int32_t rows_per_warp);
 int32_t swe_ensemble_rows_per_warp(swe_ensemble_t e);
 
