@@ -219,24 +219,31 @@ struct StepK {
 
 template <class M, bool RUN, bool MASKED, class F>
 void dispatch_v(int V, F&& f) {
-    if (V == 2) f(StepK<2, M, RUN, MASKED>{}); else f(StepK<1, M, RUN, MASKED>{});
+    using M1 = std::conditional_t<M::kExact, ExactMath, M>;  // the scalar kernel has IEEE operations only
+    if (V == 2) f(StepK<2, M, RUN, MASKED>{}); else f(StepK<1, M1, RUN, MASKED>{});
 }
 
+// f(policy) with the arithmetic of a march: IeeeMath where the exact one's branch-free
+// form does not cover the controls of the domain, or of some member of a batch.
 template <class F>
-void dispatch(int V, int arith, bool run, bool masked, F&& f) {
-    if (arith == SWE_ARITH_FAST) {
+void with_math(int arith, bool quick, F&& f) {
+    if (arith == SWE_ARITH_FAST) f(FastMath{});
+    else if (quick) f(ExactMath{});
+    else f(IeeeMath{});
+}
+
+bool quick_form(const swe_domain* d) { return (d->dd.k.forms & kFormQuick) != 0; }
+
+template <class F>
+void dispatch(const swe_domain* d, int V, bool run, F&& f) {
+    with_math(d->arith, quick_form(d), [&](auto m) {
+        using M = decltype(m);
         if (run) {
-            if (masked) dispatch_v<FastMath, true, true>(V, f); else dispatch_v<FastMath, true, false>(V, f);
+            if (d->masked) dispatch_v<M, true, true>(V, f); else dispatch_v<M, true, false>(V, f);
         } else {
-            if (masked) dispatch_v<FastMath, false, true>(V, f); else dispatch_v<FastMath, false, false>(V, f);
+            if (d->masked) dispatch_v<M, false, true>(V, f); else dispatch_v<M, false, false>(V, f);
         }
-    } else {
-        if (run) {
-            if (masked) dispatch_v<ExactMath, true, true>(V, f); else dispatch_v<ExactMath, true, false>(V, f);
-        } else {
-            if (masked) dispatch_v<ExactMath, false, true>(V, f); else dispatch_v<ExactMath, false, false>(V, f);
-        }
-    }
+    });
 }
 
 // Rows per warp of a grid that does not fill the GPU: a step then lasts as long
@@ -269,7 +276,7 @@ Plan make_plan(const swe_domain* d, int V, bool run) {
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, decltype(k)::fn(), kThreads, 0) == cudaSuccess && n > 0)
                 occ = n;
         };
-        dispatch(V, d->arith, run, d->masked, occ_of);
+        dispatch(d, V, run, occ_of);
     }
     const int wpb = kThreads / kWarp;
     const int64_t warps_avail = (int64_t)occ * d->sms * wpb;
@@ -290,7 +297,7 @@ Plan make_plan(const swe_domain* d, int V, bool run) {
 
 void launch_step(const swe_domain* d, const Plan& pl, const StepLaunch& sl, bool run,
                  cudaStream_t st, bool pdl = false) {
-    dispatch(pl.V, d->arith, run, d->masked, [&](auto k) { decltype(k)::launch(pl.blocks, sl, st, pdl); });
+    dispatch(d, pl.V, run, [&](auto k) { decltype(k)::launch(pl.blocks, sl, st, pdl); });
 }
 
 // 2-D grid of a per-cell kernel over rows x cols (for_cells): x over the
@@ -854,6 +861,7 @@ struct swe_ensemble {
     std::vector<swe_domain*> doms;
     int arith = SWE_ARITH_FAST;
     bool masked = false;
+    bool quick = true;        // every member's controls allow the branch-free exact arithmetic
     int rows_per_warp = 128;  // provisional: swe_ensemble_create sets ens_auto_rows (B200Ensemble.autotune measures)
     int auto_rows = 0;        // the default of rows_per_warp
     bool tuned = false;       // rows_per_warp is the caller's (or SWE_ENSEMBLE_ROWS), not the default
@@ -904,28 +912,24 @@ void ens_launch_t(const swe_ensemble* e, int parity, cudaStream_t st, bool pdl) 
 }
 
 void ens_launch(const swe_ensemble* e, int parity, cudaStream_t st, bool pdl = false) {
-    if (e->arith == SWE_ARITH_FAST) {
-        if (e->masked) ens_launch_t<FastMath, true>(e, parity, st, pdl); else ens_launch_t<FastMath, false>(e, parity, st, pdl);
-    } else {
-        if (e->masked) ens_launch_t<ExactMath, true>(e, parity, st, pdl); else ens_launch_t<ExactMath, false>(e, parity, st, pdl);
-    }
+    with_math(e->arith, e->quick, [&](auto m) {
+        using M = decltype(m);
+        if (e->masked) ens_launch_t<M, true>(e, parity, st, pdl); else ens_launch_t<M, false>(e, parity, st, pdl);
+    });
+}
+
+template <class M, bool MASKED>
+const void* ens_kernel(const swe_ensemble* e) {
+    if (e->params) return reinterpret_cast<const void*>(&ensemble_step_kernel_p<M, kThreads, MASKED, false>);
+    return reinterpret_cast<const void*>(&ensemble_step_kernel<M, kThreads, MASKED>);
 }
 
 int ens_occupancy(const swe_ensemble* e) {
     const void* fn = nullptr;
-    if (e->params) {
-        if (e->arith == SWE_ARITH_FAST)
-            fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel_p<FastMath, kThreads, true, false>)
-                           : reinterpret_cast<const void*>(&ensemble_step_kernel_p<FastMath, kThreads, false, false>);
-        else
-            fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel_p<ExactMath, kThreads, true, false>)
-                           : reinterpret_cast<const void*>(&ensemble_step_kernel_p<ExactMath, kThreads, false, false>);
-    } else if (e->arith == SWE_ARITH_FAST)
-        fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel<FastMath, kThreads, true>)
-                       : reinterpret_cast<const void*>(&ensemble_step_kernel<FastMath, kThreads, false>);
-    else
-        fn = e->masked ? reinterpret_cast<const void*>(&ensemble_step_kernel<ExactMath, kThreads, true>)
-                       : reinterpret_cast<const void*>(&ensemble_step_kernel<ExactMath, kThreads, false>);
+    with_math(e->arith, e->quick, [&](auto m) {
+        using M = decltype(m);
+        fn = e->masked ? ens_kernel<M, true>(e) : ens_kernel<M, false>(e);
+    });
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, 0) != cudaSuccess || n < 1) n = 1;
     return n;
@@ -2221,6 +2225,7 @@ int swe_ensemble_create(const swe_domain_desc* descs, int32_t n_members, swe_ens
         }
         e->doms.push_back(d);
         e->masked = e->masked || d->masked;
+        e->quick = e->quick && quick_form(d);
         e->sms = d->sms;
     }
     int rc = ens_rebuild(e);

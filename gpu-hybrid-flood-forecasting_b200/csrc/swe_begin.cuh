@@ -110,6 +110,7 @@ __device__ __noinline__ inline float ieee_inverse_dt(float h, float hu, float hv
 template <class M>
 __device__ __forceinline__ float inverse_dt(const Consts& k, float rdx, float rdy, float h, float hu, float hv) {
     if constexpr (M::kExact) {
+        if (!(k.forms & kFormQuick)) return ieee_inverse_dt(h, hu, hv, k.g, k.dry, k.dx, k.dy);
         // The branch-free form, and the IEEE operations for a cell outside its range.
         // (A velocity too small for it does not reach the sum: the celerity of a wet cell is above 1e-5.)
         const SoloOps o;
@@ -118,7 +119,7 @@ __device__ __forceinline__ float inverse_dt(const Consts& k, float rdx, float rd
         const float u = wet ? quick_div(o, hu, h, rh) : 0.f, v = wet ? quick_div(o, hv, h, rh) : 0.f;
         const float w = o.mul(quick_celerity_up(o, fmaxf(h, 0.f), k.g * 1.8446744073709552e19f), kDown);
         const float inv = o.add(quick_div(o, o.add(fabsf(u), w), k.dx, rdx), quick_div(o, o.add(fabsf(v), w), k.dy, rdy));
-        if ((k.forms & kFormQuick) && max3_nan(h, fabsf(u), fabsf(v)) < kQuickLimit) return inv;
+        if (max3_nan(h, fabsf(u), fabsf(v)) < kQuickLimit) return inv;
         return ieee_inverse_dt(h, hu, hv, k.g, k.dry, k.dx, k.dy);
     } else {
         float u, v;

@@ -122,6 +122,10 @@ struct ExactMath {
     __device__ static __forceinline__ float pow73(float x, float expo) { return pow73_exact(x, expo); }
 };
 
+// ExactMath with the IEEE operations throughout: the paired march of domains whose
+// controls lie outside the range of the branch-free form (swe_exact.cuh).
+struct IeeeMath : ExactMath {};
+
 struct FastMath {
     static constexpr bool kExact = false;
     __device__ static __forceinline__ float add(float a, float b) { return a + b; }

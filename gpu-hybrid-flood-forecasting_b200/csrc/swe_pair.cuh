@@ -71,16 +71,18 @@ __device__ __forceinline__ auto all_true<float2>() { return B2{true, true}; }
 template <class M>
 struct P;
 
-// The operations of P<ExactMath> with a slow path of their own are calls: the
-// march runs them only for rows outside the range of swe_exact.cuh, and inlined
-// they were most of its instructions.
+// The operations with a slow path of their own are calls in P<ExactMath>: its march
+// runs them only for rows outside the range of swe_exact.cuh, and inlined they were
+// most of its instructions.  P<IeeeMath>, whose march runs nothing else, has them
+// inline (2048^2, dry tolerance 0: 332 us a step; 464 with calls, 518 with the
+// branch-free form evaluated first).
 __device__ __noinline__ inline float ieee_div(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __noinline__ inline float ieee_sqrt(float a) { return __fsqrt_rn(a); }
 __device__ __noinline__ inline float ieee_hypot(float a, float b) { return ExactMath::hypot(a, b); }
 __device__ __noinline__ inline float ieee_pow73(float x, float e) { return pow73_exact(x, e); }
 
-template <>
-struct P<ExactMath> {
+template <bool CALLS>
+struct PExact {
     static constexpr bool kExact = true;
     __device__ static __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
     __device__ static __forceinline__ float2 add(float2 a, float2 b) {
@@ -94,19 +96,22 @@ struct P<ExactMath> {
     __device__ static __forceinline__ float2 mul(float2 a, float2 b) {
         return {__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)};
     }
-    __device__ static __forceinline__ float div(float a, float b) { return ieee_div(a, b); }
-    __device__ static __forceinline__ float2 div(float2 a, float2 b) {
-        return {ieee_div(a.x, b.x), ieee_div(a.y, b.y)};
+    __device__ static __forceinline__ float div(float a, float b) { return CALLS ? ieee_div(a, b) : __fdiv_rn(a, b); }
+    __device__ static __forceinline__ float2 div(float2 a, float2 b) { return {div(a.x, b.x), div(a.y, b.y)}; }
+    __device__ static __forceinline__ float sqrt(float a) { return CALLS ? ieee_sqrt(a) : __fsqrt_rn(a); }
+    __device__ static __forceinline__ float2 sqrt(float2 a) { return {sqrt(a.x), sqrt(a.y)}; }
+    __device__ static __forceinline__ float hypot(float a, float b) {
+        return CALLS ? ieee_hypot(a, b) : ExactMath::hypot(a, b);
     }
-    __device__ static __forceinline__ float sqrt(float a) { return ieee_sqrt(a); }
-    __device__ static __forceinline__ float2 sqrt(float2 a) { return {ieee_sqrt(a.x), ieee_sqrt(a.y)}; }
-    __device__ static __forceinline__ float hypot(float a, float b) { return ieee_hypot(a, b); }
-    __device__ static __forceinline__ float2 hypot(float2 a, float2 b) {
-        return {ieee_hypot(a.x, b.x), ieee_hypot(a.y, b.y)};
-    }
-    __device__ static __forceinline__ float pow73(float x, float e) { return ieee_pow73(x, e); }
-    __device__ static __forceinline__ float2 pow73(float2 x, float e) { return {ieee_pow73(x.x, e), ieee_pow73(x.y, e)}; }
+    __device__ static __forceinline__ float2 hypot(float2 a, float2 b) { return {hypot(a.x, b.x), hypot(a.y, b.y)}; }
+    __device__ static __forceinline__ float pow73(float x, float e) { return CALLS ? ieee_pow73(x, e) : pow73_exact(x, e); }
+    __device__ static __forceinline__ float2 pow73(float2 x, float e) { return {pow73(x.x, e), pow73(x.y, e)}; }
 };
+
+template <>
+struct P<ExactMath> : PExact<true> {};
+template <>
+struct P<IeeeMath> : PExact<false> {};
 
 template <>
 struct P<FastMath> {

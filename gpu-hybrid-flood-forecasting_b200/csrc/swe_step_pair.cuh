@@ -133,13 +133,14 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
     // same correctly rounded result (a warp-uniform branch).
     const bool pow2 = (k.forms & kFormPow2) != 0;
     const float2 rdxe = splat(__frcp_rn(k.dx)), rdye = splat(__frcp_rn(k.dy));
-    // Exact arithmetic: the operations of the branch-free form, and whether the
-    // domain's controls and the step's dt allow it at all.
+    // Exact arithmetic in a domain whose controls allow the branch-free form (kFormQuick;
+    // the others run IeeeMath): its operations, and whether the step's dt and the strip's
+    // edges allow it too.
+    constexpr bool kBranchFree = std::is_same_v<M, ExactMath>;
+    using Quick = std::conditional_t<kBranchFree, QuickExact, M>;
     const PairOps po{splat(k.one), splat(-k.one)};
     const SoloOps so1;
-    using Quick = std::conditional_t<A::kExact, QuickExact, M>;
-    const bool ieee_domain = A::kExact && (k.forms & kFormQuick) == 0;
-    bool ieee_step = ieee_domain, ieee_batch = false;  // rows that take the IEEE operations (warp-uniform)
+    bool ieee_step = false, ieee_batch = false;  // rows that take the IEEE operations (warp-uniform)
     auto over_dx = [&](float2 a) {
         if constexpr (A::kExact) return pow2 ? A::mul(a, rdxe) : A::div(a, dx2);
         else return A::mul(a, rdxe);  // not used by the fast policy
@@ -219,7 +220,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         c.z = fv[3];
         c.nm = fv[4];
         float big = 0.f;
-        if constexpr (A::kExact) {
+        if constexpr (kBranchFree) {
             quick_vel(po, c, kp);
             big = max3_nan(max3_nan(c.h.x, fabsf(c.u.x), fabsf(c.v.x)), c.h.y, max3_nan(fabsf(c.u.y), fabsf(c.v.y), 0.f));
         } else {
@@ -543,7 +544,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         CellT<float> e{E[0].h, E[0].hu, E[0].hv, E[0].z, E[0].nm, 0.f, 0.f};
         CellT<float> q{Q[0].h, Q[0].hu, Q[0].hv, Q[0].z, Q[0].nm, 0.f, 0.f};
         FaceT<float> f;
-        if constexpr (A::kExact) {
+        if constexpr (kBranchFree) {
             quick_vel(so1, l, ks);
             quick_vel(so1, e, ks);
             quick_vel(so1, q, ks);
@@ -551,9 +552,9 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             const float big = max3_nan(max3_nan(l.h, fabsf(l.u), fabsf(l.v)), max3_nan(e.h, fabsf(e.u), fabsf(e.v)),
                                        max3_nan(q.h, fabsf(q.u), fabsf(q.v)));
             // Rows whose edge cells leave the range take the IEEE operations, here and in the rows.
-            ieee_batch = ieee_domain || __any_sync(0xffffffffu, !(big < kQuickLimit));
+            ieee_batch = __any_sync(0xffffffffu, !(big < kQuickLimit));
         }
-        if (!A::kExact || ieee_batch) {
+        if (!kBranchFree || ieee_batch) {
             set_vel_t<M>(l, ks);
             set_vel_t<M>(e, ks);
             set_vel_t<M>(q, ks);
@@ -585,7 +586,7 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             w = update(policy, r, c, yT0, yT1, yT2, fy.f0, fy.f1, t2, x);
         };
         evaluate(Quick{}, cur, nxt);
-        if constexpr (A::kExact) {
+        if constexpr (kBranchFree) {
             const float big = max3_nan(big_cur, big_nxt, w.big);
             if (__any_sync(0xffffffffu, !(big < kQuickLimit)) || ieee_step || ieee_batch) {
                 CellT<float2> c = cur, n = nxt;
@@ -627,16 +628,16 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
         ndtdy2 = splat(-mp.s.dt * rdy);
         snap = mp.snap;
         dtd = mp.dtd;
-        if constexpr (A::kExact) {
+        if constexpr (kBranchFree) {
             const float adt = fabsf(mp.s.dt);
-            ieee_step = ieee_domain || !(adt < kUp) || (adt != 0.f && adt < kDown);
+            ieee_step = !(adt < kUp) || (adt != 0.f && adt < kDown);
         }
     }
     big1 = consume(0, R1);  // row r0-1
     big0 = consume(1, R0);  // row r0
     {
         FaceT<float2> f = face(Quick{}, kY, R1, R0);
-        if constexpr (A::kExact) {
+        if constexpr (kBranchFree) {
             if (ieee_step || __any_sync(0xffffffffu, !(max3_nan(big0, big1, 0.f) < kQuickLimit))) {
                 CellT<float2> c = R1, n = R0;
                 set_vel_t<M>(c, kp);
