@@ -24,11 +24,13 @@
 // adversarial pairs equal __fdiv_rn).  Small operands are kept
 // clear of that by scaling: numerators and wave speeds carry a factor
 // kUp = 2^32 (a power of two changes no rounding), so a result can differ only
-// where the IEEE one is subnormal, or in the sign of a zero.  Large, infinite and
-// NaN operands are caught per row: the march keeps the largest depth and
-// speed of the cells of a row and, when it is not below kQuickLimit on every
-// lane of the warp (a NaN is not), computes the row again with the IEEE
-// operations (one warp-uniform branch per row of 64 cells).
+// where the IEEE one is vanishing (a friction divisor above 2^94 makes a momentum
+// zero: below 2^-60 in a step that the CFL rule allows; elsewhere below 2^-94), or in
+// the sign of a zero.  Large, infinite and NaN operands are caught per row: the march keeps the largest depth
+// and speed of the cells of a row; where it is not below kQuickLimit on every lane of
+// the warp (a NaN is not) the row takes the IEEE operations, and where only its new
+// values leave the range it is computed again with them (two warp-uniform votes per
+// row of 64 cells).
 //
 // Both cells of a lane share each instruction (f32x2).  A packed multiply whose
 // result is only added would be contracted with the addition by the assembler,
@@ -42,9 +44,14 @@ namespace swe {
 
 constexpr float kUp = 4294967296.0f;            // 2^32
 constexpr float kDown = 2.3283064365386963e-10f;  // 2^-32
-// Depths (m) and speeds (m/s) above which a row is computed with the IEEE
-// operations.  With them below it no term of a face or an update leaves the float range.
-constexpr float kQuickLimit = 1024.0f;
+// Depths (m) and speeds (m/s) from which on a row is computed with the IEEE operations:
+// beyond any water on Earth, and with them below it (and gravity up to 2^6, cells from
+// 2^-10) no term leaves the float range.  The largest are the HLL numerators, 2^32 x
+// speed x momentum flux < 2^49 2^50, and an update's scaled divergence, 2^32 2^52 2^10;
+// a momentum that friction multiplies out of the range gives a NaN, which the row's
+// largest value shows.  (At 1024, a grid 2000 m deep took the IEEE operations
+// everywhere: 2048^2 302 us a step instead of 79.)
+constexpr float kQuickLimit = 65536.0f;
 
 // The exact policy's branch-free form (a tag: the operations are PairOps).
 struct QuickExact {};

@@ -585,15 +585,23 @@ __device__ __forceinline__ bool march_pair(const DomainDev& d, const StateView& 
             t2 = plus(policy, fy.f2, fy.corr_lo);
             w = update(policy, r, c, yT0, yT1, yT2, fy.f0, fy.f1, t2, x);
         };
-        evaluate(Quick{}, cur, nxt);
         if constexpr (kBranchFree) {
-            const float big = max3_nan(big_cur, big_nxt, w.big);
-            if (__any_sync(0xffffffffu, !(big < kQuickLimit)) || ieee_step || ieee_batch) {
+            // A row whose cells are known to lie outside the range takes the IEEE operations
+            // at once; one whose new values leave it is computed again with them.
+            const float big = max3_nan(big_cur, big_nxt, 0.f);
+            bool ieee = ieee_step || ieee_batch || __any_sync(0xffffffffu, !(big < kQuickLimit));
+            if (!ieee) {
+                evaluate(QuickExact{}, cur, nxt);
+                ieee = __any_sync(0xffffffffu, !(w.big < kQuickLimit));
+            }
+            if (ieee) {
                 CellT<float2> c = cur, n = nxt;
                 set_vel_t<M>(c, kp);
                 set_vel_t<M>(n, kp);
                 evaluate(M{}, c, n);
             }
+        } else {
+            evaluate(M{}, cur, nxt);
         }
         if (lead == 0 || r >= r0 + lead) account(cur, w, x);
         if constexpr (RUN) {

@@ -100,3 +100,50 @@ def test_domain_outside_the_range_evaluates_its_rows_once(cuda_device):
     with both evaluated, and the IEEE operations as calls, it took 2.7 times (63 us)."""
     m, st = _member(1024, 1024, 3)
     assert _step_us({**m, "dry_tolerance_m": 0.0}, st) < 2.1 * _step_us(m, st)
+
+
+@pytest.mark.parametrize("masked", [False, True])
+def test_deep_water_stays_in_the_range(cuda_device, masked):
+    """A grid 2000 m deep takes the branch-free form: the same time as a shallow one (three times before)."""
+    m, st = _member(1024, 1024, 5, masked)
+    deep = [np.where(m["domain_mask"], st[0] + np.float32(2000), 0).astype(np.float32), *st[1:]]
+    assert _step_us(m, deep) < 1.5 * _step_us(m, st)
+
+
+@pytest.mark.parametrize("depth,speed", [(4000.0, 30.0), (9.0e4, 1.0), (1.0, 9.0e4), (3.0e4, 3.0e4), (1.0e6, 1.0e6)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_rows_below_and_above_the_limit(cuda_device, monkeypatch, depth, speed, masked):
+    """Runs and steps whose rows lie on both sides of 65536 m or m/s, and cross it."""
+    m, st = _member(70, 200, 9, masked)
+    big, big_st = _member(70, 200, 11, masked, depth=depth, speed=speed)
+    big["domain_mask"] = m["domain_mask"]
+    pick = (np.arange(70) // 9 % 3 == 1)[:, None] & m["domain_mask"]
+    st = [np.where(pick, b, a).astype(np.float32) for a, b in zip(st, big_st)]
+    s, a = _solver(m), _dev(st)
+    ra = s.advance_(a, 25)
+    dt = 0.1 / (depth + speed)
+    one = s.step(_dev(st), dt, 3.0)
+    monkeypatch.setenv("SWE_RUN_VEC", "1")
+    b = _dev(st)
+    assert _solver(m).advance_(b, 25)[:2] == ra[:2]
+    for x, y in zip(a, b):
+        assert torch.equal(x, y)
+    wide = [torch.zeros((70, 201), device="cuda") for _ in range(3)]
+    for w, v in zip(wide, st):
+        w[:, :200] = torch.from_numpy(v)
+    for x, y in zip(one, s.step([w[:, :200] for w in wide], dt, 3.0)):
+        assert torch.equal(x, y)
+
+
+def test_large_depths_and_speeds_equal_numpy(cuda_device):
+    """Without friction every operation of the step is one IEEE operation of the reference."""
+    from oracle import swe_numpy as O
+
+    for depth, speed in ((3.0e4, 50.0), (50.0, 3.0e4), (6.0e4, 6.0e4), (2.0e5, 1.0e5)):
+        m, st = _member(40, 150, 13, depth=depth, speed=speed, manning_n=np.zeros((40, 150), np.float32))
+        got = _solver(m).step(_dev(st), 0.01, 33.0)
+        kw = {k: v for k, v in m.items() if k not in ("bed", "manning_n", "domain_mask")}
+        want = O.finite_volume_step(O.State(*st), O.make_params(m["bed"], m["manning_n"], m["domain_mask"], **kw), 0.01,
+                                    33.0)
+        for g, w in zip(got, want):
+            assert np.array_equal(g.cpu().numpy(), w)
