@@ -300,17 +300,6 @@ void launch_step(const swe_domain* d, const Plan& pl, const StepLaunch& sl, bool
     dispatch(d, pl.V, run, [&](auto k) { decltype(k)::launch(pl.blocks, sl, st, pdl); });
 }
 
-// 2-D grid of a per-cell kernel over rows x cols (for_cells): x over the
-// columns, y over the rows, about 8 CTAs per SM (and about `per_thread` cells
-// per thread on small planes).
-dim3 cell_grid(int rows, int cols, int threads, int sms, int per_thread = 1) {
-    const int64_t gx = std::max<int64_t>(1, std::min<int64_t>((cols + threads - 1) / threads, (int64_t)sms * 8));
-    const int64_t want = std::max<int64_t>(1, ((int64_t)rows * cols + (int64_t)threads * per_thread - 1) /
-                                                  ((int64_t)threads * per_thread) / gx);
-    const int64_t gy = std::max<int64_t>(1, std::min<int64_t>({(int64_t)rows, want, ((int64_t)sms * 8 + gx - 1) / gx}));
-    return dim3((unsigned)gx, (unsigned)gy);
-}
-
 // Grid of for_pieces.
 dim3 piece_grid(int rows, int cols, int sms) {
     const int64_t most = (int64_t)sms * 64;
@@ -319,8 +308,15 @@ dim3 piece_grid(int rows, int cols, int sms) {
     return dim3((unsigned)gx, (unsigned)gy);
 }
 
-// CTAs of a load or store of a domain's rows on `sms` SMs' share of the GPU.
-dim3 load_grid(const swe_domain* d, int sms) { return cell_grid(d->dd.rows, d->dd.cols, kThreads, sms); }
+// CTAs of a load or store of a domain's rows on `sms` SMs' share of the GPU: x over the
+// columns, y over the rows, a cell a thread up to about 8 CTAs per SM.
+dim3 load_grid(const swe_domain* d, int sms) {
+    const int64_t rows = d->dd.rows, cols = d->dd.cols, most = (int64_t)sms * 8;
+    const int64_t gx = std::min((cols + kThreads - 1) / kThreads, most);
+    const int64_t want = (rows * cols + kThreads - 1) / kThreads / gx;
+    const int64_t gy = std::max<int64_t>(1, std::min({rows, want, (most + gx - 1) / gx}));
+    return dim3((unsigned)gx, (unsigned)gy);
+}
 
 int reduce_blocks(const swe_domain* d) {
     const dim3 g = load_grid(d, d->sms);

@@ -1008,14 +1008,4 @@ __global__ void __launch_bounds__(THREADS, MinBlocks<V>::value) step_kernel(cons
     }
 }
 
-// Cells [r0, r1) x [0, cols) of a plane under a 2-D grid-stride launch (grid.x
-// over columns, grid.y over rows, see cell_grid on the host): body(r, c) for
-// each, with no division per cell.
-template <class F>
-__device__ __forceinline__ void for_cells(int r0, int r1, int cols, F&& body) {
-    for (int r = r0 + (int)blockIdx.y; r < r1; r += (int)gridDim.y)
-        for (int c = (int)(blockIdx.x * blockDim.x + threadIdx.x); c < cols; c += (int)(gridDim.x * blockDim.x))
-            body(r, c);
-}
-
 }  // namespace swe
