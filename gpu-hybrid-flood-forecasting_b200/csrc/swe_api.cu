@@ -166,8 +166,8 @@ namespace {
 // Programmatic stream serialisation of a sequence of steps (SWE_PDL=0 turns it off):
 // a step's CTAs are placed as the previous step's leave, and load what no step
 // writes before they wait for it (griddepcontrol.wait; without the attribute that
-// instruction does nothing).  us a step with it and without: 128^2 4.3 / 5.0, 256^2
-// exact 6.5 / 7.0, 512^2 7.5 / 7.9, 1024^2 14.4 / 15.0, 2048^2 43.5 / 44.1.
+// instruction does nothing).  us a step with it and without: 128^2 4.2 / 4.8, 256^2
+// exact 6.1 / 6.8, 512^2 7.4 / 7.8, 1024^2 14.1 / 14.7, 2048^2 42.9 / 43.5.
 // Only a kernel whose predecessor in the stream writes no bed or n^2 may carry it:
 // the steps of a run or a rollout.
 bool pdl_enabled() {
@@ -248,11 +248,11 @@ void dispatch(const swe_domain* d, int V, bool run, F&& f) {
 
 // Rows per warp of a grid that does not fill the GPU: a step then lasts as long
 // as one warp's march, so it is split until every scheduler has two warps (kFewWarps
-// per SM), but not below the split that fills one wave (`one_wave`), and not
-// beyond 4 rows, where more warps in the wave are worth more.  Measured (us a step in
-// blocks of 100 steps, fast unless said, at 1 / 2 / 4 / 8 rows): 128^2 7.3 / 8.0 /
-// 8.7 / 11.5; 300 x 420 9.8 / 8.7 / 9.2 / 12.0; 256^2 exact 10.2 / 10.5 / 12.0 / 16.2;
-// 512^2 exact 23 / 16.5 / 14.1 / 16.7; 700^2 at 4 / 6 / 8 rows 13.7 / 14.4 / 14.3.
+// per SM): 1 to 4 rows, but not below the rows of one full wave (`one_wave`).
+// Measured (us a step of 320 resident steps, fast unless said, at 1 / 2 / 4 / 8 rows):
+// 128^2 4.2 / 5.0 / 6.1 / 8.6; 300 x 420 6.4 / 5.9 / 6.9 / 9.3; 256^2 exact 6.1 / 7.2 /
+// 9.1 / 13.4; 512^2 11.0 / 7.6 / 7.5 / 9.2, exact 14.4 / 10.8 / 10.8 / 14.1; masked 517 x
+// 551 exact 17.4 / 11.9 / 11.8 / 15.9; 700^2 at 4 / 6 / 8 rows 10.5 / 12.9 / 11.0.
 constexpr int kFewWarps = 8;
 
 int march_rows(int64_t one_wave, int64_t two_a_scheduler) {
@@ -705,8 +705,8 @@ int64_t steps_expected(double t, double dt, double t_end, int steps, int outputs
 // passed.  A run to a known end time is paced: after kProbe steps the host knows
 // dt, and it queues no more than the steps expected to be left, polling one chunk
 // late while more are, so that the stream neither runs dry in the middle nor works
-// off launches past the end (a launch that finds its run ended still takes 3 us on
-// 512^2; a 22-step interval used to queue 64).
+// off launches past the end (one that finds its run ended still takes 3 us on 512^2:
+// 32-step chunks polled one late would queue 64 for an interval of 22 steps).
 template <class OnPoll>
 int run_steps(swe_domain* d, const Plan& pl, int64_t max_steps, double t_end, int n_out, cudaStream_t st, OnPoll&& on_poll) {
     constexpr int kProbe = 4;
@@ -1305,9 +1305,8 @@ int swe_domain_create(const swe_domain_desc* desc, swe_domain_t* out) {
     d->device = dev;
     d->sms = prop.multiProcessorCount;
     d->arith = q.arithmetic;
-    // Runs use the paired-lane kernel in both arithmetics (exact arithmetic keeps
-    // its operations scalar, but the paired march still measured 5.7 % faster on
-    // the 2048^2 urban step than one cell per lane; the results are the same).
+    // Runs use the paired-lane kernel in both arithmetics (the results are those of one
+    // cell per lane, which SWE_RUN_VEC=1 runs).
     d->run_vec = 2;
     if (const char* e = std::getenv("SWE_ROWS_PER_WARP")) d->rows_per_warp_override = std::atoi(e);
     if (const char* e = std::getenv("SWE_RUN_VEC")) {

@@ -2,16 +2,13 @@
 // CFL maximum and volume, and the results, each as ONE launch for any number of
 // domains.
 //
-// A run used to start with three plane copies, the fill of the strip-edge array,
-// the control block, a reduction over the copied state and the clearing of the
-// ledger slots, and to end with a fold, a copy of the control block and three
-// plane copies, per domain: 24 ensemble members queued about 290 operations
-// around 50 steps, 2.4 of the call's 10.5 ms (now 0.9 of 9.0).  A state of 96 x 130
-// was reduced in 18 us, by 12 CTAs with IEEE divisions (now compute_cfl_dt and a
-// step on it take 48 us together instead of 74).  Here the state is read once: each cell goes
-// into the run's first ping-pong buffer (and into output 0 and the strip-edge
-// array) and into the reduction in the same pass, and the domains of a batch are
-// parts of one grid, their arguments in the launch parameters.
+// The state is read once: each cell goes into the run's first ping-pong buffer (and
+// into output 0 and the strip-edge array) and into the reduction in the same pass,
+// and the domains of a batch are parts of one grid, their arguments in the launch
+// parameters.  What the calls around the steps cost is launches: 24 ensemble members
+// start and end 50 steps in 0.9 of 9.0 ms with four of them (2.4 of 10.5 ms with a
+// dozen operations a member), and compute_cfl_dt and a step of 96 x 130 take 48 us
+// together (74 us with a clear, a reduction with IEEE divisions and a copy).
 #pragma once
 
 #include "swe_exact.cuh"
@@ -112,7 +109,9 @@ __device__ __forceinline__ float inverse_dt(const Consts& k, float rdx, float rd
     if constexpr (M::kExact) {
         if (!(k.forms & kFormQuick)) return ieee_inverse_dt(h, hu, hv, k.g, k.dry, k.dx, k.dy);
         // The branch-free form, and the IEEE operations for a cell outside its range.
-        // (A velocity too small for it does not reach the sum: the celerity of a wet cell is above 1e-5.)
+        // (A velocity too small for it does not reach the sum: the celerity of a wet cell is
+        // 2^-18 at least, from the smallest gravity and dry tolerance of kFormQuick, and
+        // only quotients below 2^-94 can differ.)
         const SoloOps o;
         const bool wet = h > k.dry;
         const float rh = quick_rcp(o, h);

@@ -3,12 +3,10 @@
 // The exact policy returns what IEEE float32 arithmetic returns, operation by
 // operation.  The compiler's correctly rounded division and square root test
 // their operands and branch to a slow path outside a range (a zero numerator is
-// outside it), and a step takes about 25 divisions and 5 roots per cell: the
-// 2048 x 1024 urban step executed 41.9 warp instructions per cell with 21.5 of
-// 32 lanes active, and waited for instruction fetches and branches in 2.8 of
-// 6.9 cycles between issues.  With the form below the step of the 2048^2 urban
-// grid takes 76 us (304 us before) and that of a masked 517 x 551 grid 12.5 us (62
-// us), of which strip-edge arrays and split marches are part.  QuickExact computes
+// outside it), and a step takes about 25 divisions and 5 roots per cell: with them
+// the 2048^2 urban step executes 41.9 warp instructions per cell with 21.5 of 32
+// lanes active, waits for instruction fetches and branches in 2.8 of 6.9 cycles
+// between issues and takes 303 us; with the form below 75.5 us.  QuickExact computes
 // the same values from the published sequences for a machine with fused multiply-add (P. Markstein,
 // "Computation of elementary functions on the IBM RISC System/6000 processor",
 // IBM J. Res. Dev. 34(1), 1990):
@@ -139,7 +137,7 @@ __device__ __forceinline__ float2 quick_hypot(float2 a, float2 b) {
     return {quick_hypot(a.x, b.x), quick_hypot(a.y, b.y)};
 }
 
-// x ** float32(7/3) (pow73_core) of a pair, from rx = quick_rcp(x).
+// x ** float32(7/3) (pow73_value) of a pair, from rx = quick_rcp(x).
 __device__ __forceinline__ float2 quick_pow73(const PairOps& o, float2 x, float2 rx) {
     const float2 lg = {lg2_approx(x.x), lg2_approx(x.y)};
     const float2 e = o.mul(lg, o.splat(kThird));

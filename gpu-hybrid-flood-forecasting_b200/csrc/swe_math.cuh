@@ -5,7 +5,7 @@
 // explicit __fadd_rn/__fmul_rn/__fdiv_rn/__fsqrt_rn intrinsics, which the
 // compiler never contracts into FMA whatever the -fmad setting.  Its only
 // deliberate difference from the reference is the power in the friction term
-// (pow73_exact: within 0.5001 ulp of the exact power over the depths of a
+// (pow73_exact: within 0.50003 ulp of the exact power over the depths of a
 // flood, where NumPy's and CUDA's powf reach 0.9 ulp; powf elsewhere).
 // hypot is evaluated as glibc's hypotf does (double products, one double sqrt,
 // one rounding to float), which NumPy's float32 hypot reproduces.
@@ -42,7 +42,7 @@ __device__ __forceinline__ float ex2_approx(float a) {
     return r;
 }
 
-// Depths for which pow73_core holds: far beyond a flood's on both sides.
+// Depths for which pow73_value is used: far beyond a flood's on both sides.
 constexpr float kPowLo = 9.3132257e-10f, kPowHi = 1048576.0f;  // 2^-30, 2^20
 
 constexpr float kThird = 0.333333343f;
