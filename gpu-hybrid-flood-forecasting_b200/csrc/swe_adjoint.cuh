@@ -15,7 +15,9 @@
 // only for h > dry; hypot only for a non-zero norm; HLL speed min/max route to
 // the selected argument; the flux select follows the taken branch.
 //
-// One kernel per reverse step, adj_march_kernel; or two, where lam_out aliases lam:
+// One kernel per reverse step: adj_march_kernel where U_{k+1} is known (a rollout's
+// reverse), adj_march_faces_kernel where it is not (a single step); or two, where
+// lam_out aliases lam:
 //   adj_cell_kernel  recomputes the cell's forward update (its four faces) and
 //                    reverses the pointwise part (rain, clip, friction, masks):
 //                    lambda_upd = dL/d(upd) per cell, plus the n^2 and rain
@@ -277,6 +279,64 @@ __device__ __forceinline__ void adj_face_vjp(const FaceInT<T>& lo, const FaceInT
     }
 }
 
+// What the reverse of a cell knows of its update before the pointwise part: nothing (it is
+// rebuilt from the cell's four faces), the step's own output U_{k+1}, or the update
+// without the rain.
+enum class AdjSource { kNothing, kNext, kUpdate };
+
+// Forward flux of a face (or a pair of faces), mass, normal and tangential momentum, and
+// the pressure corrections of its two sides: adj_face_fwd without branches.
+template <class T>
+struct AdjFlux {
+    T m, n, t, lo, hi;
+};
+
+template <int AXIS, bool MASKED, class T>
+__device__ __forceinline__ AdjFlux<T> adj_flux(const FaceInT<T>& lo, const FaceInT<T>& hi, const AdjConsts& k) {
+    const T zero = lit<T>(0.f), one = lit<T>(1.f);
+    const Flag<T> hi_wall = lo.act & !hi.act, lo_wall = !lo.act & hi.act;
+    auto side = [&](const FaceInT<T>& f, const FaceInT<T>& across, const Flag<T>& wall) {
+        FaceInT<T> s = f;
+        if (AXIS == 0) {
+            s.u = f.v;
+            s.v = f.u;
+        }
+        if constexpr (MASKED) {  // the mirrored copy of the cell across a wall
+            s.h = sel(wall, across.h, s.h);
+            s.z = sel(wall, across.z, s.z);
+            s.u = sel(wall, -(AXIS == 1 ? across.u : across.v), s.u);
+            s.v = sel(wall, AXIS == 1 ? across.v : across.u, s.v);
+        }
+        return s;
+    };
+    const FaceInT<T> L = side(lo, hi, lo_wall), R = side(hi, lo, hi_wall);  // u: normal, v: tangential
+    const T zf = vmax(L.z, R.z);
+    const T HL = vmax(L.h + L.z - zf, zero), HR = vmax(R.h + R.z - zf, zero);
+    const Flag<T> wL = gt(HL, k.dry), wR = gt(HR, k.dry);
+    const T nL = sel(wL, L.u, zero), nR = sel(wR, R.u, zero), tL = sel(wL, L.v, zero), tR = sel(wR, R.v, zero);
+    const T cL = asqrt(k.g * HL), cR = asqrt(k.g * HR);
+    const T sL = vmin(nL - cL, nR - cR), sR = vmax(nL + cL, nR + cR);
+    const T spread = sR - sL;
+    const T rden = arcp(sel(gt(spread, kHllEps), spread, one)), s01 = sL * sR;
+    const Flag<T> take_l = ge(sL, zero), take_r = ge(zero, sR);
+    const T NL = HL * L.u, NR = HR * R.u;
+    auto hll = [&](T fl, T fr, T jump) {
+        return sel(take_l, fl, sel(take_r, fr, (sR * fl - sL * fr + s01 * jump) * rden));
+    };
+    AdjFlux<T> f;
+    f.m = hll(NL, NR, HR - HL);
+    f.n = hll(NL * nL + k.half_g * (HL * HL), NR * nR + k.half_g * (HR * HR), NR - NL);
+    f.t = hll(NL * tL, NR * tR, HR * R.v - HL * L.v);
+    f.lo = k.half_g * (L.h * L.h - HL * HL);
+    f.hi = k.half_g * (R.h * R.h - HR * HR);
+    if constexpr (MASKED) {
+        const Flag<T> relevant = lo.act | hi.act;
+        f = {sel(relevant, f.m, zero), sel(relevant, f.n, zero), sel(relevant, f.t, zero), sel(relevant, f.lo, zero),
+             sel(relevant, f.hi, zero)};
+    }
+    return f;
+}
+
 struct AdjLaunch {
     DomainDev d;
     StateView in;        // U_k
@@ -332,15 +392,15 @@ __device__ __noinline__ inline AdjUpd adj_cell_update(const AdjLaunch& p, int r,
 // lu = dL/d(upd); when `owned`, also adds the cell's dL/d(n^2) to grad_n2 and its
 // rain-scale term to *rain_acc.
 //
-// With NEXT the cell update before the pointwise part is rebuilt from the step's
+// With kNext the cell update before the pointwise part is rebuilt from the step's
 // own output U_{k+1} = (h1, q1, q2) instead of from the cell's four faces.  The
 // momenta invert the semi-implicit friction: with a = dt g n^2 max(h,dry)^(-7/3),
 // q = upd/(1 + a|upd|) gives upd = q/(1 - a|q|).  Where that inversion loses
 // precision (a|q| > 0.999, i.e. friction dividing the momentum by more than 1000)
 // the update is rebuilt from the faces.  For dry or clipped cells only the depth
 // part is needed: the momentum outputs are zero and carry no gradient.
-template <bool NEXT, bool MASKED>
-__device__ __forceinline__ void adj_pointwise(const AdjLaunch& p, int r, int c, V2 nm, const V2 lam[3], const V2 next[3],
+template <AdjSource SRC, bool MASKED>
+__device__ __forceinline__ void adj_pointwise(const AdjLaunch& p, int r, int c, V2 nm, const V2 lam[3], const V2 known[3],
                                               B2 live, B2 owned, double* rain_acc, V2 lu[3]) {
     const DomainDev& d = p.d;
     const V2 zero = lit<V2>(0.f), n2 = MASKED ? vabs(nm) : nm;
@@ -351,27 +411,34 @@ __device__ __forceinline__ void adj_pointwise(const AdjLaunch& p, int r, int c, 
     }
     V2 u0 = zero, u1 = zero, u2 = zero;  // u0: the depth after the rain (before the clip)
     B2 rebuild = live;
-    if constexpr (NEXT) {
-        u0 = next[0];
+    if constexpr (SRC == AdjSource::kUpdate) {
+        u0 = known[0] + p.s.dt_rain * mult;
+        u1 = known[1];
+        u2 = known[2];
+    }
+    if constexpr (SRC == AdjSource::kNext) {
+        u0 = known[0];
         const B2 wet = gt(u0, p.k.dry);
         const V2 pw = apow(vmax(u0, lit<V2>(p.k.dry)), -7.0f / 3.0f);
-        const V2 aq = p.s.dt_g * n2 * pw * asqrt(next[1] * next[1] + next[2] * next[2]);
+        const V2 aq = p.s.dt_g * n2 * pw * asqrt(known[1] * known[1] + known[2] * known[2]);
         const V2 den = arcp(lit<V2>(1.f) - aq);
-        u1 = sel(wet, next[1] * den, zero);
-        u2 = sel(wet, next[2] * den, zero);
+        u1 = sel(wet, known[1] * den, zero);
+        u2 = sel(wet, known[2] * den, zero);
         rebuild = live & wet & B2{!(aq.v.x <= 0.999f), !(aq.v.y <= 0.999f)};
     }
-    if (rebuild.x) {
-        const AdjUpd t = adj_cell_update(p, r, c);
-        u0.v.x = t.u0 + p.s.dt_rain * mult.v.x;
-        u1.v.x = t.u1;
-        u2.v.x = t.u2;
-    }
-    if (rebuild.y) {
-        const AdjUpd t = adj_cell_update(p, r, c + 1);
-        u0.v.y = t.u0 + p.s.dt_rain * mult.v.y;
-        u1.v.y = t.u1;
-        u2.v.y = t.u2;
+    if constexpr (SRC != AdjSource::kUpdate) {
+        if (rebuild.x) {
+            const AdjUpd t = adj_cell_update(p, r, c);
+            u0.v.x = t.u0 + p.s.dt_rain * mult.v.x;
+            u1.v.x = t.u1;
+            u2.v.x = t.u2;
+        }
+        if (rebuild.y) {
+            const AdjUpd t = adj_cell_update(p, r, c + 1);
+            u0.v.y = t.u0 + p.s.dt_rain * mult.v.y;
+            u1.v.y = t.u1;
+            u2.v.y = t.u2;
+        }
     }
     const V2 h = vmax(u0, zero);
     const V2 pw = apow(vmax(h, lit<V2>(p.k.dry)), -7.0f / 3.0f);
@@ -432,7 +499,7 @@ __global__ void __launch_bounds__(THREADS) adj_cell_kernel(const __grid_constant
             next[1] = one(p.next.hu[no]);
             next[2] = one(p.next.hv[no]);
         }
-        adj_pointwise<NEXT, true>(p, r, c, one(nm), lam, next, B2{active(nm), false}, B2{true, false}, &rain_acc, lu);
+        adj_pointwise<NEXT ? AdjSource::kNext : AdjSource::kNothing, true>(p, r, c, one(nm), lam, next, B2{active(nm), false}, B2{true, false}, &rain_acc, lu);
         const int64_t lo = (int64_t)r * p.lpitch + c;
         p.lupd[0][lo] = lu[0].v.x;
         p.lupd[1][lo] = lu[1].v.x;
@@ -616,21 +683,22 @@ __device__ __forceinline__ void load_lam(const AdjLaunch& p, int r, int c0, int 
     a.l2 = load2<VEC, false>(p.lam.hv, lo, c0, c1);
 }
 
-template <bool NEXT, bool VEC>
+template <bool VEC>
 __device__ __forceinline__ AdjRaw adj_raw(const AdjLaunch& p, int r, int c0, int c1) {
     AdjRaw a;
-    load_states<NEXT, VEC>(p, r, c0, c1, a);
+    load_states<true, VEC>(p, r, c0, c1, a);
     load_lam<VEC>(p, r, c0, c1, a);
     return a;
 }
 
-// Cells (r, c) and (r, c + 1) from their loaded values: velocities, and the
-// pointwise reverse (rain, clip, friction, masks) of the cells inside the grid
-// (flags `in`); the others carry no dL/d(upd).  Owned cells add their n^2 and
-// rain-scale gradients.
-template <bool NEXT, bool MASKED, bool VEC>
-__device__ __forceinline__ AdjCells adj_cells(const AdjLaunch& p, AdjRaw a, int r, int c, B2 in, B2 owned,
-                                              double* rain_acc) {
+// The momenta that a cell's faces see: those of the ghost ring are mirrored.
+struct AdjMomenta {
+    V2 hu, hv;
+};
+
+// Cells (r, c) and (r, c + 1) from their loaded values: velocities, no dL/d(upd) yet.
+template <bool MASKED, bool VEC>
+__device__ __forceinline__ AdjCells adj_velocities(const AdjLaunch& p, AdjRaw& a, int r, int c, AdjMomenta& m) {
     const DomainDev& d = p.d;
     if (VEC && (c < 0 || c >= d.cols)) {
         auto edge = [&](V2& x) { c < 0 ? x.v.y = x.v.x : x.v.x = x.v.y; };
@@ -645,6 +713,7 @@ __device__ __forceinline__ AdjCells adj_cells(const AdjLaunch& p, AdjRaw a, int 
     if (d.bnd[0] == 0) hu = {{c < 0 ? -hu.v.x : hu.v.x, c + 1 < 0 ? -hu.v.y : hu.v.y}};
     if (d.bnd[1] == 0) hu = {{c >= d.cols ? -hu.v.x : hu.v.x, c + 1 >= d.cols ? -hu.v.y : hu.v.y}};
     if ((r < 0 && d.bnd[2] == 0) || (r >= d.rows && d.bnd[3] == 0)) hv = -hv;
+    m = {hu, hv};
     const V2 zero = lit<V2>(0.f);
     AdjCells k;
     k.f.h = a.h;
@@ -655,10 +724,21 @@ __device__ __forceinline__ AdjCells adj_cells(const AdjLaunch& p, AdjRaw a, int 
     k.f.u = sel(deep, hu * k.f.rh, zero);
     k.f.v = sel(deep, hv * k.f.rh, zero);
     k.l[0] = k.l[1] = k.l[2] = zero;
-    if (r >= 0 && r < d.rows) {
+    return k;
+}
+
+// The same with the pointwise reverse (rain, clip, friction, masks) of the cells inside
+// the grid (flags `in`) from U_{k+1}; the others carry no dL/d(upd).  Owned cells add
+// their n^2 and rain-scale gradients.
+template <bool MASKED, bool VEC>
+__device__ __forceinline__ AdjCells adj_cells(const AdjLaunch& p, AdjRaw a, int r, int c, B2 in, B2 owned,
+                                              double* rain_acc) {
+    AdjMomenta m;
+    AdjCells k = adj_velocities<MASKED, VEC>(p, a, r, c, m);
+    if (r >= 0 && r < p.d.rows) {
         const B2 live = in & k.f.act;
         const V2 lam[3] = {a.l0, a.l1, a.l2}, next[3] = {a.h1, a.q1, a.q2};
-        adj_pointwise<NEXT, MASKED>(p, r, c, a.nm, lam, next, live, owned, rain_acc, k.l);
+        adj_pointwise<AdjSource::kNext, MASKED>(p, r, c, a.nm, lam, next, live, owned, rain_acc, k.l);
     }
     return k;
 }
@@ -687,7 +767,71 @@ __device__ __forceinline__ void adj_faces(const AdjConsts& k, const AdjCells& lo
     adj_face_vjp<AXIS, MASKED, V2>(lo.f, hi.f, k, lF, -(s * lo.l[nq]), s * hi.l[nq], dlo, dhi);
 }
 
-template <int THREADS, bool NEXT, bool MASKED, bool VEC>
+// dL/dU_k of row r into lam_out: the faces left, right, below (their upper side, carried in
+// `below`) and above of the row's cells.
+template <bool MASKED, bool VEC>
+__device__ __forceinline__ void adj_gather(const AdjLaunch& p, const AdjCells& cur, const AdjCells& nxt, int r, int c, B2 mine,
+                                           float ax, float ay, V2 below[3]) {
+    const DomainDev& d = p.d;
+    V2 lo[3], hi[3], g[3];
+    adj_faces<0, MASKED>(p.k, cur, nxt, ay, lo, hi);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        g[q] = cur.l[q] + below[q] + lo[q];
+        below[q] = hi[q];
+    }
+    if (r == d.rows - 1) {
+        g[0] = g[0] + hi[0];
+        g[1] = g[1] + hi[1];
+        g[2] = g[2] + (d.bnd[3] == 0 ? -hi[2] : hi[2]);
+    }
+    adj_faces<1, MASKED>(p.k, cur, right_of<MASKED>(cur), ax, lo, hi);
+    const float sw = d.bnd[0] == 0 ? -1.f : 1.f, se = d.bnd[1] == 0 ? -1.f : 1.f;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        // hi.x is this lane's second cell's left side, hi.y the next lane's first cell's.
+        const float from_left = __shfl_up_sync(0xffffffffu, hi[q].v.y, 1);
+        g[q] = g[q] + lo[q] + V2{{from_left, hi[q].v.x}};
+        const float west = __shfl_up_sync(0xffffffffu, lo[q].v.y, 1);  // the ghost left of column 0
+        if (c == 0) g[q].v.x += (q == 1 ? sw : 1.f) * west;
+        if (c == d.cols - 1) g[q].v.x += (q == 1 ? se : 1.f) * hi[q].v.x;
+        if (c + 1 == d.cols - 1) g[q].v.y += (q == 1 ? se : 1.f) * hi[q].v.y;
+    }
+    const uint32_t o = (uint32_t)r * (uint32_t)p.lam_out.pitch + (uint32_t)c;
+    if (VEC && mine.y) {
+        *reinterpret_cast<float2*>(p.lam_out.h + o) = g[0].v;
+        *reinterpret_cast<float2*>(p.lam_out.hu + o) = g[1].v;
+        *reinterpret_cast<float2*>(p.lam_out.hv + o) = g[2].v;
+    } else {
+        if (mine.x) {
+            p.lam_out.h[o] = g[0].v.x;
+            p.lam_out.hu[o] = g[1].v.x;
+            p.lam_out.hv[o] = g[2].v.x;
+        }
+        if (mine.y) {
+            p.lam_out.h[o + 1] = g[0].v.y;
+            p.lam_out.hu[o + 1] = g[1].v.y;
+            p.lam_out.hv[o + 1] = g[2].v.y;
+        }
+    }
+}
+
+// The upper side of the face between a chunk's first row and the row below it.
+template <bool MASKED>
+__device__ __forceinline__ void adj_first_face(const AdjLaunch& p, const AdjCells& cur, const AdjCells& nxt, int r0, float ay,
+                                               V2 below[3]) {
+    V2 blo[3];
+    adj_faces<0, MASKED>(p.k, cur, nxt, ay, blo, below);
+    // Ghost cells are mirrored copies of their boundary cell: their side of a
+    // boundary face belongs to that cell (normal momentum sign-flipped on reflective edges).
+    if (r0 == 0) {
+        below[0] = below[0] + blo[0];
+        below[1] = below[1] + blo[1];
+        below[2] = below[2] + (p.d.bnd[2] == 0 ? -blo[2] : blo[2]);
+    }
+}
+
+template <int THREADS, bool MASKED, bool VEC>
 __global__ void __launch_bounds__(THREADS) adj_march_kernel(const __grid_constant__ AdjLaunch p, int nstrips,
                                                             int rows_per_warp) {
     const DomainDev& d = p.d;
@@ -709,73 +853,98 @@ __global__ void __launch_bounds__(THREADS) adj_march_kernel(const __grid_constan
         // The states are those of a finished forward pass; only lam (and the gradients)
         // come from the reverse step before, which is waited for once they are loading.
         AdjRaw raw, ahead;
-        load_states<NEXT, VEC>(p, r0 - 1, c0, c1, raw);
-        load_states<NEXT, VEC>(p, r0, c0, c1, ahead);
+        load_states<true, VEC>(p, r0 - 1, c0, c1, raw);
+        load_states<true, VEC>(p, r0, c0, c1, ahead);
         pdl_enter();
         load_lam<VEC>(p, r0 - 1, c0, c1, raw);
         load_lam<VEC>(p, r0, c0, c1, ahead);
-        AdjCells cur = adj_cells<NEXT, MASKED, VEC>(p, raw, r0 - 1, c, in, B2{false, false}, &rain_acc);
+        AdjCells cur = adj_cells<MASKED, VEC>(p, raw, r0 - 1, c, in, B2{false, false}, &rain_acc);
         raw = ahead;
-        ahead = adj_raw<NEXT, VEC>(p, r0 + 1, c0, c1);
-        AdjCells nxt = adj_cells<NEXT, MASKED, VEC>(p, raw, r0, c, in, mine, &rain_acc);
+        ahead = adj_raw<VEC>(p, r0 + 1, c0, c1);
+        AdjCells nxt = adj_cells<MASKED, VEC>(p, raw, r0, c, in, mine, &rain_acc);
         V2 below[3];  // the upper side of the y-face below the row
-        {
-            V2 blo[3];
-            adj_faces<0, MASKED>(p.k, cur, nxt, ay, blo, below);
-            // Ghost cells are mirrored copies of their boundary cell: their side of a
-            // boundary face belongs to that cell (normal momentum sign-flipped on reflective edges).
-            if (r0 == 0) {
-                below[0] = below[0] + blo[0];
-                below[1] = below[1] + blo[1];
-                below[2] = below[2] + (d.bnd[2] == 0 ? -blo[2] : blo[2]);
-            }
-        }
+        adj_first_face<MASKED>(p, cur, nxt, r0, ay, below);
         for (int r = r0; r < r1; ++r) {
             cur = nxt;
             raw = ahead;
-            if (r + 2 <= r1) ahead = adj_raw<NEXT, VEC>(p, r + 2, c0, c1);
-            nxt = adj_cells<NEXT, MASKED, VEC>(p, raw, r + 1, c, in, r + 1 < r1 ? mine : B2{false, false}, &rain_acc);
-            V2 lo[3], hi[3], g[3];
-            adj_faces<0, MASKED>(p.k, cur, nxt, ay, lo, hi);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                g[q] = cur.l[q] + below[q] + lo[q];
-                below[q] = hi[q];
-            }
-            if (r == d.rows - 1) {
-                g[0] = g[0] + hi[0];
-                g[1] = g[1] + hi[1];
-                g[2] = g[2] + (d.bnd[3] == 0 ? -hi[2] : hi[2]);
-            }
-            adj_faces<1, MASKED>(p.k, cur, right_of<MASKED>(cur), ax, lo, hi);
-            const float sw = d.bnd[0] == 0 ? -1.f : 1.f, se = d.bnd[1] == 0 ? -1.f : 1.f;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                // hi.x is this lane's second cell's left side, hi.y the next lane's first cell's.
-                const float from_left = __shfl_up_sync(0xffffffffu, hi[q].v.y, 1);
-                g[q] = g[q] + lo[q] + V2{{from_left, hi[q].v.x}};
-                const float west = __shfl_up_sync(0xffffffffu, lo[q].v.y, 1);  // the ghost left of column 0
-                if (c == 0) g[q].v.x += (q == 1 ? sw : 1.f) * west;
-                if (c == d.cols - 1) g[q].v.x += (q == 1 ? se : 1.f) * hi[q].v.x;
-                if (c + 1 == d.cols - 1) g[q].v.y += (q == 1 ? se : 1.f) * hi[q].v.y;
-            }
-            const uint32_t o = (uint32_t)r * (uint32_t)p.lam_out.pitch + (uint32_t)c;
-            if (VEC && mine.y) {
-                *reinterpret_cast<float2*>(p.lam_out.h + o) = g[0].v;
-                *reinterpret_cast<float2*>(p.lam_out.hu + o) = g[1].v;
-                *reinterpret_cast<float2*>(p.lam_out.hv + o) = g[2].v;
-            } else {
-                if (mine.x) {
-                    p.lam_out.h[o] = g[0].v.x;
-                    p.lam_out.hu[o] = g[1].v.x;
-                    p.lam_out.hv[o] = g[2].v.x;
-                }
-                if (mine.y) {
-                    p.lam_out.h[o + 1] = g[0].v.y;
-                    p.lam_out.hu[o + 1] = g[1].v.y;
-                    p.lam_out.hv[o + 1] = g[2].v.y;
-                }
-            }
+            if (r + 2 <= r1) ahead = adj_raw<VEC>(p, r + 2, c0, c1);
+            nxt = adj_cells<MASKED, VEC>(p, raw, r + 1, c, in, r + 1 < r1 ? mine : B2{false, false}, &rain_acc);
+            adj_gather<MASKED, VEC>(p, cur, nxt, r, c, mine, ax, ay, below);
+        }
+    }
+    adj_flush_rain<THREADS>(p, rain_acc);
+}
+
+// The same without U_{k+1}: the updates are rebuilt from the faces' forward fluxes, each
+// evaluated once within the warp, one row ahead of the reverse (the rows and columns
+// outside the strip once more).  us a call at 257 x 333 masked, 512^2, 700^2, 1024^2,
+// 2048^2 and masked 3000 x 3001: 22 (the host), 22, 23, 54, 208 and 458; with each
+// cell's update rebuilt apart from its four faces and their cells' loads 25, 36, 49, 116,
+// 370 and 796, in a tile of 32 x 16 cells 22, 31, 46, 102, 399 and 874.
+template <int THREADS, bool MASKED, bool VEC>
+__global__ void __launch_bounds__(THREADS, 3) adj_march_faces_kernel(const __grid_constant__ AdjLaunch p, int nstrips,
+                                                                  int rows_per_warp) {
+    const DomainDev& d = p.d;
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * (THREADS / kWarp) + (threadIdx.x >> 5);
+    const int r0 = (gw / nstrips) * rows_per_warp, r1 = min(r0 + rows_per_warp, d.rows);
+    const int c = (gw % nstrips) * kMarchCols - 2 + 2 * lane;
+    const int c0 = min(max(c, 0), VEC ? d.cols - 2 : d.cols - 1), c1 = min(max(c + 1, 0), d.cols - 1);
+    const B2 in{c >= 0 && c < d.cols, c + 1 >= 0 && c + 1 < d.cols};
+    const bool strip = lane >= 1 && lane <= kWarp - 2;
+    const B2 mine{strip && in.x, strip && in.y}, none{false, false};
+    const float ax = p.s.dt * p.rdx, ay = p.s.dt * p.rdy;
+    double rain_acc = 0.0;
+    if (r0 < d.rows) {
+        struct Row {
+            AdjCells k;
+            AdjMomenta m;
+            V2 nm;
+        };
+        struct Flux {
+            V2 m, n, t;  // mass, normal (with the side's pressure correction) and tangential momentum
+        };
+        auto row = [&](int r) -> Row {
+            AdjRaw a;
+            load_states<false, VEC>(p, r, c0, c1, a);
+            Row w;
+            w.k = adj_velocities<MASKED, VEC>(p, a, r, c, w.m);
+            w.nm = a.nm;
+            return w;
+        };
+        Flux low;  // the upper side of the face below the row
+        auto face_above = [&](const Row& w, const Row& above) -> Flux {
+            const AdjFlux<V2> f = adj_flux<0, MASKED, V2>(w.k.f, above.k.f, p.k);
+            low = {f.m, f.n + f.hi, f.t};
+            return {f.m, f.n + f.lo, f.t};
+        };
+        // dL/d(upd) of row r of cells w from its faces.
+        auto reverse = [&](Row& w, const Row& above, int r, B2 owned) {
+            const Flux yb = low, yt = face_above(w, above);
+            const AdjFlux<V2> f = adj_flux<1, MASKED, V2>(w.k.f, right_of<MASKED>(w.k).f, p.k);
+            // f.x is the face between a lane's cells, f.y the one to the next lane's first cell.
+            auto left = [](V2 x) { return V2{{__shfl_up_sync(0xffffffffu, x.v.y, 1), x.v.x}}; };
+            const V2 xm = f.m - left(f.m), xn = f.n + f.lo - left(f.n + f.hi), xt = f.t - left(f.t);
+            if (r < 0 || r >= d.rows) return;
+            const V2 upd[3] = {w.k.f.h - (ax * xm + ay * (yt.m - yb.m)), w.m.hu - (ax * xn + ay * (yt.t - yb.t)),
+                               w.m.hv - (ax * xt + ay * (yt.n - yb.n))};
+            AdjRaw a;
+            load_lam<VEC>(p, r, c0, c1, a);
+            const V2 lam[3] = {a.l0, a.l1, a.l2};
+            adj_pointwise<AdjSource::kUpdate, MASKED>(p, r, c, w.nm, lam, upd, in & w.k.f.act, owned, &rain_acc, w.k.l);
+        };
+        Row cur = row(r0 - 1), nxt = row(r0), ahead = row(r0 + 1);
+        face_above(row(r0 - 2), cur);
+        reverse(cur, nxt, r0 - 1, none);
+        reverse(nxt, ahead, r0, mine);
+        V2 below[3];
+        adj_first_face<MASKED>(p, cur.k, nxt.k, r0, ay, below);
+        for (int r = r0; r < r1; ++r) {
+            cur = nxt;
+            nxt = ahead;
+            ahead = row(r + 2);
+            reverse(nxt, ahead, r + 1, r + 1 < r1 ? mine : none);
+            adj_gather<MASKED, VEC>(p, cur.k, nxt.k, r, c, mine, ax, ay, below);
         }
     }
     adj_flush_rain<THREADS>(p, rain_acc);

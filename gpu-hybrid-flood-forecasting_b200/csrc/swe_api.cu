@@ -1545,14 +1545,14 @@ int adjoint_step_impl(swe_domain* d, const float* h, const float* hu, const floa
         cudaLaunchAttribute attr[1];
         attach_pdl(cfg, attr, chained);
         auto launch = [&](auto kernel) { cudaLaunchKernelEx(&cfg, kernel, al, nstrips, R); };
-        auto pick = [&](auto nx, auto mk) {
-            constexpr bool N = decltype(nx)::value, M = decltype(mk)::value;
-            if (vec) launch(adj_march_kernel<kThreads, N, M, true>); else launch(adj_march_kernel<kThreads, N, M, false>);
+        auto pick = [&](auto mk, auto vc) {
+            constexpr bool M = decltype(mk)::value, V = decltype(vc)::value;
+            if (next) launch(adj_march_kernel<kThreads, M, V>); else launch(adj_march_faces_kernel<kThreads, M, V>);
         };
-        if (next) {
-            if (d->masked) pick(std::true_type{}, std::true_type{}); else pick(std::true_type{}, std::false_type{});
+        if (d->masked) {
+            if (vec) pick(std::true_type{}, std::true_type{}); else pick(std::true_type{}, std::false_type{});
         } else {
-            if (d->masked) pick(std::false_type{}, std::true_type{}); else pick(std::false_type{}, std::false_type{});
+            if (vec) pick(std::false_type{}, std::true_type{}); else pick(std::false_type{}, std::false_type{});
         }
     } else {
         if (next)
