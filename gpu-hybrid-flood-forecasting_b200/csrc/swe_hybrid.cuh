@@ -38,8 +38,8 @@ struct FeatureArgs {
 // together, and coalesced at every pitch and alignment.  All of them are bound
 // by memory; with one cell at a time a warp had too few bytes in flight.  us at
 // 2048^2 on a cold cache, one cell and four: features (float32, six channels)
-// 56 and 33, correction 22.8 + 38 and 22.4 + 37.8 with a plane less in memory,
-// output fields 33.5 and 21.9; the calls together 159 and 122.
+// 56 and 33, output fields 33.5 and 21.9, the two correction passes 61 and 55 with a
+// plane less in memory; the calls together 159 and 117.
 constexpr int kCells = 4;  // cells a lane takes at a time
 constexpr int kPiece = kCells * kWarp;
 constexpr int kPieceWarps = 8;  // per CTA
